@@ -149,7 +149,7 @@ Tensor permute(Ctx& c, const Tensor& in, const std::vector<int>& perm);
 Tensor clone(Ctx& c, const Tensor& in);
 
 // C = alpha*op(A)*op(B) + beta*C, column-major, op in {'N','T','C'}.
-// Dispatches on c.precision for real operands (FP64 DMMA or 3xTF32 tcgen05).
+// Dispatches on c.precision and the size for real operands (FP64 DMMA or 3xTF32 tcgen05).
 void gemm(Ctx& c, DType dt, char opA, char opB, int64_t m, int64_t n, int64_t k,
           cuDoubleComplex alpha, const void* A, int64_t lda, const void* B, int64_t ldb,
           cuDoubleComplex beta, void* C, int64_t ldc, bool force_fp64 = false);
@@ -180,6 +180,9 @@ void gemm_tf32x3_planes(Ctx& c, const Planes& A, const Planes& B, int64_t m, int
 void gemm_tf32x3(Ctx& c, char opA, char opB, int64_t m, int64_t n, int64_t k, double alpha,
                  const double* A, int64_t lda, const double* B, int64_t ldb, double beta, double* C,
                  int64_t ldc);
+
+// whether the mixed form runs an m x n x k product as 3xTF32 (else in FP64)
+bool tf32x3_pays(int64_t m, int64_t n, int64_t k);
 
 inline cuDoubleComplex cplx(double r, double i = 0) { return make_cuDoubleComplex(r, i); }
 

@@ -36,14 +36,15 @@ const Planes& planes_col(Ctx& c, const Tensor& Rt, PlaneCache* pc) {
   return pc->col;
 }
 
-bool use_planes(const Ctx& c, const MatRef& R, const PlaneCache* pc) {
-  return pc && c.precision == kPrecMixed && R.t.dt == DType::F64;
+bool use_planes(const Ctx& c, const MatRef& R, const PlaneCache* pc, int64_t cols) {
+  return pc && c.precision == kPrecMixed && R.t.dt == DType::F64 && tf32x3_pays(R.rows(), cols, R.cols()) &&
+         tf32x3_pays(R.cols(), cols, R.rows());
 }
 
 }  // namespace
 
 Tensor apply(Ctx& c, const MatRef& R, char op, const Tensor& X, PlaneCache* pc) {
-  if (use_planes(c, R, pc)) {
+  if (use_planes(c, R, pc, X.nd > 1 ? X.dims[1] : 1)) {
     const bool t = (op == 'T') != R.trans;
     const int64_t m = (op == 'N') ? R.rows() : R.cols();
     const int64_t kk = (op == 'N') ? R.cols() : R.rows();
@@ -59,7 +60,7 @@ Tensor apply(Ctx& c, const MatRef& R, char op, const Tensor& X, PlaneCache* pc) 
 }
 
 Tensor apply_left_T(Ctx& c, const Tensor& X, const MatRef& R, char op, PlaneCache* pc) {
-  if (use_planes(c, R, pc)) {
+  if (use_planes(c, R, pc, X.dims[1])) {
     const bool t = (op == 'T') != R.trans;
     const int64_t kk = (op == 'N') ? R.rows() : R.cols();
     const int64_t n = (op == 'N') ? R.cols() : R.rows();

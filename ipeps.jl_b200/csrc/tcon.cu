@@ -204,11 +204,23 @@ Tensor matmul(Ctx& c, const Tensor& A, char opA, const Tensor& B, char opB) {
   return C;
 }
 
+// Which products of the mixed form run as 3xTF32.  Measured per product on B200
+// (splits and split-K sums included): splitting both operands and the pipeline's
+// start cost 20-30 us whatever the size, and the split moves 24 bytes per operand
+// element, so the FP64 kernel is the faster one below ~0.4 GFLOP (1024 x 130 x
+// 1024, 0.27 GFLOP: 28 us against 31; 1450 x 118 x 1450, 0.50 GFLOP: 39 against
+// 34; 2500 x 160 x 2500: 112 against 58) and, at any size, for short inner
+// dimensions (250000 x 50 x 25: 63 us against 89; 1450 x 1450 x 58: 20 against
+// 33; 1975 x 1975 x 79: 39 against 31).
+bool tf32x3_pays(int64_t m, int64_t n, int64_t k) {
+  return k >= 64 && 2.0 * double(m) * double(n) * double(k) >= 4e8;
+}
+
 void gemm(Ctx& c, DType dt, char opA, char opB, int64_t m, int64_t n, int64_t k,
           cuDoubleComplex alpha, const void* A, int64_t lda, const void* B, int64_t ldb,
           cuDoubleComplex beta, void* C, int64_t ldc, bool force_fp64) {
   if (dt == DType::F64 && c.precision == kPrecMixed && !force_fp64 && alpha.y == 0 && beta.y == 0 &&
-      opA != 'C' && opB != 'C') {
+      opA != 'C' && opB != 'C' && tf32x3_pays(m, n, k)) {
     gemm_tf32x3(c, opA, opB, m, n, k, alpha.x, static_cast<const double*>(A), lda,
                 static_cast<const double*>(B), ldb, beta.x, static_cast<double*>(C), ldc);
     return;
