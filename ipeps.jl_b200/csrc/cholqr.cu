@@ -1,0 +1,383 @@
+// Cholesky factor and triangular solve of one CholeskyQR pass for sketches of
+// up to 160 columns: G = R^T R (shifted, guarded), then Q = Y R^-1.
+//
+// Both work on 8 x 8 blocks so that all but the 8 x 8 diagonal factors runs on
+// the FP64 tensor pipe (mma.sync m8n8k4; tcgen05 has no FP64 kind).  R goes from
+// the first kernel to the second in packed blocks, the diagonal ones already
+// inverted.
+//
+// chol_panel is bound by latency: one CTA and k/8 dependent panel steps, of about
+// 1650 cycles (0.85 us) each once the trailing updates fit beside them.  The kernel
+// this one replaces eliminated column by column, ~900 cycles each for the pivot,
+// the barrier and the broadcast loads.  Back-to-back launches at k = 62 / 128 / 160:
+// 10.5 / 20.7 / 28.8 us (18.5 us at k = 62 and 74 us at k = 160 before).
+// trsm_panel is bound by its dependent DMMA steps (one warp of eight rows per
+// scheduler, 33 cycles per DMMA where the pipe takes one in 16): 6.3 us at
+// N = 120, k = 62 and 13.1 us at N = 2500, k = 160 (10.7 and 27 us for the
+// substitution by rows that it replaces).
+// One CholeskyQR pass at N = 2500 without its Gram product, event-timed: 96.9 ->
+// 58 us at k = 160, 71.1 -> 45 us at k = 128, 61.5 -> 39 us at k = 101.
+#include "linalg.cuh"
+
+#include <algorithm>
+
+namespace ipeps {
+namespace {
+
+// Warp w runs on scheduler w mod 4: warp 0 has scheduler 0 to itself (the FP64
+// pipe of each scheduler takes a DMMA every 16 cycles, and the pivots' chain
+// must not queue behind those); the update warps share the other three.
+constexpr int kCpWarps = 16;
+constexpr int kCpThreads = 32 * kCpWarps;
+constexpr int kUpdateWarps = kCpWarps / 4 * 3;
+constexpr int kUpdateThreads = 32 * kUpdateWarps;
+
+__device__ __forceinline__ void dmma8(double& d0, double& d1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+      : "+d"(d0), "+d"(d1)
+      : "d"(a), "d"(b));
+}
+// the same with the sum in another register pair
+__device__ __forceinline__ void dmma8(double& d0, double& d1, double a, double b, double c0, double c1) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%4,%5};\n"
+      : "=d"(d0), "=d"(d1)
+      : "d"(a), "d"(b), "d"(c0), "d"(c1));
+}
+template <int ID, int N>
+__device__ __forceinline__ void bar_wait() {
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(N) : "memory");
+}
+template <int ID, int N>
+__device__ __forceinline__ void bar_post() {
+  asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(N) : "memory");
+}
+
+// 1 / sqrt(d) of a normal d > 0 (anything else: unspecified), within 2 ulp: the
+// hardware estimate y and one third-order step of the series of (1 - e)^(-1/2),
+// e = 1 - d y^2 (Householder's method).  Without rsqrt's cases the compiler is free
+// to fill the pivots' chain with the independent products around it.
+__device__ __forceinline__ double rsqrt_normal(double d) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double e = fma(-d * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// Packed upper block triangle of R, block row by block row: block (I, J) at
+// col_base(I) + J - I.  Inside a block the entries (2t, g) and (2t + 1, g) are
+// neighbours, at 2 (8 t + g): lane (g, t) of a warp then has with one 16-byte
+// access what it needs of the block as the B operand of two m8n8k4 products
+// over k = {2t} and k = {2t + 1}, and what an accumulator or an A operand
+// holds of the transposed block.
+__host__ __device__ __forceinline__ int col_base(int I, int nb) { return I * nb - I * (I - 1) / 2; }
+
+// The matrix sits in shared memory in this layout, as the lower-triangle blocks
+// (I, J) of L = R^T, I >= J; panel p:
+//   warp 0 factors the diagonal block (every lane the whole of it, in registers,
+//     without exchange) and inverts it (lane j column j), forms L_{p+1,p} and
+//     brings the next diagonal block up to date, then goes on with it; barrier 1
+//     tells the others that R_pp^-1 is there;
+//   the update warps form L_Ip = C_Ip R_pp^-1 (barrier 3 among them) and subtract
+//     L_Ip L_Jp^T from the blocks right of the panel, first from the two that
+//     warp 0 reads next (barrier 2).
+// So warp 0's chain never waits for the bulk of an update.  The loops are kept
+// rolled: with the trailing blocks in registers (unrolled by slot) the SM spent
+// its time fetching instructions (55 us at k = 160).
+// The contract is that of chol_blocked: shift_factor * trace is added to the
+// diagonal, a pivot at or below 1e-32 trace leaves R[j][j] = 1 and row j zero.
+__global__ void __launch_bounds__(kCpThreads, 1)
+    chol_panel_kernel(double* G, int k, int64_t ldg, double shift_factor, double2* __restrict__ Rpk, int write_g) {
+  extern __shared__ __align__(16) double2 S[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int nb = (k + 7) >> 3, nblk = nb * (nb + 1) / 2;
+
+  // G's upper triangle (columns from k on: the identity)
+  {
+    constexpr int U = 7;  // blocks in flight per warp
+    int J = 0, first = 0;
+    for (int b0 = warp; b0 < nblk; b0 += U * kCpWarps) {
+      double2 v[U];
+#pragma unroll
+      for (int q = 0; q < U; ++q) {
+        const int b = b0 + q * kCpWarps;
+        while (J < nb && b >= first + nb - J) {
+          first += nb - J;
+          ++J;
+        }
+        const int I = J + b - first, r = 8 * I + g, c = 8 * J + 2 * t;
+        v[q] = make_double2(r == c ? 1.0 : 0.0, r == c + 1 ? 1.0 : 0.0);
+        if (b < nblk && r < k) {
+          if (c < k) v[q].x = G[min(r, c) + int64_t(max(r, c)) * ldg];
+          if (c + 1 < k) v[q].y = G[min(r, c + 1) + int64_t(max(r, c + 1)) * ldg];
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < U; ++q)
+        if (b0 + q * kCpWarps < nblk) S[(b0 + q * kCpWarps) * 32 + lane] = v[q];
+    }
+  }
+  __syncthreads();
+
+  if (warp == 0) {
+    double tr = 0;
+    for (int i = lane; i < k; i += 32) {
+      const double2 q = S[col_base(i >> 3, nb) * 32 + (i & 7) * 4 + ((i & 7) >> 1)];
+      tr += fabs((i & 1) ? q.y : q.x);
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) tr += __shfl_xor_sync(0xffffffffu, tr, o);
+    const double shift = shift_factor > 0 ? shift_factor * tr : 0.0;
+    const double tiny = 1e-300 + 1e-32 * (tr + shift * k);
+    const int me = lane & 7;
+    for (int p = 0; p < nb; ++p) {
+      double2* D = S + col_base(p, nb) * 32;
+      double d[8][8], x[8];  // d[c][r], c <= r: entry (r, c) of the block; x: row `me` of the inverse
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+#pragma unroll
+        for (int c = 0; c <= r; c += 2) {
+          const double2 q = D[r * 4 + c / 2];
+          d[c][r] = q.x;
+          if (c < r) d[c + 1][r] = q.y;
+        }
+        d[r][r] += 8 * p + r < k ? shift : 0.0;
+        x[r] = r == me ? 1.0 : 0.0;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const double piv = d[j][j];
+        const bool ok = piv > tiny || 8 * p + j >= k;
+        const double rt = rsqrt_normal(piv);
+        const double rs = __hiloint2double(ok ? __double2hiint(rt) : 0, ok ? __double2loint(rt) : 0);
+        x[j] *= ok ? rs : 1.0;
+        d[j][j] = ok ? piv * rs : 1.0;
+#pragma unroll
+        for (int l = j + 1; l < 8; ++l) d[j][l] *= rs;
+#pragma unroll
+        for (int i = j + 1; i < 8; ++i) {
+#pragma unroll
+          for (int l = i; l < 8; ++l) d[i][l] = fma(-d[j][i], d[j][l], d[i][l]);
+          x[i] = fma(-d[j][i], x[j], x[i]);
+        }
+      }
+      __syncwarp();
+      if (lane < 8) {
+        double* inv = reinterpret_cast<double*>(D) + me;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) inv[8 * j] = x[j];
+      }
+      __syncwarp();
+      const double2 q = D[lane];
+      if (p + 1 < nb) {
+        if (p > 0) bar_wait<2, 64>();
+        const double2 c = D[32 + lane];
+        double x0 = 0.0, x1 = 0.0;
+        dmma8(x0, x1, c.x, q.x);
+        dmma8(x0, x1, c.y, q.y);
+        D[32 + lane] = make_double2(x0, x1);
+        double2* N = S + col_base(p + 1, nb) * 32 + lane;
+        double2 n = *N;
+        dmma8(n.x, n.y, -x0, x0);
+        dmma8(n.x, n.y, -x1, x1);
+        *N = n;
+        __syncwarp();
+        bar_post<1, 32 + kUpdateThreads>();
+        Rpk[(col_base(p, nb) + 1) * 32 + lane] = make_double2(x0, x1);
+      }
+      Rpk[col_base(p, nb) * 32 + lane] = q;
+      if (write_g && lane < 8) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          if (c == me && 8 * p + c < k) {
+#pragma unroll
+            for (int r = 0; r <= c; ++r) G[8 * p + r + int64_t(8 * p + c) * ldg] = d[r][c];
+          }
+      }
+    }
+  } else if (warp & 3) {
+    const int u = warp - 1 - (warp >> 2);
+    for (int p = 0; p + 1 < nb; ++p) {
+      double2* L = S + (col_base(p, nb) - p) * 32 + lane;  // L_Ip at L[32 I]
+      bar_wait<1, 32 + kUpdateThreads>();
+      const double2 q = L[32 * p];
+      for (int I = p + 2 + u; I < nb; I += kUpdateWarps) {
+        const double2 c = L[32 * I];
+        double x0 = 0.0, x1 = 0.0;
+        dmma8(x0, x1, c.x, q.x);
+        dmma8(x0, x1, c.y, q.y);
+        L[32 * I] = make_double2(x0, x1);
+        Rpk[(col_base(p, nb) + I - p) * 32 + lane] = make_double2(x0, x1);
+      }
+      bar_wait<3, kUpdateThreads>();
+      // the blocks right of the panel in 2 x 2 groups of rows I, I + 1 and columns J, J + 1
+      // (each block of L read once for two products); group 0 holds what warp 0 reads next
+      auto update = [&](int I, int J) {
+        const bool i1 = I + 1 < nb, diag = I == J;
+        const double2 a0 = L[32 * I], a1 = L[32 * (i1 ? I + 1 : I)];
+        const double2 b0 = diag ? a0 : L[32 * J], b1 = diag ? a1 : L[32 * (J + 1)];
+        double2* C0 = S + (col_base(J, nb) + I - J) * 32 + lane;      // (I, J), (I + 1, J)
+        double2* C1 = S + (col_base(J + 1, nb) + I - J) * 32 + lane;  // (I + 1, J + 1) at 0, (I, J + 1) before it
+        if (I > p + 1) {  // (p + 1, p + 1) is warp 0's
+          double2 c = C0[0];
+          dmma8(c.x, c.y, -a0.x, b0.x);
+          dmma8(c.x, c.y, -a0.y, b0.y);
+          C0[0] = c;
+        }
+        if (i1) {
+          double2 c = C0[32], d = C1[0];
+          dmma8(c.x, c.y, -a1.x, b0.x);
+          dmma8(d.x, d.y, -a1.x, b1.x);
+          dmma8(c.x, c.y, -a1.y, b0.y);
+          dmma8(d.x, d.y, -a1.y, b1.y);
+          C0[32] = c;
+          C1[0] = d;
+        }
+        if (!diag) {
+          double2 c = C1[-32];
+          dmma8(c.x, c.y, -a0.x, b1.x);
+          dmma8(c.x, c.y, -a0.y, b1.y);
+          C1[-32] = c;
+        }
+      };
+      if (u == 0 && p + 2 < nb) {
+        update(p + 1, p + 1);
+        bar_post<2, 64>();
+      }
+      // the other groups (i, j), j <= i, row by row, dealt to the warps in turn
+      const int m = (nb - p) / 2;  // groups per side, over the rows p + 1 .. nb - 1
+      int i = 1, j = u == 0 ? kUpdateWarps - 1 : u - 1;
+      for (;;) {
+        while (i < m && j > i) {
+          j -= i + 1;
+          ++i;
+        }
+        if (i >= m) break;
+        update(p + 1 + 2 * i, p + 1 + 2 * j);
+        j += kUpdateWarps;
+      }
+    }
+  }
+  if (write_g) {
+    // R's rows right of the diagonal blocks, and zeros below the diagonal
+    __syncthreads();
+    for (int c = warp; c < k; c += kCpWarps)
+      for (int r = lane; r < k; r += 32) {
+        if (r > c) G[r + int64_t(c) * ldg] = 0.0;
+        else if ((r >> 3) < (c >> 3)) {
+          const double2 q = S[(col_base(r >> 3, nb) + (c >> 3) - (r >> 3)) * 32 + (c & 7) * 4 + ((r & 7) >> 1)];
+          G[r + int64_t(c) * ldg] = (r & 1) ? q.y : q.x;
+        }
+      }
+  }
+}
+
+// Q = Y R^-1: x R = y for eight rows per warp, held as NB accumulator blocks, the
+// current block column in a[0] (the array moves down by one block per step, so the
+// loop's code stays small: executed once, an unrolled one waits for its own
+// instructions).  X_J = T_J R_JJ^-1 with the inverse from R's diagonal block, then
+// X_J times R's block row J is subtracted from the columns after it.  An
+// accumulator block is an A operand as it stands: lane (g, t) holds the columns
+// 2t and 2t + 1.  The CTA's warps beyond those with rows only help to stage R.
+constexpr int kTpThreads = 256;
+
+template <int NB>
+__global__ void __launch_bounds__(kTpThreads) trsm_panel_kernel(const double* __restrict__ Y, int64_t ldy, int64_t N,
+                                                                int k, int warps, const double2* __restrict__ Rpk,
+                                                                double* __restrict__ Q, int64_t ldq) {
+  extern __shared__ __align__(16) double2 Rs[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int nb = (k + 7) >> 3, n2 = nb * (nb + 1) / 2 * 32;
+  const int64_t row = (int64_t(blockIdx.x) * warps + warp) * 8 + g;
+  const bool mine = warp < warps && row < N;
+  double a[NB][2];
+#pragma unroll
+  for (int J = 0; J < NB; ++J)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int c = 8 * J + 2 * t + e;
+      a[J][e] = (mine && c < k) ? Y[row + int64_t(c) * ldy] : 0.0;
+    }
+  // (all of R in flight at once: 16-byte copies that bypass the registers)
+  for (int i = tid; i < n2; i += kTpThreads)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(unsigned(__cvta_generic_to_shared(Rs + i))),
+                 "l"(Rpk + i));
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  if (warp >= warps) return;
+  const double2* R = Rs + lane;
+  for (int J = 0; J < nb; ++J) {
+    const double2 b = R[0];
+    double x0 = 0.0, x1 = 0.0;
+    dmma8(x0, x1, a[0][0], b.x);
+    dmma8(x0, x1, a[0][1], b.y);
+    const int c = 8 * J + 2 * t;
+    if (mine && c < k) Q[row + int64_t(c) * ldq] = x0;
+    if (mine && c + 1 < k) Q[row + int64_t(c + 1) * ldq] = x1;
+    const double m0 = -x0, m1 = -x1;
+    // four blocks at a time, as far as there are any (a group may run over the end of
+    // the block row: what it computes there is not used)
+#pragma unroll
+    for (int K0 = 1; K0 < NB; K0 += 4)
+      if (J + K0 < nb) {
+        double2 q[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) q[i] = R[(K0 + i) * 32];
+#pragma unroll
+        for (int i = 0; i < 4 && K0 + i < NB; ++i)
+          dmma8(a[K0 + i - 1][0], a[K0 + i - 1][1], m0, q[i].x, a[K0 + i][0], a[K0 + i][1]);
+#pragma unroll
+        for (int i = 0; i < 4 && K0 + i < NB; ++i) dmma8(a[K0 + i - 1][0], a[K0 + i - 1][1], m1, q[i].y);
+      }
+    R += (nb - J) * 32;
+  }
+}
+
+SmemAttrOnce g_chol_panel_attr, g_trsm_panel_attr[6];
+
+template <int NB>
+void launch_trsm(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const double* Rpk, double* Q, int64_t ldq) {
+  const size_t pad = 3 * 512;  // a group of four blocks reads over the end
+  const size_t smem = size_t(cholqr_packed(k)) * 8 + pad;
+  g_trsm_panel_attr[NB / 4].ensure(trsm_panel_kernel<NB>, int(size_t(cholqr_packed(8 * NB)) * 8 + pad));
+  // eight rows per warp; one CTA per SM as long as eight warps hold its rows (R is staged once per CTA)
+  const int64_t groups = (N + 7) / 8;
+  const int64_t warps = std::min<int64_t>(kTpThreads / 32, (groups + c.sm_count - 1) / c.sm_count);
+  trsm_panel_kernel<NB><<<unsigned((groups + warps - 1) / warps), kTpThreads, smem, c.stream>>>(
+      Y, ldy, N, k, int(warps), reinterpret_cast<const double2*>(Rpk), Q, ldq);
+}
+
+}  // namespace
+
+bool cholqr_fits(int k) { return k >= 1 && k <= 160; }
+
+int64_t cholqr_packed(int k) {
+  const int64_t nb = (k + 7) / 8;
+  return nb * (nb + 1) / 2 * 64;
+}
+
+void chol_packed(Ctx& c, double* G, int k, int64_t ldg, double shift_factor, double* Rpk, bool write_g) {
+  IPEPS_CHECK(cholqr_fits(k), "chol_packed: k out of range");
+  ProfScope ps(c, KFam::SmallLinalg);
+  g_chol_panel_attr.ensure(chol_panel_kernel, int(size_t(cholqr_packed(160)) * 8));
+  chol_panel_kernel<<<1, kCpThreads, size_t(cholqr_packed(k)) * 8, c.stream>>>(
+      G, k, ldg, shift_factor, reinterpret_cast<double2*>(Rpk), write_g);
+  IPEPS_LAUNCH_CHECK();
+  c.count(KFam::SmallLinalg, double(k) * k * k / 3.0);
+}
+
+void trsm_packed(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const double* Rpk, double* Q, int64_t ldq) {
+  IPEPS_CHECK(cholqr_fits(k), "trsm_packed: k out of range");
+  if (N == 0) return;
+  ProfScope ps(c, KFam::SmallLinalg);
+  switch ((k + 31) / 32) {
+    case 1: launch_trsm<4>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
+    case 2: launch_trsm<8>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
+    case 3: launch_trsm<12>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
+    case 4: launch_trsm<16>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
+    default: launch_trsm<20>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
+  }
+  IPEPS_LAUNCH_CHECK();
+  c.count(KFam::SmallLinalg, double(N) * k * k);
+}
+
+}  // namespace ipeps

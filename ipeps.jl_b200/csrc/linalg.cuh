@@ -29,6 +29,13 @@ bool trsm_fits(int k);
 // Rrow (optional): the same R packed row by row as written by chol_blocked.
 void trsm_right_upper(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const double* R, int64_t ldr,
                       double* Q, int64_t ldq, const double* Rrow = nullptr);
+// The same pass for k <= 160 (cholqr_fits): R in packed 8 x 8 blocks of
+// cholqr_packed(k) doubles (16-byte aligned), the diagonal blocks inverted.  G
+// receives R (strict lower triangle zeroed) when write_g.
+bool cholqr_fits(int k);
+int64_t cholqr_packed(int k);
+void chol_packed(Ctx& c, double* G, int k, int64_t ldg, double shift_factor, double* Rpk, bool write_g);
+void trsm_packed(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const double* Rpk, double* Q, int64_t ldq);
 // jacobi_svd with X held in shared memory and J formed from the logged
 // rotations when it fits; tol <= 0 means m * eps
 void jacobi_svd_auto(Ctx& c, double* X, int m, int k, int64_t ldx, double* J, int64_t ldj, double* S,

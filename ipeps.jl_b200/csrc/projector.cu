@@ -110,15 +110,20 @@ Tensor orth(Ctx& c, const Tensor& Y0, int passes, Tensor* Rout) {
   Tensor Racc;
   double* d_tr = reinterpret_cast<double*>(c.scal->p) + 8;
   const double u = 1.1102230246251565e-16;
-  const bool blocked = chol_fits(k) && trsm_fits(k);
-  Tensor Rrow = blocked ? c.alloc(DType::F64, {int64_t(k) * (k + 1) / 2}) : Tensor();
+  const bool packed = cholqr_fits(k), blocked = !packed && chol_fits(k) && trsm_fits(k);
+  Tensor Rrow = packed    ? c.alloc(DType::F64, {cholqr_packed(k)})
+                : blocked ? c.alloc(DType::F64, {int64_t(k) * (k + 1) / 2})
+                          : Tensor();
   for (int pass = 0; pass < passes; ++pass) {
     // G = Y^T Y  (FP64 always: the Gram matrix is where precision is lost)
     gemm(c, DType::F64, 'T', 'N', k, k, N, cplx(1), Y.data(), N, Y.data(), N, cplx(0), G.data(), k, true);
     // shifted CholeskyQR: the first pass adds 11 (N k + k (k+1)) u trace(G) to the diagonal
     const double sf = (pass == 0) ? 11.0 * (double(N) * k + double(k) * (k + 1)) * u : 0.0;
     Tensor Yn = c.alloc(DType::F64, {N, k});
-    if (blocked) {
+    if (packed) {
+      chol_packed(c, G.f64(), k, k, sf, Rrow.f64(), Rout != nullptr);
+      trsm_packed(c, Y.f64(), N, N, k, Rrow.f64(), Yn.f64(), N);
+    } else if (blocked) {
       chol_blocked(c, G.f64(), k, k, sf, Rrow.f64());
       trsm_right_upper(c, Y.f64(), N, N, k, G.f64(), k, Yn.f64(), N, Rrow.f64());
     } else {

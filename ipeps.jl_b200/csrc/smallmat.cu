@@ -3,10 +3,9 @@
 //   chol_blocked      G = R^T R in one CTA, 32-column panels: one warp factors the
 //                     diagonal block in registers, the block's rows of R are solved
 //                     column-parallel, the trailing update is a register-tiled SYRK.
-//   chol_ldl          the same for k <= 160 with the upper triangle in registers: one
-//                     barrier per elimination step.
 //   trsm_right_upper  Q = Y R^-1, two rows of Y per warp (the rows are independent), at
 //                     most one CTA per SM, R staged row-major in each CTA's shared memory.
+//                     (Both for k > 160; sketches of up to 160 columns: cholqr.cu.)
 //   jacobi_svd_auto   one-sided Jacobi with only X in shared memory; every rotation is
 //                     logged, and J = product of the rotations is formed afterwards by a
 //                     row-parallel kernel (each row of J sees the same rotation sequence).
@@ -202,171 +201,6 @@ __global__ void __launch_bounds__(kCholThreads) chol_blocked_kernel(double* G, i
     for (int i = lane; i < k; i += 32) G[i + int64_t(j) * ldg] = (i <= j) ? P[pku(i, j)] : 0.0;
   if (Rrow)
     for (int i = warp; i < k; i += nw)
-      for (int jj = lane; jj < k - i; jj += 32) Rrow[rowoff(i, k) + jj] = P[pku(i, i + jj)];
-}
-
-// Register-resident Cholesky for k <= 32 NBB (NBB <= 5), same contract as
-// chol_blocked_kernel.  The right-looking elimination is written as
-// G = U^T D U (U unit upper): step j subtracts a[j][r] a[j][c] / a[j][j] from
-// every a[r][c] with c >= r > j, and R = D^1/2 U at the end.  512 threads
-// hold the upper triangle in registers, thread (w, l) of warp w and lane l the
-// entries (w + 16 a, l + 32 b) (slots a <= 2b + 1 can reach the triangle), so a
-// step costs one barrier: the warp owning row j publishes the row and the row
-// divided by the pivot in shared memory (double-buffered by the parity of j),
-// and every thread updates its slots from two broadcast loads per row and
-// one load per column block.
-constexpr int kLdlThreads = 512;
-
-size_t chol_ldl_smem_doubles(int k) {
-  const size_t npk = (size_t(k) * (k + 1) / 2 + 1) & ~size_t(1);
-  return npk + 4 * 160 + 2 * 160 + 8;
-}
-
-// Publishes row j (16 JB <= j < 16 JB + 16, held in slot a = JB of the calling
-// warp): a[j][c] (c >= j) into rw, a[j][c] / a[j][j] (c > j) into sc, the
-// pivot into dd[j] (0 for a failed pivot).
-template <int NBB, int JB>
-__device__ __forceinline__ void ldl_publish(const double (&v)[2 * NBB][NBB], int j, int k, int lane, double* rw,
-                                            double* sc, double* dd, double tiny) {
-  constexpr int B0 = JB / 2;
-  // the pivot a[j][j] sits in column block JB / 2 of lane j mod 32
-  const double d = __shfl_sync(kFull, v[JB][B0], j & 31);
-  const bool ok = d > tiny;
-  const double inv = ok ? __drcp_rn(d) : 0.0;
-#pragma unroll
-  for (int b = B0; b < NBB; ++b) {
-    const int c = lane + 32 * b;
-    if (c >= j && c < k) {
-      rw[c] = v[JB][b];
-      if (c > j) sc[c] = v[JB][b] * inv;
-    }
-  }
-  if (lane == 0) dd[j] = ok ? d : 0.0;
-}
-
-// Elimination steps j = 16 JB .. 16 JB + 15 of chol_ldl_kernel, then the next
-// block of 16 (JB is a compile-time constant, so the slots of rows that are
-// finished, a < JB, and of column blocks left of every pivot of the block,
-// 32 b + 31 <= 16 JB, drop out of the code instead of being tested per step).
-// Step j: the warp holding row j (warp j mod 16, slot a = JB) publishes it in
-// shared memory, double-buffered by the parity of j, and after the barrier
-// every slot of a row r > j takes a[r][c] -= a[j][r] (a[j][c] / a[j][j]).
-// Slots left of the diagonal take stale buffer entries and are never read.
-// (Publishing row j + 1 during step j, as soon as its warp has updated it,
-// measured no faster: the steps are bound by the barrier and the shared-memory
-// broadcasts, not by the pivot's reciprocal.)
-template <int NBB, int JB>
-__device__ __forceinline__ void ldl_steps(double (&v)[2 * NBB][NBB], int k, int warp, int lane, double* raw,
-                                          double* scl, double* dd, double tiny) {
-  constexpr int NBA = 2 * NBB, KP = 32 * NBB, B0 = JB / 2;
-  const int tmax = min(16, k - 16 * JB);
-  for (int t = 0; t < tmax; ++t) {
-    const int j = 16 * JB + t;
-    double* rw = raw + (t & 1) * KP;
-    double* sc = scl + (t & 1) * KP;
-    if (warp == t) ldl_publish<NBB, JB>(v, j, k, lane, rw, sc, dd, tiny);
-    __syncthreads();
-    double s[NBB];
-#pragma unroll
-    for (int b = B0; b < NBB; ++b) s[b] = sc[lane + 32 * b];
-    if (warp > t) {  // slot a = JB holds row 16 JB + warp > j
-      const double ra = rw[16 * JB + warp];
-#pragma unroll
-      for (int b = B0; b < NBB; ++b) v[JB][b] = fma(-ra, s[b], v[JB][b]);
-    }
-#pragma unroll
-    for (int a = JB + 1; a < NBA; ++a) {
-      const double ra = rw[warp + 16 * a];
-#pragma unroll
-      for (int b = B0; b < NBB; ++b) {
-        if (a > 2 * b + 1) continue;
-        v[a][b] = fma(-ra, s[b], v[a][b]);
-      }
-    }
-  }
-  if constexpr (JB + 1 < NBA) ldl_steps<NBB, JB + 1>(v, k, warp, lane, raw, scl, dd, tiny);
-}
-
-template <int NBB>
-__global__ void __launch_bounds__(kLdlThreads, 1) chol_ldl_kernel(double* G, int k, int64_t ldg, double shift_factor,
-                                                                double* Rrow) {
-  constexpr int NBA = 2 * NBB, KP = 32 * NBB;
-  extern __shared__ __align__(16) double sm[];
-  const int npk = ((k * (k + 1)) / 2 + 1) & ~1;
-  double* P = sm;             // packed upper triangle, column by column
-  double* raw = P + npk;      // [2][KP]: row j of the eliminated matrix
-  double* scl = raw + 2 * KP; // [2][KP]: the same divided by the pivot (0 for a failed pivot)
-  double* dd = scl + 2 * KP;  // pivots (0: failed)
-  double* rs = dd + KP;       // 1 / sqrt(pivot), 0 for a failed pivot
-  __shared__ double s_red[kLdlThreads / 32];
-  __shared__ double s_tr;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
-  {
-    constexpr int kU = 4;
-    const int kk2 = k * k;
-    for (int t0 = tid; t0 < kk2; t0 += kU * kLdlThreads) {
-      double v[kU];
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const int t = t0 + u * kLdlThreads, i = t % k, j = t / k;
-        v[u] = (t < kk2 && i <= j) ? G[i + int64_t(j) * ldg] : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const int t = t0 + u * kLdlThreads, i = t % k, j = t / k;
-        if (t < kk2 && i <= j) P[pku(i, j)] = v[u];
-      }
-    }
-    for (int t = tid; t < 4 * KP; t += kLdlThreads) raw[t] = 0.0;  // raw and scl, rows >= k stay 0
-  }
-  __syncthreads();
-  double t = 0;
-  for (int i = tid; i < k; i += kLdlThreads) t += fabs(P[pku(i, i)]);
-  for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
-  if (lane == 0) s_red[warp] = t;
-  __syncthreads();
-  if (tid == 0) {
-    double s = 0;
-    for (int w = 0; w < kLdlThreads / 32; ++w) s += s_red[w];
-    s_tr = s;
-  }
-  __syncthreads();
-  const double shift = shift_factor > 0 ? shift_factor * s_tr : 0.0;
-  const double tiny = 1e-300 + 1e-32 * (s_tr + shift * k);
-
-  double v[NBA][NBB];
-#pragma unroll
-  for (int a = 0; a < NBA; ++a)
-#pragma unroll
-    for (int b = 0; b < NBB; ++b) {
-      if (a > 2 * b + 1) continue;
-      const int r = warp + 16 * a, c = lane + 32 * b;
-      double x = (r <= c && c < k) ? P[pku(r, c)] : 0.0;
-      if (r == c) x += shift;
-      v[a][b] = x;
-    }
-
-  ldl_steps<NBB, 0>(v, k, warp, lane, raw, scl, dd, tiny);
-  for (int i = tid; i < k; i += kLdlThreads) rs[i] = dd[i] > 0.0 ? rsqrt(dd[i]) : 0.0;
-  __syncthreads();
-  // R = D^1/2 U into P; a failed pivot gives R[j][j] = 1 and row j zero
-#pragma unroll
-  for (int a = 0; a < NBA; ++a)
-#pragma unroll
-    for (int b = 0; b < NBB; ++b) {
-      if (a > 2 * b + 1) continue;
-      const int r = warp + 16 * a, c = lane + 32 * b;
-      if (r <= c && c < k) {
-        const double q = rs[r];
-        P[pku(r, c)] = (r == c) ? (q > 0.0 ? dd[r] * q : 1.0) : v[a][b] * q;
-      }
-    }
-  __syncthreads();
-  for (int j = warp; j < k; j += kLdlThreads / 32)
-    for (int i = lane; i < k; i += 32) G[i + int64_t(j) * ldg] = (i <= j) ? P[pku(i, j)] : 0.0;
-  if (Rrow)
-    for (int i = warp; i < k; i += kLdlThreads / 32)
       for (int jj = lane; jj < k - i; jj += 32) Rrow[rowoff(i, k) + jj] = P[pku(i, i + jj)];
 }
 
@@ -673,14 +507,7 @@ __global__ void __launch_bounds__(kApplyRows * 32) jacobi_apply_kernel(const dou
 }
 
 // shared-memory opt-in, once per kernel and device
-SmemAttrOnce g_chol_attr, g_ldl_attr[6], g_trsm_attr[9], g_jlog_attr[11], g_apply_attr;
-
-template <int NBB>
-void launch_ldl(Ctx& c, double* G, int k, int64_t ldg, double shift_factor, double* Rrow) {
-  const size_t smem = chol_ldl_smem_doubles(k) * 8;
-  g_ldl_attr[NBB].ensure(chol_ldl_kernel<NBB>, int(kSmemMax));
-  chol_ldl_kernel<NBB><<<1, kLdlThreads, smem, c.stream>>>(G, k, ldg, shift_factor, Rrow);
-}
+SmemAttrOnce g_chol_attr, g_trsm_attr[9], g_jlog_attr[11], g_apply_attr;
 
 template <int NV>
 void launch_jacobi(Ctx& c, double* X, int m, int k, int64_t ldx, double2* rot, int max_sweeps, double tol, double* S,
@@ -704,40 +531,25 @@ void launch_trsm(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const d
 
 }  // namespace
 
-bool chol_fits(int k) { return k >= 1 && chol_smem_doubles(k) * 8 <= kSmemMax; }
+bool chol_fits(int k) { return k > 160 && chol_smem_doubles(k) * 8 <= kSmemMax; }
 
 void chol_blocked(Ctx& c, double* G, int k, int64_t ldg, double shift_factor, double* Rrow) {
-  IPEPS_CHECK(chol_fits(k), "chol_blocked: k too large for shared memory");
+  IPEPS_CHECK(chol_fits(k), "chol_blocked: k out of range");
   ProfScope ps(c, KFam::SmallLinalg);
-  if (k <= 160 && chol_ldl_smem_doubles(k) * 8 <= kSmemMax) {
-    switch ((k + 31) / 32) {
-      case 1: launch_ldl<1>(c, G, k, ldg, shift_factor, Rrow); break;
-      case 2: launch_ldl<2>(c, G, k, ldg, shift_factor, Rrow); break;
-      case 3: launch_ldl<3>(c, G, k, ldg, shift_factor, Rrow); break;
-      case 4: launch_ldl<4>(c, G, k, ldg, shift_factor, Rrow); break;
-      default: launch_ldl<5>(c, G, k, ldg, shift_factor, Rrow); break;
-    }
-  } else {
-    g_chol_attr.ensure(chol_blocked_kernel, int(kSmemMax));
-    chol_blocked_kernel<<<1, kCholThreads, chol_smem_doubles(k) * 8, c.stream>>>(G, k, ldg, shift_factor, Rrow);
-  }
+  g_chol_attr.ensure(chol_blocked_kernel, int(kSmemMax));
+  chol_blocked_kernel<<<1, kCholThreads, chol_smem_doubles(k) * 8, c.stream>>>(G, k, ldg, shift_factor, Rrow);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::SmallLinalg, double(k) * k * k / 3.0);
 }
 
-bool trsm_fits(int k) { return k >= 1 && k <= 256 && trsm_smem_bytes(k, trsm_warps(k)) <= kSmemMax; }
+bool trsm_fits(int k) { return k > 160 && k <= 256 && trsm_smem_bytes(k, trsm_warps(k)) <= kSmemMax; }
 
 void trsm_right_upper(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const double* R, int64_t ldr, double* Q,
                       int64_t ldq, const double* Rrow) {
-  IPEPS_CHECK(trsm_fits(k), "trsm_right_upper: k too large for shared memory");
+  IPEPS_CHECK(trsm_fits(k), "trsm_right_upper: k out of range");
   if (N == 0) return;
   ProfScope ps(c, KFam::SmallLinalg);
   switch ((k + 31) / 32) {
-    case 1: launch_trsm<1>(c, Y, ldy, N, k, R, ldr, Rrow, Q, ldq); break;
-    case 2: launch_trsm<2>(c, Y, ldy, N, k, R, ldr, Rrow, Q, ldq); break;
-    case 3: launch_trsm<3>(c, Y, ldy, N, k, R, ldr, Rrow, Q, ldq); break;
-    case 4: launch_trsm<4>(c, Y, ldy, N, k, R, ldr, Rrow, Q, ldq); break;
-    case 5: launch_trsm<5>(c, Y, ldy, N, k, R, ldr, Rrow, Q, ldq); break;
     case 6: launch_trsm<6>(c, Y, ldy, N, k, R, ldr, Rrow, Q, ldq); break;
     case 7: launch_trsm<7>(c, Y, ldy, N, k, R, ldr, Rrow, Q, ldq); break;
     default: launch_trsm<8>(c, Y, ldy, N, k, R, ldr, Rrow, Q, ldq); break;

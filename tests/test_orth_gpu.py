@@ -57,3 +57,21 @@ def test_orth_ill_conditioned_and_rank_deficient(engine, pkg, k):
     assert np.isfinite(Q).all() and np.isfinite(R).all()
     assert np.abs(Q.T @ Q - np.eye(k)).max() <= 1e-10  # a CPU restatement gives 1.3e-11 at k = 160
     assert np.linalg.norm(Yr - Q @ (Q.T @ Yr)) <= 1e-13 * np.linalg.norm(Yr)
+
+
+@pytest.mark.parametrize("N,k", [(1, 1), (7, 7), (8, 8), (40, 9), (33, 16), (129, 24), (120, 62), (333, 76), (97, 97),
+                                 (1201, 104), (160, 159), (3000, 160), (170, 161)])
+def test_orth_block_edges(engine, pkg, N, k):
+    """Panel edges of the blocked Cholesky and triangular solve (8 columns, 8 rows; k <= 160 and the
+    first k beyond), square Y among them.  Bars: two unshifted CholeskyQR passes after the shifted one
+    leave rounding, 10 k eps in Q^T Q and in Q R = Y; R against the Cholesky factor of Y^T Y (64-bit,
+    backward stable) differs by its conditioning, 100 k eps cond(Y)^2."""
+    rng = np.random.default_rng(N * 1000 + k)
+    Y = rng.standard_normal((N, k)) + (4.0 * N ** 0.5 * np.eye(N, k) if N < 2 * k else 0.0)
+    eps = np.finfo(float).eps
+    Q, R = pkg.orth(Y, 3, engine=engine)
+    assert np.abs(Q.T @ Q - np.eye(k)).max() <= 10 * k * eps
+    assert np.linalg.norm(Q @ R - Y) <= 10 * k * eps * np.linalg.norm(Y)
+    assert np.array_equal(np.tril(R, -1), np.zeros((k, k)))
+    ref = np.linalg.cholesky(Y.T @ Y).T
+    assert np.linalg.norm(R - ref) <= 100 * k * eps * np.linalg.cond(Y) ** 2 * np.linalg.norm(ref)
