@@ -59,6 +59,12 @@ struct Ctx {
   // small device scalars (max-abs, traces, status words)
   std::shared_ptr<DBuf> scal;
   int* d_status = nullptr;
+  // tile configuration and K split of the FP64 GEMM by (m, n, k, upper): chosen
+  // from an estimate over all of them, so kept (bounded: emptied at 4096 shapes)
+  struct GemmPlan {
+    int config = 0, S = 1, cs = 1;
+  };
+  std::map<std::tuple<int64_t, int64_t, int64_t, bool>, GemmPlan> gemm_plans;
   // per-kernel-family CUDA-event timing (enabled by ipeps_prof_enable)
   bool prof = false;
   // with prof: wall ms of the E+grad pullback's phases (checkpoint iterations,
@@ -157,9 +163,11 @@ void gemm(Ctx& c, DType dt, char opA, char opB, int64_t m, int64_t n, int64_t k,
 void gemm_f64(Ctx& c, DType dt, char opA, char opB, int64_t m, int64_t n, int64_t k,
               cuDoubleComplex alpha, const void* A, int64_t lda, const void* B, int64_t ldb,
               cuDoubleComplex beta, void* C, int64_t ldc);
-// real FP64 GEMM on the DMMA (FP64 tensor-core) path, op in {N, T}
+// real FP64 GEMM on the DMMA (FP64 tensor-core) path, op in {N, T}; upper: C is symmetric and only its
+// upper triangle is needed (entries below the diagonal are left undefined)
 void gemm_f64_dmma(Ctx& c, char opA, char opB, int64_t m, int64_t n, int64_t k, double alpha, const double* A,
-                   int64_t lda, const double* B, int64_t ldb, double beta, double* C, int64_t ldc);
+                   int64_t lda, const double* B, int64_t ldb, double beta, double* C, int64_t ldc,
+                   bool upper = false);
 // 3xTF32 tcgen05 GEMM for real operands (FP32-accumulated split products)
 // BF16 operands (rounded from FP32 while staged), FP32 accumulation and result; op in {N, T}
 void gemm_bf16(Ctx& c, char opA, char opB, int64_t m, int64_t n, int64_t k, float alpha, const float* A, int64_t lda,
@@ -181,8 +189,9 @@ void gemm_tf32x3(Ctx& c, char opA, char opB, int64_t m, int64_t n, int64_t k, do
                  const double* A, int64_t lda, const double* B, int64_t ldb, double beta, double* C,
                  int64_t ldc);
 
-// whether the mixed form runs an m x n x k product as 3xTF32 (else in FP64)
-bool tf32x3_pays(int64_t m, int64_t n, int64_t k);
+// whether the mixed form runs an m x n x k product as 3xTF32 (else in FP64); planes_kept:
+// its large operand is split already
+bool tf32x3_pays(int64_t m, int64_t n, int64_t k, bool planes_kept = false);
 
 inline cuDoubleComplex cplx(double r, double i = 0) { return make_cuDoubleComplex(r, i); }
 

@@ -37,8 +37,8 @@ const Planes& planes_col(Ctx& c, const Tensor& Rt, PlaneCache* pc) {
 }
 
 bool use_planes(const Ctx& c, const MatRef& R, const PlaneCache* pc, int64_t cols) {
-  return pc && c.precision == kPrecMixed && R.t.dt == DType::F64 && tf32x3_pays(R.rows(), cols, R.cols()) &&
-         tf32x3_pays(R.cols(), cols, R.rows());
+  return pc && c.precision == kPrecMixed && R.t.dt == DType::F64 && tf32x3_pays(R.rows(), cols, R.cols(), true) &&
+         tf32x3_pays(R.cols(), cols, R.rows(), true);
 }
 
 }  // namespace
@@ -115,8 +115,9 @@ Tensor orth(Ctx& c, const Tensor& Y0, int passes, Tensor* Rout) {
                 : blocked ? c.alloc(DType::F64, {int64_t(k) * (k + 1) / 2})
                           : Tensor();
   for (int pass = 0; pass < passes; ++pass) {
-    // G = Y^T Y  (FP64 always: the Gram matrix is where precision is lost)
-    gemm(c, DType::F64, 'T', 'N', k, k, N, cplx(1), Y.data(), N, Y.data(), N, cplx(0), G.data(), k, true);
+    // G = Y^T Y  (FP64 always: the Gram matrix is where precision is lost), its upper triangle: all
+    // that the Cholesky kernels read
+    gemm_f64_dmma(c, 'T', 'N', k, k, N, 1.0, Y.f64(), N, Y.f64(), N, 0.0, G.f64(), k, true);
     // shifted CholeskyQR: the first pass adds 11 (N k + k (k+1)) u trace(G) to the diagonal
     const double sf = (pass == 0) ? 11.0 * (double(N) * k + double(k) * (k + 1)) * u : 0.0;
     Tensor Yn = c.alloc(DType::F64, {N, k});

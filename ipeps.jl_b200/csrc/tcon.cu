@@ -207,13 +207,14 @@ Tensor matmul(Ctx& c, const Tensor& A, char opA, const Tensor& B, char opB) {
 // Which products of the mixed form run as 3xTF32.  Measured per product on B200
 // (splits and split-K sums included): splitting both operands and the pipeline's
 // start cost 20-30 us whatever the size, and the split moves 24 bytes per operand
-// element, so the FP64 kernel is the faster one below ~0.4 GFLOP (1024 x 130 x
-// 1024, 0.27 GFLOP: 28 us against 31; 1450 x 118 x 1450, 0.50 GFLOP: 39 against
-// 34; 2500 x 160 x 2500: 112 against 58) and, at any size, for short inner
-// dimensions (250000 x 50 x 25: 63 us against 89; 1450 x 1450 x 58: 20 against
-// 33; 1975 x 1975 x 79: 39 against 31).
-bool tf32x3_pays(int64_t m, int64_t n, int64_t k) {
-  return k >= 64 && 2.0 * double(m) * double(n) * double(k) >= 4e8;
+// element, so the FP64 kernel is the faster one below ~0.9 GFLOP (1450 x 118 x
+// 1450, 0.50 GFLOP: 29 us against 34; 2250 x 2250 x 90, 0.91 GFLOP: 48 against 47;
+// 2500 x 160 x 2500, 2 GFLOP: 84 against 58) and, at any size, for short inner
+// dimensions (250000 x 50 x 25: 62 us against 88).  planes_kept: the large operand's
+// split is shared by all products of a projector (0.4 GFLOP: about the split of
+// 1150 x 1150, 10 us, less).
+bool tf32x3_pays(int64_t m, int64_t n, int64_t k, bool planes_kept) {
+  return k >= 64 && 2.0 * double(m) * double(n) * double(k) >= (planes_kept ? 4e8 : 9e8);
 }
 
 void gemm(Ctx& c, DType dt, char opA, char opB, int64_t m, int64_t n, int64_t k,

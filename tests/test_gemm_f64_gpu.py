@@ -63,3 +63,28 @@ def test_gemm_f64_split_k_is_deterministic(engine, pkg):
     ref = A.T @ B
     bound = 2 * 2500 * EPS * (np.abs(A.T) @ np.abs(B))
     assert np.all(np.abs(outs[0] - ref) <= bound)
+
+
+@pytest.mark.parametrize("op", ["NN", "TN", "NT", "TT"])
+@pytest.mark.parametrize("m,n,k,beta", [
+    (33, 31, 65, 0.0),      # a 32 x 32 tile and its remainders, two K chunks at most
+    (120, 62, 120, 0.5),    # 32 x 32 tiles in clusters of three
+    (37, 37, 333, 0.0),     # clusters of seven, odd leading dimensions (8-byte copies)
+    (65, 33, 1000, -1.0),   # 64 x 32 tiles' remainders, clusters of eight
+    (9, 18, 12321, 0.0),    # more than one cluster per tile: sums through the workspace
+    (17, 23, 40001, 2.0),   # the same with a remainder in K and beta
+    (2500, 79, 1111, 0.0),  # one 80-column tile, partial sums without clusters
+    (300, 900, 5, 1.0),     # less than one K step
+])
+def test_gemm_f64_tiles_and_splits(engine, pkg, op, m, n, k, beta):
+    """Every tile configuration and way of summing the K chunks, with remainders; bound as above."""
+    rng = np.random.default_rng(m + 3 * n + 7 * k)
+    A = np.asfortranarray(rng.standard_normal((m, k) if op[0] == "N" else (k, m)))
+    B = np.asfortranarray(rng.standard_normal((k, n) if op[1] == "N" else (n, k)))
+    C = rng.standard_normal((m, n))
+    a, b = (A if op[0] == "N" else A.T), (B if op[1] == "N" else B.T)
+    out = pkg.host.gemm_f64(op[0], op[1], A, B, alpha=1.25, beta=beta, C=C, engine=engine)
+    bound = 2 * k * EPS * 1.25 * (np.abs(a) @ np.abs(b)) + 2 * EPS * np.abs(beta * C) + 1e-300
+    assert np.all(np.abs(out - (1.25 * (a @ b) + beta * C)) <= bound)
+    again = pkg.host.gemm_f64(op[0], op[1], A, B, alpha=1.25, beta=beta, C=C, engine=engine)
+    assert np.array_equal(out, again)
