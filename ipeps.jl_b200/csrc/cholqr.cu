@@ -52,17 +52,6 @@ __device__ __forceinline__ void bar_post() {
   asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(N) : "memory");
 }
 
-// 1 / sqrt(d) of a normal d > 0 (anything else: unspecified), within 2 ulp: the
-// hardware estimate y and one third-order step of the series of (1 - e)^(-1/2),
-// e = 1 - d y^2 (Householder's method).  Without rsqrt's cases the compiler is free
-// to fill the pivots' chain with the independent products around it.
-__device__ __forceinline__ double rsqrt_normal(double d) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  const double e = fma(-d * y, y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 // Packed upper block triangle of R, block row by block row: block (I, J) at
 // col_base(I) + J - I.  Inside a block the entries (2t, g) and (2t + 1, g) are
 // neighbours, at 2 (8 t + g): lane (g, t) of a warp then has with one 16-byte
@@ -147,7 +136,7 @@ __global__ void __launch_bounds__(kCpThreads, 1)
       for (int j = 0; j < 8; ++j) {
         const double piv = d[j][j];
         const bool ok = piv > tiny || 8 * p + j >= k;
-        const double rt = rsqrt_normal(piv);
+        const double rt = rsqrt_normal(piv);  // (without rsqrt's cases the chain's shadow is filled)
         const double rs = __hiloint2double(ok ? __double2hiint(rt) : 0, ok ? __double2loint(rt) : 0);
         x[j] *= ok ? rs : 1.0;
         d[j][j] = ok ? piv * rs : 1.0;

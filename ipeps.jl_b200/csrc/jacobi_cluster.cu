@@ -26,16 +26,17 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-constexpr int kJP = 8;                 // CTAs per cluster (portable cluster size)
+constexpr int kJP = 8;                 // CTAs per cluster (portable cluster size; 16: 508 us instead of 556 at k = 160,
+                                       // slower below k = 128)
 constexpr int kJBlocks = 2 * kJP;      // column blocks
 constexpr int kJWarps = 16;            // warps per CTA (>= b)
-constexpr int kJMaxRowsPerLane = 16;   // H <= 512
+constexpr int kJMaxRowsPerLane = 16;   // height of [X; J] <= 512
 constexpr size_t kJSmemMax = 200 * 1024;
 
 struct JcArgs {
   const double* X;
   int64_t ldx;
-  int m, k, b, H;  // rows of X, columns, block width (even), padded height of [X; J]
+  int m, k, b;  // rows of X, columns, block width
   int max_sweeps;
   double tol2;
   double* Xout;
@@ -68,67 +69,76 @@ __device__ __forceinline__ void pos_owner(int p, int& rank, int& slot) {
   }
 }
 
-// rotate columns u (registers) and the shared column y; returns true when it rotated
-__device__ __forceinline__ bool rotate_pair(double (&u)[kJMaxRowsPerLane], double* y, int m, int H, int lane,
-                                            double tol2) {
-  double v[kJMaxRowsPerLane];
-  double a = 0, bb = 0, c = 0;
+// Rotates column u (registers, squared norm nu) against the shared column y
+// (squared norm *ny); true when it rotated.  The dot product runs over the rows of
+// X only (nx of the NR rows per lane), the rotation over those of [X; J].
+template <int NR>
+__device__ __forceinline__ bool rotate_pair(double (&u)[NR], double& nu, double* y, double* ny, int m, int nx, int H,
+                                            int lane, double tol2) {
+  double v[NR];
+  double c0 = 0, c1 = 0;
+  const double nv = *ny;
 #pragma unroll
-  for (int j = 0; j < kJMaxRowsPerLane; ++j) {
-    const int r = lane + 32 * j;
-    v[j] = (r < H) ? y[r] : 0.0;
-    if (r < m) {
-      a = fma(u[j], u[j], a);
-      bb = fma(v[j], v[j], bb);
-      c = fma(u[j], v[j], c);
+  for (int j = 0; j < NR; ++j) v[j] = y[lane + 32 * j];
+#pragma unroll
+  for (int j = 0; j < NR; ++j)
+    if (j < nx) {
+      const double w = lane + 32 * j < m ? v[j] : 0.0;
+      if (j & 1) c1 = fma(u[j], w, c1);
+      else c0 = fma(u[j], w, c0);
     }
-  }
+  double c = c0 + c1;
 #pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    a += __shfl_xor_sync(0xffffffffu, a, o);
-    bb += __shfl_xor_sync(0xffffffffu, bb, o);
-    c += __shfl_xor_sync(0xffffffffu, c, o);
-  }
-  if (!(c != 0.0 && a > 0.0 && bb > 0.0 && c * c > tol2 * (a * bb))) return false;
-  const double d = bb - a;
-  const double rho = rsqrt(fma(d, d, 4.0 * c * c));
+  for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  if (!(c != 0.0 && nu > 0.0 && nv > 0.0 && c * c > tol2 * (nu * nv))) return false;
+  const double d = nv - nu;
+  const double rho = rsqrt_normal(fma(d, d, 4.0 * c * c));
   const double c2 = fabs(d) * rho, s2 = copysign(1.0, d) * (2.0 * c * rho);
   const double uu = 0.5 * (1.0 + c2);
-  const double ru = rsqrt(uu);
+  const double ru = rsqrt_normal(uu);
   const double cs = uu * ru, sn = 0.5 * s2 * ru;
 #pragma unroll
-  for (int j = 0; j < kJMaxRowsPerLane; ++j) {
-    const int r = lane + 32 * j;
+  for (int j = 0; j < NR; ++j) {
     const double up = cs * u[j] - sn * v[j], vq = sn * u[j] + cs * v[j];
     u[j] = up;
-    if (r < H) y[r] = vq;
+    y[lane + 32 * j] = vq;
   }
+  const double tc = 0.5 * s2 * c * (ru * ru);  // tan(t) * c
+  nu -= tc;
+  if (lane == 0) *ny = nv + tc;
   return true;
 }
 
-__device__ __forceinline__ void load_col(double (&u)[kJMaxRowsPerLane], const double* x, int H, int lane) {
+template <int NR>
+__device__ __forceinline__ void load_col(double (&u)[NR], const double* x, int lane) {
 #pragma unroll
-  for (int j = 0; j < kJMaxRowsPerLane; ++j) {
-    const int r = lane + 32 * j;
-    u[j] = (r < H) ? x[r] : 0.0;
-  }
+  for (int j = 0; j < NR; ++j) u[j] = x[lane + 32 * j];
 }
 
-__device__ __forceinline__ void store_col(const double (&u)[kJMaxRowsPerLane], double* x, int H, int lane) {
+template <int NR>
+__device__ __forceinline__ void store_col(const double (&u)[NR], double* x, int lane) {
 #pragma unroll
-  for (int j = 0; j < kJMaxRowsPerLane; ++j) {
-    const int r = lane + 32 * j;
-    if (r < H) x[r] = u[j];
-  }
+  for (int j = 0; j < NR; ++j) x[lane + 32 * j] = u[j];
 }
 
+// NR: rows of [X; J] per lane, H = 32 NR.  Bound by the latency of a sub-round (load,
+// dot product, reduction, angle, store, barrier: ~0.8 us at k = 160) and of the
+// exchange between rounds (~1.1 us).  A pair costs 5 NR / 2 FP64 instructions per
+// lane: the dot product runs over the rows of X, the squared norms are carried
+// (recomputed every sweep) and exchanged with the blocks.  Four sweeps, before (16
+// rows per lane whatever the size, norms from every pair, even block widths) -> now:
+// k = 62 244 -> 128 us, k = 98 587 -> 288, k = 128 588 -> 336, k = 160 888 -> 556.
+template <int NR>
 __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) jacobi_cluster_kernel(JcArgs a) {
   extern __shared__ __align__(16) double jsm[];
   cg::cluster_group cluster = cg::this_cluster();
+  constexpr int H = 32 * NR;
   const int rank = int(cluster.block_rank());
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int b = a.b, H = a.H, m = a.m;
-  const size_t slot_sz = size_t(b) * H;
+  const int b = a.b, m = a.m, nx = (a.m + 31) >> 5;
+  // a slot: b columns of H rows, then their squared norms
+  const int be = (b + 1) & ~1;  // players of the round robin inside a block (b odd: one sits out)
+  const size_t slot_sz = size_t(b) * H + be;
   // buf[cur][slot] columns, then the block ids of the slots per buffer, then the flags
   double* buf = jsm;
   int* blk = reinterpret_cast<int*>(jsm + 4 * slot_sz);  // [2 buffers][2 slots]
@@ -160,22 +170,35 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
   bool converged = false;
   for (; sweep < a.max_sweeps && !converged; ++sweep) {
     if (tid == 0) s_rot = 0;
+    for (int j = warp; j < 2 * b; j += kJWarps) {
+      double* S = buf + (cur * 2 + (j >= b)) * slot_sz;
+      const int jj = j >= b ? j - b : j;
+      double n = 0;
+      for (int r = lane; r < m; r += 32) n = fma(S[jj * H + r], S[jj * H + r], n);
+#pragma unroll
+      for (int o = 16; o; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+      if (lane == 0) S[size_t(b) * H + jj] = n;
+    }
     __syncthreads();
     bool rot = false;
     for (int round = 0; round < kJBlocks - 1; ++round) {
       double* A = buf + (cur * 2 + 0) * slot_sz;
       double* B = buf + (cur * 2 + 1) * slot_sz;
+      double *nA = A + size_t(b) * H, *nB = B + size_t(b) * H;
       if (round == 0) {
-        // pairs inside each block: b - 1 sub-rounds of b/2 pairs per block
-        for (int t = 0; t < b - 1; ++t) {
-          for (int w = warp; w < b; w += kJWarps) {
-            double* base = (w < b / 2) ? A : B;
+        // pairs inside each block: be - 1 sub-rounds of be/2 pairs per block
+        for (int t = 0; t < be - 1; ++t) {
+          for (int w = warp; w < be; w += kJWarps) {
+            double* base = (w < be / 2) ? A : B;
+            double* nb = (w < be / 2) ? nA : nB;
             int p, q;
-            circle_pair(w % (b / 2), t, b, p, q);
-            double u[kJMaxRowsPerLane];
-            load_col(u, base + size_t(p) * H, H, lane);
-            if (rotate_pair(u, base + size_t(q) * H, m, H, lane, a.tol2)) {
-              store_col(u, base + size_t(p) * H, H, lane);
+            circle_pair(w % (be / 2), t, be, p, q);
+            if (p >= b || q >= b) continue;
+            double u[NR], nu = nb[p];
+            load_col<NR>(u, base + size_t(p) * H, lane);
+            if (rotate_pair<NR>(u, nu, base + size_t(q) * H, nb + q, m, nx, H, lane, a.tol2)) {
+              store_col<NR>(u, base + size_t(p) * H, lane);
+              if (lane == 0) nb[p] = nu;
               rot = true;
             }
           }
@@ -183,17 +206,20 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
         }
       }
       // pairs between the two blocks: warp i keeps column A_i, meets B_{(i+t) % b}
-      for (int i = warp; i < b; i += kJWarps) {
-        double u[kJMaxRowsPerLane];
-        load_col(u, A + size_t(i) * H, H, lane);
+      if (warp < b) {
+        double u[NR], nu = nA[warp];
+        load_col<NR>(u, A + size_t(warp) * H, lane);
         bool any = false;
+        int q = warp;
         for (int t = 0; t < b; ++t) {
           // B columns are touched by one warp per sub-round: sync the warps that share them
-          if (rotate_pair(u, B + size_t((i + t) % b) * H, m, H, lane, a.tol2)) any = true;
-          asm volatile("bar.sync 1, %0;" ::"r"(((b + 0) < kJWarps ? b : kJWarps) * 32) : "memory");
+          if (rotate_pair<NR>(u, nu, B + size_t(q) * H, nB + q, m, nx, H, lane, a.tol2)) any = true;
+          q = q + 1 == b ? 0 : q + 1;
+          asm volatile("bar.sync 1, %0;" ::"r"(b * 32) : "memory");
         }
         if (any) {
-          store_col(u, A + size_t(i) * H, H, lane);
+          store_col<NR>(u, A + size_t(warp) * H, lane);
+          if (lane == 0) nA[warp] = nu;
           rot = true;
         }
       }
@@ -205,9 +231,10 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
         const int np = (pos == 0) ? 0 : (pos == kJBlocks - 1 ? 1 : pos + 1);
         int drank, dslot;
         pos_owner(np, drank, dslot);
-        double* src = buf + (cur * 2 + s) * slot_sz;
-        double* dst = cluster.map_shared_rank(buf + (nxt * 2 + dslot) * slot_sz, drank);
-        for (size_t e = tid; e < slot_sz; e += kJWarps * 32) dst[e] = src[e];
+        const double2* src = reinterpret_cast<const double2*>(buf + (cur * 2 + s) * slot_sz);
+        double2* dst =
+            reinterpret_cast<double2*>(cluster.map_shared_rank(buf + (nxt * 2 + dslot) * slot_sz, drank));
+        for (int e = tid; e < int(slot_sz / 2); e += kJWarps * 32) dst[e] = src[e];
         if (tid == 0) *cluster.map_shared_rank(blk + nxt * 2 + dslot, drank) = blk[cur * 2 + s];
       }
       cluster.sync();
@@ -253,33 +280,39 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
   cluster.sync();
 }
 
-SmemAttrOnce g_jc_attr;
+template <int NR>
+void launch_cluster(Ctx& c, const JcArgs& a, size_t smem) {
+  static SmemAttrOnce attr;
+  attr.ensure(jacobi_cluster_kernel<NR>, int(kJSmemMax));
+  jacobi_cluster_kernel<NR><<<kJP, kJWarps * 32, smem, c.stream>>>(a);
+}
+
+// rows of [X; J] per lane, rounded up to the next instance
+int rows_per_lane(int m, int k) {
+  const int n = (m + k + 31) / 32;
+  return n <= 8 ? n : (n + 1) & ~1;
+}
+int block_width(int k) { return (k + kJBlocks - 1) / kJBlocks; }
+size_t cluster_smem(int b, int nr) { return (size_t(4) * (b * 32 * nr + ((b + 1) & ~1)) + 64) * 8; }
 
 }  // namespace
 
 bool jacobi_cluster_fits(int m, int k) {
-  if (m < 1 || k < 2 || k > 2 * kJBlocks * 16) return false;
-  const int kk = (k + 1) & ~1;
-  int b = (kk + kJBlocks - 1) / kJBlocks;
-  b += b & 1;
-  const int H = ((m + k + 31) / 32) * 32;
-  return b <= kJWarps && H <= 32 * kJMaxRowsPerLane && (size_t(4) * b * H + 64) * 8 <= kJSmemMax;
+  if (m < 1 || k < 2) return false;
+  const int b = block_width(k), nr = rows_per_lane(m, k);
+  return b <= kJWarps && nr <= kJMaxRowsPerLane && cluster_smem(b, nr) <= kJSmemMax;
 }
 
 void jacobi_svd_cluster(Ctx& c, double* X, int m, int k, int64_t ldx, double* J, int64_t ldj, double* S,
                         int max_sweeps, double tol, int* d_sweeps) {
   IPEPS_CHECK(jacobi_cluster_fits(m, k), "jacobi_svd_cluster: problem does not fit");
   if (tol <= 0) tol = double(m) * 2.220446049250313e-16;
-  const int kk = (k + 1) & ~1;
-  int b = (kk + kJBlocks - 1) / kJBlocks;
-  b += b & 1;
   JcArgs a{};
   a.X = X;
   a.ldx = ldx;
   a.m = m;
   a.k = k;
-  a.b = b;
-  a.H = ((m + k + 31) / 32) * 32;
+  a.b = block_width(k);
   a.max_sweeps = max_sweeps;
   a.tol2 = tol * tol;
   a.Xout = X;
@@ -288,10 +321,23 @@ void jacobi_svd_cluster(Ctx& c, double* X, int m, int k, int64_t ldx, double* J,
   a.S = S;
   a.status = c.d_status;
   a.sweeps_out = d_sweeps;
-  const size_t smem = (size_t(4) * b * a.H + 64) * 8;
-  g_jc_attr.ensure(jacobi_cluster_kernel, int(kJSmemMax));
+  const int nr = rows_per_lane(m, k);
+  const size_t smem = cluster_smem(a.b, nr);
   ProfScope ps(c, KFam::Jacobi);
-  jacobi_cluster_kernel<<<kJP, kJWarps * 32, smem, c.stream>>>(a);
+  switch (nr) {
+    case 1: launch_cluster<1>(c, a, smem); break;
+    case 2: launch_cluster<2>(c, a, smem); break;
+    case 3: launch_cluster<3>(c, a, smem); break;
+    case 4: launch_cluster<4>(c, a, smem); break;
+    case 5: launch_cluster<5>(c, a, smem); break;
+    case 6: launch_cluster<6>(c, a, smem); break;
+    case 7: launch_cluster<7>(c, a, smem); break;
+    case 8: launch_cluster<8>(c, a, smem); break;
+    case 10: launch_cluster<10>(c, a, smem); break;
+    case 12: launch_cluster<12>(c, a, smem); break;
+    case 14: launch_cluster<14>(c, a, smem); break;
+    default: launch_cluster<16>(c, a, smem); break;
+  }
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Jacobi, 6.0 * double(m + k) * k * k / 2.0);
 }

@@ -4,6 +4,18 @@
 
 namespace ipeps {
 
+// 1 / sqrt(d) of a normal d > 0 (anything else: unspecified), within 2 ulp: the
+// hardware estimate y and one third-order step of the series of (1 - e)^(-1/2),
+// e = 1 - d y^2 (Householder's method).  It has no special cases, so the compiler
+// may fill its latency with the independent work around it.
+__device__ __forceinline__ double rsqrt_normal(double d) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double e = fma(-d * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+
 // In-place guarded Cholesky of a k x k SPD matrix: G = R^T R (upper R,
 // strict lower triangle zeroed).  If d_trace_shift is given, shift_factor *
 // (*d_trace_shift) is first added to the diagonal (shifted CholeskyQR).

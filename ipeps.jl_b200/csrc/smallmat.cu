@@ -320,8 +320,11 @@ __device__ __forceinline__ bool rr_pair(int pi, int r, int kk, int k, int& p, in
 }
 
 constexpr int kJacThreads = 512;  // 64 groups of 8 lanes, one column pair each per round
-// sketch width from which the Jacobi SVD runs on a cluster of 8 CTAs
-constexpr int kClusterJacobiMinK = 96;
+// Sketch width from which the Jacobi SVD runs on a cluster of 8 CTAs.  Four sweeps on
+// one CTA with the rotations applied to J afterwards against the cluster: 80 us and
+// 82 us at k = 26, 121 and 103 at k = 34, 163 and 104 at k = 46, 252 and 128 at k = 62
+// (six or seven sweeps: 156 and 173 at k = 34, 242 and 154 at k = 46).
+constexpr int kClusterJacobiMinK = 40;
 
 // One-sided Jacobi on X (m x k, rows zero-padded to 16 NV) held in shared
 // memory.  Each 8-lane group takes one column pair per round: it reads both
@@ -438,7 +441,7 @@ __global__ void __launch_bounds__(kJacThreads) jacobi_log_kernel(double* Xg, int
 
 constexpr int kApplyRows = 8;  // rows of J per CTA, one warp each
 constexpr int kChunk = 16;     // rounds of the log staged per step
-constexpr int kMaxPairs = 128; // kk/2 <= 128 (k <= 256)
+constexpr int kMaxPairs = 32;  // kk/2 <= 32 (k < kClusterJacobiMinK)
 
 size_t apply_smem_bytes(int k) {
   const int np = ((k + 1) & ~1) / 2;
@@ -507,7 +510,7 @@ __global__ void __launch_bounds__(kApplyRows * 32) jacobi_apply_kernel(const dou
 }
 
 // shared-memory opt-in, once per kernel and device
-SmemAttrOnce g_chol_attr, g_trsm_attr[9], g_jlog_attr[11], g_apply_attr;
+SmemAttrOnce g_chol_attr, g_trsm_attr[9], g_jlog_attr[5], g_apply_attr;
 
 template <int NV>
 void launch_jacobi(Ctx& c, double* X, int m, int k, int64_t ldx, double2* rot, int max_sweeps, double tol, double* S,
@@ -566,7 +569,7 @@ void jacobi_svd_auto(Ctx& c, double* X, int m, int k, int64_t ldx, double* J, in
   }
   const int nv = (m + 15) / 16;
   const size_t smem = (size_t(16) * nv * k + k) * 8;
-  if (k < 2 || nv > 10 || k > 2 * kMaxPairs || smem > kSmemMax || apply_smem_bytes(k) > kSmemMax) {
+  if (k < 2 || nv > 4 || k > 2 * kMaxPairs || smem > kSmemMax || apply_smem_bytes(k) > kSmemMax) {
     jacobi_svd(c, X, m, k, ldx, J, ldj, S, max_sweeps, tol, d_sweeps);
     return;
   }
@@ -579,13 +582,7 @@ void jacobi_svd_auto(Ctx& c, double* X, int m, int k, int64_t ldx, double* J, in
       case 1: launch_jacobi<1>(c, X, m, k, ldx, rp, max_sweeps, tol, S, d_sweeps, smem); break;
       case 2: launch_jacobi<2>(c, X, m, k, ldx, rp, max_sweeps, tol, S, d_sweeps, smem); break;
       case 3: launch_jacobi<3>(c, X, m, k, ldx, rp, max_sweeps, tol, S, d_sweeps, smem); break;
-      case 4: launch_jacobi<4>(c, X, m, k, ldx, rp, max_sweeps, tol, S, d_sweeps, smem); break;
-      case 5: launch_jacobi<5>(c, X, m, k, ldx, rp, max_sweeps, tol, S, d_sweeps, smem); break;
-      case 6: launch_jacobi<6>(c, X, m, k, ldx, rp, max_sweeps, tol, S, d_sweeps, smem); break;
-      case 7: launch_jacobi<7>(c, X, m, k, ldx, rp, max_sweeps, tol, S, d_sweeps, smem); break;
-      case 8: launch_jacobi<8>(c, X, m, k, ldx, rp, max_sweeps, tol, S, d_sweeps, smem); break;
-      case 9: launch_jacobi<9>(c, X, m, k, ldx, rp, max_sweeps, tol, S, d_sweeps, smem); break;
-      default: launch_jacobi<10>(c, X, m, k, ldx, rp, max_sweeps, tol, S, d_sweeps, smem); break;
+      default: launch_jacobi<4>(c, X, m, k, ldx, rp, max_sweeps, tol, S, d_sweeps, smem); break;
     }
     c.count(KFam::Jacobi, 6.0 * double(m) * k * k / 2.0);
   }

@@ -75,3 +75,25 @@ def test_orth_block_edges(engine, pkg, N, k):
     assert np.array_equal(np.tril(R, -1), np.zeros((k, k)))
     ref = np.linalg.cholesky(Y.T @ Y).T
     assert np.linalg.norm(R - ref) <= 100 * k * eps * np.linalg.cond(Y) ** 2 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("n", [2, 17, 38, 39, 40, 41, 47, 48, 64, 66, 81, 97, 113, 144, 160])
+def test_projector_jacobi_block_edges(engine, pkg, n):
+    """The Jacobi SVD inside the projector at the widths where its kernels change (one CTA below 40
+    columns, clusters of 8 CTAs with 16 column blocks from there, odd block widths, rows per lane):
+    n x n corners whose sketch is the whole space, singular values 1 .. 1e-4 known by construction.
+    Bars: Jacobi and CholeskyQR on an n x n product leave n eps s_1 in each value and, for P1 P2 =
+    R2 V S^-1 U^T R1 of the n - 1 leading triplets, that times s_1 / s_n (1e4) and the inverse
+    relative gap of the truncated pair (>= 9.2 / n), all with a factor 20."""
+    rng = np.random.default_rng(n)
+    eps = np.finfo(float).eps
+    s = np.logspace(0, -4, n)
+    U, _ = np.linalg.qr(rng.standard_normal((n, n)))
+    V, _ = np.linalg.qr(rng.standard_normal((n, n)))
+    Z, _ = np.linalg.qr(rng.standard_normal((n, n)))
+    R1, R2 = (U * np.sqrt(s)) @ Z, Z.T @ (np.sqrt(s)[:, None] * V.T)
+    P1, P2, got = pkg.get_projector(R1, R2, n - 1, engine=engine)
+    assert got.shape == (n - 1,)
+    assert np.abs(got - s[:-1]).max() <= 20 * n * eps
+    ref = Z.T[:, :-1] @ Z[:-1]  # R2 V S^-1 U^T R1 on the leading triplets
+    assert np.abs(P1 @ P2 - ref).max() <= 20 * n * eps * 1e4 * max(1.0, n / 9.2)
