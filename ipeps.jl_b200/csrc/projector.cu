@@ -101,7 +101,7 @@ Tensor apply_left_T(Ctx& c, const Tensor& X, const MatRef& R, char op) {
   return Y;
 }
 
-Tensor orth(Ctx& c, const Tensor& Y0, int passes, Tensor* Rout) {
+Tensor orth(Ctx& c, const Tensor& Y0, int passes, Tensor* Rout, std::vector<Tensor>* factors) {
   const int64_t N = Y0.dims[0];
   const int k = int(Y0.dims[1]);
   Tensor Y = Y0;
@@ -122,7 +122,9 @@ Tensor orth(Ctx& c, const Tensor& Y0, int passes, Tensor* Rout) {
     const double sf = (pass == 0) ? 11.0 * (double(N) * k + double(k) * (k + 1)) * u : 0.0;
     Tensor Yn = c.alloc(DType::F64, {N, k});
     if (packed) {
+      if (factors && pass > 0) Rrow = c.alloc(DType::F64, {cholqr_packed(k)});
       chol_packed(c, G.f64(), k, k, sf, Rrow.f64(), Rout != nullptr);
+      if (factors) factors->push_back(Rrow);
       trsm_packed(c, Y.f64(), N, N, k, Rrow.f64(), Yn.f64(), N);
     } else if (blocked) {
       chol_blocked(c, G.f64(), k, k, sf, Rrow.f64());
@@ -174,6 +176,13 @@ __global__ void colnorm_max_kernel(const double* X, int64_t m, int nc, unsigned 
   if (lane == 0) atomicMax(out, static_cast<unsigned long long>(__double_as_longlong(sqrt(s))));
 }
 
+// y -= f norm^2 x
+__global__ void sub_shift_kernel(double f, const double* norm, const double* x, double* y, int64_t n) {
+  const double a = -f * norm[0] * norm[0];
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+    y[i] = fma(a, x[i], y[i]);
+}
+
 // ------------------------------------------------------------------ backends
 // The projector logic below is written once over two backends: real (FP64)
 // and complex (complex128) enlarged corners.  M = R1 R2 is N1 x N2 with
@@ -195,6 +204,27 @@ struct RealOps {
   Tensor M(const Tensor& X) { return apply(c, R1, 'N', apply(c, R2, 'N', X, &pc2), &pc1); }   // M X
   Tensor MH(const Tensor& X) { return apply(c, R2, 'T', apply(c, R1, 'T', X, &pc1), &pc2); }  // M^T X
   Tensor orth_(const Tensor& Y, int passes) { return orth(c, Y, passes, nullptr); }
+  // shifted power iterations: real sketches within the packed CholeskyQR
+  static bool can_shift(int k) { return cholqr_fits(k); }
+  // orth(M^T Q - sigma Z R^-1) with Q R = Y = M Z, sigma = f |M z_1|^2 with *norm =
+  // |M z_1|: an orthonormal basis of (M^T M - sigma) Z, without forming M^T M Z
+  // (whose columns span s_k^2 .. s_1^2)
+  Tensor shifted(const Tensor& Y, const Tensor& Z, double f, const double* norm, int inter) {
+    std::vector<Tensor> R;
+    Tensor W = MH(orth(c, Y, inter, nullptr, &R));
+    Tensor T = Z;
+    for (const Tensor& f : R) {
+      Tensor Tn = c.alloc(dt, Z.shape());
+      trsm_packed(c, T.f64(), N2(), N2(), int(Z.dims[1]), f.f64(), Tn.f64(), N2());
+      T = Tn;
+    }
+    const int64_t n = W.numel();
+    const unsigned grid = unsigned(std::min<int64_t>((n + 255) / 256, int64_t(c.sm_count) * 8));
+    sub_shift_kernel<<<grid, 256, 0, c.stream>>>(f, norm, T.f64(), W.f64(), n);
+    IPEPS_LAUNCH_CHECK();
+    c.count(KFam::Elementwise, 0, 24.0 * n);
+    return orth_(W, inter);
+  }
   // X = Bh^H Q2 (k x k) for Bh = M^H Q (N2 x k)
   Tensor small(const Tensor& Bh, const Tensor& Q2, int k) {
     Tensor X = c.alloc(dt, {k, k});
@@ -262,6 +292,8 @@ struct ComplexOps {
     return cmm(c, 'C', 'N', N2(), n, K1(), R2, K1(), cmm(c, 'C', 'N', K1(), n, N1(), R1, N1(), X, N1()), K1());
   }
   Tensor orth_(const Tensor& Y, int passes) { return orth_c(c, Y, passes); }
+  static bool can_shift(int) { return false; }
+  Tensor shifted(const Tensor& Y, const Tensor&, double, const double*, int inter) { return orth_(MH(orth_(Y, inter)), inter); }
   Tensor small(const Tensor& Bh, const Tensor& Q2, int k) { return cmm(c, 'C', 'N', k, k, N2(), Bh, N2(), Q2, N2()); }
   void jacobi(Tensor& X, Tensor& J, Tensor& S, int k, const SvdParams& sp, int* d_sweeps) {
     jacobi_c_svd(c, X.data(), k, k, k, J.data(), k, S.f64(), sp.jacobi_max_sweeps, sp.jacobi_tol, d_sweeps);
@@ -286,14 +318,28 @@ struct Sketch {
 // suppresses directions below ~sqrt(shift) ~ 1e-6 s_1, which over the power
 // iterations then decay away; three passes (sCholQR3) keep them, as needed
 // when the truncation reaches down to the 1e-12 relative cutoff.
+// b > 0: the power iterations are shifted, Z <- orth((M^T M - sigma_j) Z) with the
+// sigma_j at the Chebyshev nodes of [0, b s_1^2]: the product over the iterations is
+// the Chebyshev polynomial of degree q on that interval.  With b = (s_k / s_1)^2 the
+// directions outside the sketch shrink against s_n by exp(-q acosh(2 s_n^2 / s_k^2 - 1))
+// instead of (s_k / s_n)^2q: at D=5 chi=100 (s_n / s_k = 1.6) by ~5 per iteration
+// instead of ~1.8.  s_1 is |M z_1| of the first column (the leading seed), a lower
+// bound: the scale of M changes from call to call.
 template <class Ops>
-Sketch sketch_pass(Ctx& c, Ops& o, const Tensor& Om, int q, const SvdParams& sp, int inter) {
+Sketch sketch_pass(Ctx& c, Ops& o, const Tensor& Om, int q, const SvdParams& sp, int inter, double b) {
   const int k = int(Om.dims[1]);
   Sketch s;
-  Tensor Y = o.M(Om);
+  Tensor Z = Om, Y = o.M(Om);
+  double* norm = reinterpret_cast<double*>(c.scal->p) + 56;
+  if (b > 0 && q > 0) {
+    colnorms_kernel<<<1, 32, 0, c.stream>>>(Y.f64(), o.N1(), 1, norm);
+    IPEPS_LAUNCH_CHECK();
+  }
   for (int it = 0; it < q; ++it) {
-    Tensor Q = o.orth_(Y, inter);
-    Tensor Z = o.orth_(o.MH(Q), inter);
+    if (b > 0)
+      Z = o.shifted(Y, Z, 0.5 * b * (1.0 + std::cos((2 * it + 1) * 3.14159265358979323846 / (2.0 * q))), norm, inter);
+    else
+      Z = o.orth_(o.MH(o.orth_(Y, inter)), inter);
     Y = o.M(Z);
   }
   s.Q = o.orth_(Y, 3);
@@ -321,6 +367,17 @@ Sketch sketch_pass(Ctx& c, Ops& o, const Tensor& Om, int q, const SvdParams& sp,
 void copy_cols(Ctx& c, Tensor& dst, const Tensor& src, int64_t rows, int ncols, int words) {
   IPEPS_CUDA(cudaMemcpyAsync(dst.data(), src.data(), size_t(rows) * ncols * 8 * words, cudaMemcpyDeviceToDevice,
                              c.stream));
+}
+
+// Whether one shifted CholeskyQR pass keeps the directions of the first n triplets of
+// a sketch with singular values s: its shift, 11 (N k + k (k + 1)) u times the trace
+// of the Gram matrix (<= the sum of s_i^2 for a product of M with an orthonormal
+// basis), damps a direction by s_i / sqrt(s_i^2 + shift) per pass.
+bool one_pass_keeps(const std::vector<double>& s, int64_t N, int k, int n) {
+  double tr = 0;
+  for (double v : s) tr += v * v;
+  const double shift = 11.0 * (double(N) * k + double(k) * (k + 1)) * 1.1102230246251565e-16 * tr;
+  return s[size_t(n - 1)] * s[size_t(n - 1)] >= 10.0 * shift;
 }
 
 template <class Ops>
@@ -371,8 +428,31 @@ ProjResult projector_impl(Ctx& c, Ops& o, int chi, const SvdParams& sp, ProjCach
     inter = std::max(inter, 3);
     q += std::min(6, int(std::ceil(std::log(cache->seed_tol(sp.seed_older) / rtol) / std::log(7.0))));
   }
-  const bool adapt = q > 0 && cache && inter >= 3;
+  // Shifted iterations (see sketch_pass) where the seeds' spectrum is known and not
+  // cutoff-limited: as many as this direction's last call needed, corrected for
+  // another tolerance, at the rate of the Chebyshev polynomial (a quarter off: s_k of
+  // the sketch is a lower bound of the first value outside it).  Done up front an
+  // iteration costs two products with M and two CholeskyQR passes; as an extra pass
+  // it costs a Rayleigh-Ritz step (two sCholQR3, a Jacobi SVD) besides.
+  // The target is a thirtieth of the tolerance, as an extra pass overshoots it (a
+  // residual just below the tolerance leaves the errors of a whole trajectory larger).
+  const auto rate_of = [](double sn2, double b) { return 0.75 * std::acosh(2.0 * sn2 / b - 1.0); };
+  constexpr double kAim = 1.0 / 30.0;
+  constexpr int kMaxShifted = 8;
+  double b = 0;
+  const bool shift = warm && q > 0 && Ops::can_shift(k) && !cache->cutoff_limited &&
+                     cache->seed_spec(sp.seed_older).k == k;
+  if (shift) {
+    const auto& spec = cache->seed_spec(sp.seed_older);
+    b = std::min(spec.sk2, 0.9 * spec.sn2);
+    double need = cache->need;
+    if (cache->rtol > 0) need += std::log(cache->rtol / rtol) / rate_of(spec.sn2, b);
+    q = std::max(sp.power_iters_warm, std::min(kMaxShifted, int(std::ceil(need))));
+    inter = std::max(sp.inter_passes, spec.one_pass ? 1 : 3);
+  }
+  const bool adapt = q > 0 && cache && inter >= 3 && !shift;
   if (adapt) q += cache->qbonus;
+  int iters = q;  // power iterations of all passes
   int extra = 0;
   double res_final = 1.0;
 
@@ -386,7 +466,7 @@ ProjResult projector_impl(Ctx& c, Ops& o, int chi, const SvdParams& sp, ProjCach
   double* d_res = reinterpret_cast<double*>(c.scal->p) + 48;
   double prev_res = 1e300;
   for (int attempt = 0;; ++attempt) {
-    sk = sketch_pass(c, o, Om, q, sp, inter);
+    sk = sketch_pass(c, o, Om, q, sp, inter, b);
     d_perm = static_cast<int*>(sk.perm.data());
     IPEPS_CUDA(cudaMemcpyAsync(all.data(), sk.Ss.data(), size_t(k) * 8, cudaMemcpyDeviceToHost, c.stream));
     c.sync();
@@ -403,6 +483,7 @@ ProjResult projector_impl(Ctx& c, Ops& o, int chi, const SvdParams& sp, ProjCach
       Om = c.alloc(dt, {N2, k});
       randn(c, Om);
       q = sp.power_iters;
+      b = 0;
       --attempt;
       continue;
     }
@@ -455,9 +536,16 @@ ProjResult projector_impl(Ctx& c, Ops& o, int chi, const SvdParams& sp, ProjCach
       break;
     }
     prev_res = res;
-    // not converged: one more power iteration from the current right vectors
+    // not converged: more power iterations from the current right vectors
     Om = Vk;
     q = 1;
+    if (Ops::can_shift(k) && n_above >= new_chi && all[n - 1] > 0) {
+      const double sn2 = std::pow(all[n - 1] / smax, 2);
+      b = std::min(std::pow(all[k - 1] / smax, 2), 0.9 * sn2);
+      q = std::max(1, std::min(kMaxShifted, int(std::ceil(std::log(res_final / (kAim * rtol)) / rate_of(sn2, b))) - 1));
+      if (!one_pass_keeps(all, N1, k, n)) inter = std::max(inter, 3);
+    }
+    iters += q + 1;
     c.projector_extra_passes++;
     ++extra;
   }
@@ -484,6 +572,18 @@ ProjResult projector_impl(Ctx& c, Ops& o, int chi, const SvdParams& sp, ProjCach
     cache->tol_old = cache->tol;
     cache->tol = std::max(res_final, 1e-15);  // the residual these vectors reached
     cache->cutoff_limited = n_above_last < new_chi;
+    cache->spec_old = cache->spec;
+    cache->spec = {};
+    if (n_above_last >= new_chi && all[n - 1] > 0) {
+      cache->spec = {k, std::pow(all[n - 1] / all[0], 2), std::pow(all[k - 1] / all[0], 2),
+                     one_pass_keeps(all, N1, k, n)};
+      const double r = rate_of(cache->spec.sn2, std::min(cache->spec.sk2, 0.9 * cache->spec.sn2));
+      cache->need = std::min(iters, kMaxShifted) + std::log(std::max(res_final, 1e-16) / (kAim * rtol)) / r;
+      // without an extra pass at least one less: the mixed form's residuals stay at
+      // the floor of its products whatever the iterations
+      if (extra == 0) cache->need = std::min(cache->need, double(iters - 1));
+      cache->rtol = rtol;
+    }
     if (adapt)
       cache->qbonus = extra > 0 ? std::min(cache->qbonus + extra, sp.max_extra_passes) : std::max(cache->qbonus - 1, 0);
   }

@@ -56,7 +56,18 @@ struct ProjCache {
   int qbonus = 0;
   // residual (relative to s_1) the call that produced V (Vold) reached
   double tol = 1.0, tol_old = 1.0;
+  // the sketch of that call: width, (s_n / s_1)^2 and (s_k / s_1)^2 (kept and last
+  // value: the interval of the next call's shifts), and whether single shifted CholeskyQR
+  // passes keep its directions (see projector.cu)
+  struct Spectrum {
+    int k = 0;
+    double sn2 = 0, sk2 = 0;
+    bool one_pass = false;
+  } spec, spec_old;
+  // shifted power iterations that the last call needed for the residual rtol
+  double need = 0, rtol = 0;
   const Tensor& seed(bool older) const { return (older && !Vold.empty()) ? Vold : V; }
+  const Spectrum& seed_spec(bool older) const { return (older && !Vold.empty()) ? spec_old : spec; }
   double seed_tol(bool older) const { return (older && !Vold.empty()) ? tol_old : tol; }
 };
 
@@ -99,6 +110,7 @@ Tensor apply_left_T(Ctx& c, const Tensor& X, const MatRef& R, char op, PlaneCach
 
 // Orthonormalise the columns of Y (N x k) by shifted CholeskyQR; if Rout is
 // non-null it receives R with Y = Q R.
-Tensor orth(Ctx& c, const Tensor& Y, int passes, Tensor* Rout);
+// passes (k <= 160): receives the packed R of each pass, Y = Q R_last ... R_first.
+Tensor orth(Ctx& c, const Tensor& Y, int passes, Tensor* Rout, std::vector<Tensor>* factors = nullptr);
 
 }  // namespace ipeps
