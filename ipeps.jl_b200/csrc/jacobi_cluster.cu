@@ -69,6 +69,10 @@ __device__ __forceinline__ void pos_owner(int p, int& rank, int& slot) {
   }
 }
 
+// 1 / sqrt(h) of h > 0, subnormal ones too: the columns of a rank-deficient X shrink
+// by the rounding level with every sweep, until their squared norms underflow.
+__device__ __forceinline__ double rsqrt_pos(double h) { return h >= 1e-300 ? rsqrt_normal(h) : rsqrt(h); }
+
 // Rotates column u (registers, squared norm nu) against the shared column y
 // (squared norm *ny); true when it rotated.  The dot product runs over the rows of
 // X only (nx of the NR rows per lane), the rotation over those of [X; J].
@@ -92,7 +96,7 @@ __device__ __forceinline__ bool rotate_pair(double (&u)[NR], double& nu, double*
   for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
   if (!(c != 0.0 && nu > 0.0 && nv > 0.0 && c * c > tol2 * (nu * nv))) return false;
   const double d = nv - nu;
-  const double rho = rsqrt_normal(fma(d, d, 4.0 * c * c));
+  const double rho = rsqrt_pos(fma(d, d, 4.0 * c * c));
   const double c2 = fabs(d) * rho, s2 = copysign(1.0, d) * (2.0 * c * rho);
   const double uu = 0.5 * (1.0 + c2);
   const double ru = rsqrt_normal(uu);

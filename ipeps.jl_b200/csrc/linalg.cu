@@ -161,7 +161,8 @@ __global__ void __launch_bounds__(kThreads) jacobi_kernel(double* X, int m, int 
 __global__ void sort_desc_kernel(const double* S, int k, double* S_out, int* perm) {
   extern __shared__ unsigned char sm_raw[];
   double* v = reinterpret_cast<double*>(sm_raw);
-  for (int i = threadIdx.x; i < k; i += blockDim.x) v[i] = S[i];
+  // (a NaN sorts last: perm stays a permutation, the gathers that use it stay in range)
+  for (int i = threadIdx.x; i < k; i += blockDim.x) v[i] = isnan(S[i]) ? -1.0 : S[i];
   __syncthreads();
   // rank sort: position = #{j : v[j] > v[i]} + #{j > i : v[j] == v[i]}
   for (int i = threadIdx.x; i < k; i += blockDim.x) {
@@ -171,7 +172,7 @@ __global__ void sort_desc_kernel(const double* S, int k, double* S_out, int* per
       double y = v[j];
       pos += (y > x) || (y == x && j > i);
     }
-    S_out[pos] = x;
+    S_out[pos] = S[i];
     perm[pos] = i;
   }
 }

@@ -97,3 +97,18 @@ def test_projector_jacobi_block_edges(engine, pkg, n):
     assert np.abs(got - s[:-1]).max() <= 20 * n * eps
     ref = Z.T[:, :-1] @ Z[:-1]  # R2 V S^-1 U^T R1 on the leading triplets
     assert np.abs(P1 @ P2 - ref).max() <= 20 * n * eps * 1e4 * max(1.0, n / 9.2)
+
+
+@pytest.mark.parametrize("n,rank", [(62, 5), (100, 20)])
+def test_projector_rank_deficient_corners(engine, pkg, n, rank):
+    """Corners of exact low rank: the discarded columns of the Jacobi SVD are rounding noise that every
+    sweep shrinks further, down to underflow.  The kept values against numpy's (n eps s_1, factor 20)."""
+    rng = np.random.default_rng(n)
+    # the Gram matrices of the product scale with the fourth power, their pivot guard is absolute at 1e-300
+    for scale in (1.0, 1e-20, 1e-40):
+        R1 = scale * (rng.standard_normal((n, rank)) @ rng.standard_normal((rank, n)))
+        R2 = scale * (rng.standard_normal((n, rank)) @ rng.standard_normal((rank, n)))
+        s_ref = np.linalg.svd(R1 / scale @ (R2 / scale), compute_uv=False)
+        P1, P2, s = pkg.get_projector(R1, R2, rank, engine=engine)
+        assert np.isfinite(P1).all() and np.isfinite(P2).all()
+        assert np.abs(s[:rank] / scale ** 2 - s_ref[:rank]).max() <= 20 * n * np.finfo(float).eps * s_ref[0]
