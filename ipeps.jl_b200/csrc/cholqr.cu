@@ -1,5 +1,5 @@
 // Cholesky factor and triangular solve of one CholeskyQR pass for sketches of
-// up to 160 columns: G = R^T R (shifted, guarded), then Q = Y R^-1.
+// up to 192 columns: G = R^T R (shifted, guarded), then Q = Y R^-1.
 //
 // Both work on 8 x 8 blocks so that all but the 8 x 8 diagonal factors runs on
 // the FP64 tensor pipe (mma.sync m8n8k4; tcgen05 has no FP64 kind).  R goes from
@@ -17,6 +17,9 @@
 // substitution by rows that it replaces).
 // One CholeskyQR pass at N = 2500 without its Gram product, event-timed: 96.9 ->
 // 58 us at k = 160, 71.1 -> 45 us at k = 128, 61.5 -> 39 us at k = 101.
+// Complex sketches run on the same kernels as real ones of twice the width (66
+// columns: one CTA with a barrier per column and a row per warp before; a pass
+// without its Gram product ~200 -> ~35 us).
 #include "linalg.cuh"
 
 #include <algorithm>
@@ -74,6 +77,10 @@ __host__ __device__ __forceinline__ int col_base(int I, int nb) { return I * nb 
 // its time fetching instructions (55 us at k = 160).
 // The contract is that of chol_blocked: shift_factor * trace is added to the
 // diagonal, a pivot at or below 1e-32 trace leaves R[j][j] = 1 and row j zero.
+// CX: G is complex Hermitian of k / 2 columns, taken as the real symmetric matrix of
+// its 2 x 2 blocks [[re, -im], [im, re]].  The factor of that is the same form of the
+// complex factor (the Cholesky factor is unique), so the real kernels do the work.
+template <bool CX>
 __global__ void __launch_bounds__(kCpThreads, 1)
     chol_panel_kernel(double* G, int k, int64_t ldg, double shift_factor, double2* __restrict__ Rpk, int write_g) {
   extern __shared__ __align__(16) double2 S[];
@@ -95,7 +102,15 @@ __global__ void __launch_bounds__(kCpThreads, 1)
         }
         const int I = J + b - first, r = 8 * I + g, c = 8 * J + 2 * t;
         v[q] = make_double2(r == c ? 1.0 : 0.0, r == c + 1 ? 1.0 : 0.0);
-        if (b < nblk && r < k) {
+        if constexpr (CX) {
+          if (b < nblk && r < k && c < k) {
+            const int rr = r >> 1, cc = c >> 1;
+            double2 z = reinterpret_cast<const double2*>(G)[min(rr, cc) + int64_t(max(rr, cc)) * ldg];
+            if (rr > cc) z.y = -z.y;  // the upper triangle is stored
+            if (rr == cc) z.y = 0.0;
+            v[q] = (r & 1) ? make_double2(z.y, z.x) : make_double2(z.x, -z.y);
+          }
+        } else if (b < nblk && r < k) {
           if (c < k) v[q].x = G[min(r, c) + int64_t(max(r, c)) * ldg];
           if (c + 1 < k) v[q].y = G[min(r, c + 1) + int64_t(max(r, c + 1)) * ldg];
         }
@@ -269,7 +284,9 @@ __global__ void __launch_bounds__(kCpThreads, 1)
 // 2t and 2t + 1.  The CTA's warps beyond those with rows only help to stage R.
 constexpr int kTpThreads = 256;
 
-template <int NB>
+// CX: complex Y and Q of k / 2 columns; a row enters as (re, -im) pairs, the first row
+// of its 2 x 2 blocks, one element per lane and block.
+template <int NB, bool CX>
 __global__ void __launch_bounds__(kTpThreads) trsm_panel_kernel(const double* __restrict__ Y, int64_t ldy, int64_t N,
                                                                 int k, int warps, const double2* __restrict__ Rpk,
                                                                 double* __restrict__ Q, int64_t ldq) {
@@ -280,12 +297,18 @@ __global__ void __launch_bounds__(kTpThreads) trsm_panel_kernel(const double* __
   const bool mine = warp < warps && row < N;
   double a[NB][2];
 #pragma unroll
-  for (int J = 0; J < NB; ++J)
+  for (int J = 0; J < NB; ++J) {
+    const int c = 8 * J + 2 * t;
+    if constexpr (CX) {
+      double2 z = make_double2(0.0, 0.0);
+      if (mine && c < k) z = reinterpret_cast<const double2*>(Y)[row + int64_t(c >> 1) * ldy];
+      a[J][0] = z.x;
+      a[J][1] = -z.y;
+    } else {
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int c = 8 * J + 2 * t + e;
-      a[J][e] = (mine && c < k) ? Y[row + int64_t(c) * ldy] : 0.0;
+      for (int e = 0; e < 2; ++e) a[J][e] = (mine && c + e < k) ? Y[row + int64_t(c + e) * ldy] : 0.0;
     }
+  }
   // (all of R in flight at once: 16-byte copies that bypass the registers)
   for (int i = tid; i < n2; i += kTpThreads)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(unsigned(__cvta_generic_to_shared(Rs + i))),
@@ -300,8 +323,12 @@ __global__ void __launch_bounds__(kTpThreads) trsm_panel_kernel(const double* __
     dmma8(x0, x1, a[0][0], b.x);
     dmma8(x0, x1, a[0][1], b.y);
     const int c = 8 * J + 2 * t;
-    if (mine && c < k) Q[row + int64_t(c) * ldq] = x0;
-    if (mine && c + 1 < k) Q[row + int64_t(c + 1) * ldq] = x1;
+    if constexpr (CX) {
+      if (mine && c < k) reinterpret_cast<double2*>(Q)[row + int64_t(c >> 1) * ldq] = make_double2(x0, -x1);
+    } else {
+      if (mine && c < k) Q[row + int64_t(c) * ldq] = x0;
+      if (mine && c + 1 < k) Q[row + int64_t(c + 1) * ldq] = x1;
+    }
     const double m0 = -x0, m1 = -x1;
     // four blocks at a time, as far as there are any (a group may run over the end of
     // the block row: what it computes there is not used)
@@ -321,23 +348,42 @@ __global__ void __launch_bounds__(kTpThreads) trsm_panel_kernel(const double* __
   }
 }
 
-SmemAttrOnce g_chol_panel_attr, g_trsm_panel_attr[6];
+template <bool CX>
+void launch_chol(Ctx& c, double* G, int k, int64_t ldg, double shift_factor, double* Rpk, bool write_g) {
+  static SmemAttrOnce attr;
+  attr.ensure(chol_panel_kernel<CX>, int(size_t(cholqr_packed(kCholqrMax)) * 8));
+  chol_panel_kernel<CX><<<1, kCpThreads, size_t(cholqr_packed(k)) * 8, c.stream>>>(
+      G, k, ldg, shift_factor, reinterpret_cast<double2*>(Rpk), write_g);
+  IPEPS_LAUNCH_CHECK();
+}
 
-template <int NB>
+template <int NB, bool CX>
 void launch_trsm(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const double* Rpk, double* Q, int64_t ldq) {
   const size_t pad = 3 * 512;  // a group of four blocks reads over the end
   const size_t smem = size_t(cholqr_packed(k)) * 8 + pad;
-  g_trsm_panel_attr[NB / 4].ensure(trsm_panel_kernel<NB>, int(size_t(cholqr_packed(8 * NB)) * 8 + pad));
+  static SmemAttrOnce attr;
+  attr.ensure(trsm_panel_kernel<NB, CX>, int(size_t(cholqr_packed(8 * NB)) * 8 + pad));
   // eight rows per warp; one CTA per SM as long as eight warps hold its rows (R is staged once per CTA)
   const int64_t groups = (N + 7) / 8;
   const int64_t warps = std::min<int64_t>(kTpThreads / 32, (groups + c.sm_count - 1) / c.sm_count);
-  trsm_panel_kernel<NB><<<unsigned((groups + warps - 1) / warps), kTpThreads, smem, c.stream>>>(
+  trsm_panel_kernel<NB, CX><<<unsigned((groups + warps - 1) / warps), kTpThreads, smem, c.stream>>>(
       Y, ldy, N, k, int(warps), reinterpret_cast<const double2*>(Rpk), Q, ldq);
+  IPEPS_LAUNCH_CHECK();
+}
+
+template <bool CX>
+void trsm_by_width(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const double* Rpk, double* Q, int64_t ldq) {
+  switch ((k + 31) / 32) {
+    case 1: launch_trsm<4, CX>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
+    case 2: launch_trsm<8, CX>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
+    case 3: launch_trsm<12, CX>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
+    case 4: launch_trsm<16, CX>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
+    case 5: launch_trsm<20, CX>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
+    default: launch_trsm<24, CX>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
+  }
 }
 
 }  // namespace
-
-bool cholqr_fits(int k) { return k >= 1 && k <= 160; }
 
 int64_t cholqr_packed(int k) {
   const int64_t nb = (k + 7) / 8;
@@ -347,10 +393,7 @@ int64_t cholqr_packed(int k) {
 void chol_packed(Ctx& c, double* G, int k, int64_t ldg, double shift_factor, double* Rpk, bool write_g) {
   IPEPS_CHECK(cholqr_fits(k), "chol_packed: k out of range");
   ProfScope ps(c, KFam::SmallLinalg);
-  g_chol_panel_attr.ensure(chol_panel_kernel, int(size_t(cholqr_packed(160)) * 8));
-  chol_panel_kernel<<<1, kCpThreads, size_t(cholqr_packed(k)) * 8, c.stream>>>(
-      G, k, ldg, shift_factor, reinterpret_cast<double2*>(Rpk), write_g);
-  IPEPS_LAUNCH_CHECK();
+  launch_chol<false>(c, G, k, ldg, shift_factor, Rpk, write_g);
   c.count(KFam::SmallLinalg, double(k) * k * k / 3.0);
 }
 
@@ -358,15 +401,24 @@ void trsm_packed(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const d
   IPEPS_CHECK(cholqr_fits(k), "trsm_packed: k out of range");
   if (N == 0) return;
   ProfScope ps(c, KFam::SmallLinalg);
-  switch ((k + 31) / 32) {
-    case 1: launch_trsm<4>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
-    case 2: launch_trsm<8>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
-    case 3: launch_trsm<12>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
-    case 4: launch_trsm<16>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
-    default: launch_trsm<20>(c, Y, ldy, N, k, Rpk, Q, ldq); break;
-  }
-  IPEPS_LAUNCH_CHECK();
+  trsm_by_width<false>(c, Y, ldy, N, k, Rpk, Q, ldq);
   c.count(KFam::SmallLinalg, double(N) * k * k);
+}
+
+// the real form of G has twice its trace: half the shift factor is the same shift
+void chol_packed_c(Ctx& c, const void* G, int k, int64_t ldg, double shift_factor, double* Rpk) {
+  IPEPS_CHECK(cholqr_fits(2 * k), "chol_packed_c: k out of range");
+  ProfScope ps(c, KFam::SmallLinalg);
+  launch_chol<true>(c, static_cast<double*>(const_cast<void*>(G)), 2 * k, ldg, 0.5 * shift_factor, Rpk, false);
+  c.count(KFam::SmallLinalg, 8.0 * double(k) * k * k / 6.0);
+}
+
+void trsm_packed_c(Ctx& c, const void* Y, int64_t ldy, int64_t N, int k, const double* Rpk, void* Q, int64_t ldq) {
+  IPEPS_CHECK(cholqr_fits(2 * k), "trsm_packed_c: k out of range");
+  if (N == 0) return;
+  ProfScope ps(c, KFam::SmallLinalg);
+  trsm_by_width<true>(c, static_cast<const double*>(Y), ldy, N, 2 * k, Rpk, static_cast<double*>(Q), ldq);
+  c.count(KFam::SmallLinalg, 4.0 * double(N) * k * k);
 }
 
 }  // namespace ipeps

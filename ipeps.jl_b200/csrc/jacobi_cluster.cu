@@ -34,13 +34,13 @@ constexpr int kJMaxRowsPerLane = 16;   // height of [X; J] <= 512
 constexpr size_t kJSmemMax = 200 * 1024;
 
 struct JcArgs {
-  const double* X;
+  const void* X;
   int64_t ldx;
   int m, k, b;  // rows of X, columns, block width
   int max_sweeps;
   double tol2;
-  double* Xout;
-  double* J;
+  void* Xout;
+  void* J;
   int64_t ldj;
   double* S;
   int* status;
@@ -113,14 +113,65 @@ __device__ __forceinline__ bool rotate_pair(double (&u)[NR], double& nu, double*
   return true;
 }
 
+// The complex pair: c = u^H y = |c| e^{i phi} is rotated as the real pair (u,
+// e^{-i phi} y); the transform of the columns is unitary.
 template <int NR>
-__device__ __forceinline__ void load_col(double (&u)[NR], const double* x, int lane) {
+__device__ __forceinline__ bool rotate_pair(double2 (&u)[NR], double& nu, double2* y, double* ny, int m, int nx, int H,
+                                            int lane, double tol2) {
+  double2 v[NR];
+  double cr = 0, ci = 0;
+  const double nv = *ny;
+#pragma unroll
+  for (int j = 0; j < NR; ++j) v[j] = y[lane + 32 * j];
+#pragma unroll
+  for (int j = 0; j < NR; ++j)
+    if (j < nx) {
+      const double2 w = lane + 32 * j < m ? v[j] : make_double2(0.0, 0.0);
+      cr = fma(u[j].x, w.x, fma(u[j].y, w.y, cr));
+      ci = fma(u[j].x, w.y, fma(-u[j].y, w.x, ci));
+    }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    cr += __shfl_xor_sync(0xffffffffu, cr, o);
+    ci += __shfl_xor_sync(0xffffffffu, ci, o);
+  }
+  const double mag2 = fma(cr, cr, ci * ci);
+  // (an underflowing |c|^2 has no usable phase: null columns of a rank-deficient X are left as they are)
+  if (!(mag2 >= 1e-300 && nu > 0.0 && nv > 0.0 && mag2 > tol2 * (nu * nv))) return false;
+  const double im = rsqrt_normal(mag2), mag = mag2 * im;
+  const double ex = cr * im, ey = -ci * im;        // e^{-i phi}
+  const double d = nv - nu;
+  const double rho = rsqrt_normal(fma(d, d, 4.0 * mag2));  // >= 4 |c|^2
+  const double c2 = fabs(d) * rho, s2 = copysign(1.0, d) * (2.0 * mag * rho);
+  const double uu = 0.5 * (1.0 + c2);
+  const double ru = rsqrt_normal(uu);
+  const double cs = uu * ru, sn = 0.5 * s2 * ru;
+#pragma unroll
+  for (int j = 0; j < NR; ++j) {
+    const double2 w = make_double2(ex * v[j].x - ey * v[j].y, ex * v[j].y + ey * v[j].x);
+    const double2 p = u[j];
+    u[j] = make_double2(cs * p.x - sn * w.x, cs * p.y - sn * w.y);
+    y[lane + 32 * j] = make_double2(sn * p.x + cs * w.x, sn * p.y + cs * w.y);
+  }
+  const double tc = 0.5 * s2 * mag * (ru * ru);
+  nu -= tc;
+  if (lane == 0) *ny = nv + tc;
+  return true;
+}
+
+__device__ __forceinline__ double norm2_of(double x) { return x * x; }
+__device__ __forceinline__ double norm2_of(double2 x) { return fma(x.x, x.x, x.y * x.y); }
+__device__ __forceinline__ void set_real(double& x, double r) { x = r; }
+__device__ __forceinline__ void set_real(double2& x, double r) { x = make_double2(r, 0.0); }
+
+template <class T, int NR>
+__device__ __forceinline__ void load_col(T (&u)[NR], const T* x, int lane) {
 #pragma unroll
   for (int j = 0; j < NR; ++j) u[j] = x[lane + 32 * j];
 }
 
-template <int NR>
-__device__ __forceinline__ void store_col(const double (&u)[NR], double* x, int lane) {
+template <class T, int NR>
+__device__ __forceinline__ void store_col(const T (&u)[NR], T* x, int lane) {
 #pragma unroll
   for (int j = 0; j < NR; ++j) x[lane + 32 * j] = u[j];
 }
@@ -132,7 +183,7 @@ __device__ __forceinline__ void store_col(const double (&u)[NR], double* x, int 
 // (recomputed every sweep) and exchanged with the blocks.  Four sweeps, before (16
 // rows per lane whatever the size, norms from every pair, even block widths) -> now:
 // k = 62 244 -> 128 us, k = 98 587 -> 288, k = 128 588 -> 336, k = 160 888 -> 556.
-template <int NR>
+template <class T, int NR>
 __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) jacobi_cluster_kernel(JcArgs a) {
   extern __shared__ __align__(16) double jsm[];
   cg::cluster_group cluster = cg::this_cluster();
@@ -142,7 +193,9 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
   const int b = a.b, m = a.m, nx = (a.m + 31) >> 5;
   // a slot: b columns of H rows, then their squared norms
   const int be = (b + 1) & ~1;  // players of the round robin inside a block (b odd: one sits out)
-  const size_t slot_sz = size_t(b) * H + be;
+  const size_t cols = size_t(b) * H, slot_sz = cols * (sizeof(T) / 8) + be;  // (T's, doubles)
+  const T* X = static_cast<const T*>(a.X);
+  T *Xout = static_cast<T*>(a.Xout), *J = static_cast<T*>(a.J);
   // buf[cur][slot] columns, then the block ids of the slots per buffer, then the flags
   double* buf = jsm;
   int* blk = reinterpret_cast<int*>(jsm + 4 * slot_sz);  // [2 buffers][2 slots]
@@ -154,16 +207,15 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
   __syncthreads();
   // load [X; I] columns of both blocks (columns >= k are zero)
   for (int s = 0; s < 2; ++s) {
-    double* dst = buf + (0 * 2 + s) * slot_sz;
+    T* dst = reinterpret_cast<T*>(buf + (0 * 2 + s) * slot_sz);
     const int b0 = blk[s] * b;
     for (int j = warp; j < b; j += kJWarps) {
       const int col = b0 + j;
       for (int r = lane; r < H; r += 32) {
-        double v = 0.0;
-        if (col < a.k) {
-          if (r < m) v = a.X[r + int64_t(col) * a.ldx];
-          else if (r - m == col) v = 1.0;
-        }
+        T v;
+        set_real(v, r - m == col ? 1.0 : 0.0);
+        if (r < m && col < a.k) v = X[r + int64_t(col) * a.ldx];
+        if (col >= a.k) set_real(v, 0.0);
         dst[j * H + r] = v;
       }
     }
@@ -178,30 +230,31 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
       double* S = buf + (cur * 2 + (j >= b)) * slot_sz;
       const int jj = j >= b ? j - b : j;
       double n = 0;
-      for (int r = lane; r < m; r += 32) n = fma(S[jj * H + r], S[jj * H + r], n);
+      for (int r = lane; r < m; r += 32) n += norm2_of(reinterpret_cast<const T*>(S)[jj * H + r]);
 #pragma unroll
       for (int o = 16; o; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-      if (lane == 0) S[size_t(b) * H + jj] = n;
+      if (lane == 0) S[cols * (sizeof(T) / 8) + jj] = n;
     }
     __syncthreads();
     bool rot = false;
     for (int round = 0; round < kJBlocks - 1; ++round) {
-      double* A = buf + (cur * 2 + 0) * slot_sz;
-      double* B = buf + (cur * 2 + 1) * slot_sz;
-      double *nA = A + size_t(b) * H, *nB = B + size_t(b) * H;
+      T* A = reinterpret_cast<T*>(buf + (cur * 2 + 0) * slot_sz);
+      T* B = reinterpret_cast<T*>(buf + (cur * 2 + 1) * slot_sz);
+      double *nA = reinterpret_cast<double*>(A + cols), *nB = reinterpret_cast<double*>(B + cols);
       if (round == 0) {
         // pairs inside each block: be - 1 sub-rounds of be/2 pairs per block
         for (int t = 0; t < be - 1; ++t) {
           for (int w = warp; w < be; w += kJWarps) {
-            double* base = (w < be / 2) ? A : B;
+            T* base = (w < be / 2) ? A : B;
             double* nb = (w < be / 2) ? nA : nB;
             int p, q;
             circle_pair(w % (be / 2), t, be, p, q);
             if (p >= b || q >= b) continue;
-            double u[NR], nu = nb[p];
-            load_col<NR>(u, base + size_t(p) * H, lane);
+            T u[NR];
+            double nu = nb[p];
+            load_col<T, NR>(u, base + size_t(p) * H, lane);
             if (rotate_pair<NR>(u, nu, base + size_t(q) * H, nb + q, m, nx, H, lane, a.tol2)) {
-              store_col<NR>(u, base + size_t(p) * H, lane);
+              store_col<T, NR>(u, base + size_t(p) * H, lane);
               if (lane == 0) nb[p] = nu;
               rot = true;
             }
@@ -211,8 +264,9 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
       }
       // pairs between the two blocks: warp i keeps column A_i, meets B_{(i+t) % b}
       if (warp < b) {
-        double u[NR], nu = nA[warp];
-        load_col<NR>(u, A + size_t(warp) * H, lane);
+        T u[NR];
+        double nu = nA[warp];
+        load_col<T, NR>(u, A + size_t(warp) * H, lane);
         bool any = false;
         int q = warp;
         for (int t = 0; t < b; ++t) {
@@ -222,7 +276,7 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
           asm volatile("bar.sync 1, %0;" ::"r"(b * 32) : "memory");
         }
         if (any) {
-          store_col<NR>(u, A + size_t(warp) * H, lane);
+          store_col<T, NR>(u, A + size_t(warp) * H, lane);
           if (lane == 0) nA[warp] = nu;
           rot = true;
         }
@@ -257,19 +311,19 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
 
   // write back W = X J columns, J, and the column norms of W
   for (int s = 0; s < 2; ++s) {
-    const double* src = buf + (cur * 2 + s) * slot_sz;
+    const T* src = reinterpret_cast<const T*>(buf + (cur * 2 + s) * slot_sz);
     const int b0 = blk[cur * 2 + s] * b;
     for (int j = warp; j < b; j += kJWarps) {
       const int col = b0 + j;
       if (col >= a.k) continue;
       double nn = 0;
       for (int r = lane; r < H; r += 32) {
-        const double v = src[j * H + r];
+        const T v = src[j * H + r];
         if (r < m) {
-          a.Xout[r + int64_t(col) * a.ldx] = v;
-          nn = fma(v, v, nn);
+          Xout[r + int64_t(col) * a.ldx] = v;
+          nn += norm2_of(v);
         } else if (r - m < a.k) {
-          a.J[(r - m) + int64_t(col) * a.ldj] = v;
+          J[(r - m) + int64_t(col) * a.ldj] = v;
         }
       }
 #pragma unroll
@@ -284,11 +338,12 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
   cluster.sync();
 }
 
-template <int NR>
+template <class T, int NR>
 void launch_cluster(Ctx& c, const JcArgs& a, size_t smem) {
   static SmemAttrOnce attr;
-  attr.ensure(jacobi_cluster_kernel<NR>, int(kJSmemMax));
-  jacobi_cluster_kernel<NR><<<kJP, kJWarps * 32, smem, c.stream>>>(a);
+  attr.ensure(jacobi_cluster_kernel<T, NR>, int(kJSmemMax));
+  jacobi_cluster_kernel<T, NR><<<kJP, kJWarps * 32, smem, c.stream>>>(a);
+  IPEPS_LAUNCH_CHECK();
 }
 
 // rows of [X; J] per lane, rounded up to the next instance
@@ -297,19 +352,17 @@ int rows_per_lane(int m, int k) {
   return n <= 8 ? n : (n + 1) & ~1;
 }
 int block_width(int k) { return (k + kJBlocks - 1) / kJBlocks; }
-size_t cluster_smem(int b, int nr) { return (size_t(4) * (b * 32 * nr + ((b + 1) & ~1)) + 64) * 8; }
+size_t cluster_smem(int b, int nr, int words) { return (size_t(4) * (b * 32 * nr * words + ((b + 1) & ~1)) + 64) * 8; }
 
-}  // namespace
-
-bool jacobi_cluster_fits(int m, int k) {
+bool fits(int m, int k, int words, int max_rows) {
   if (m < 1 || k < 2) return false;
   const int b = block_width(k), nr = rows_per_lane(m, k);
-  return b <= kJWarps && nr <= kJMaxRowsPerLane && cluster_smem(b, nr) <= kJSmemMax;
+  return b <= kJWarps && nr <= max_rows && cluster_smem(b, nr, words) <= kJSmemMax;
 }
 
-void jacobi_svd_cluster(Ctx& c, double* X, int m, int k, int64_t ldx, double* J, int64_t ldj, double* S,
-                        int max_sweeps, double tol, int* d_sweeps) {
-  IPEPS_CHECK(jacobi_cluster_fits(m, k), "jacobi_svd_cluster: problem does not fit");
+template <class T>
+void svd_cluster(Ctx& c, void* X, int m, int k, int64_t ldx, void* J, int64_t ldj, double* S, int max_sweeps,
+                 double tol, int* d_sweeps) {
   if (tol <= 0) tol = double(m) * 2.220446049250313e-16;
   JcArgs a{};
   a.X = X;
@@ -326,24 +379,45 @@ void jacobi_svd_cluster(Ctx& c, double* X, int m, int k, int64_t ldx, double* J,
   a.status = c.d_status;
   a.sweeps_out = d_sweeps;
   const int nr = rows_per_lane(m, k);
-  const size_t smem = cluster_smem(a.b, nr);
+  const size_t smem = cluster_smem(a.b, nr, sizeof(T) / 8);
   ProfScope ps(c, KFam::Jacobi);
   switch (nr) {
-    case 1: launch_cluster<1>(c, a, smem); break;
-    case 2: launch_cluster<2>(c, a, smem); break;
-    case 3: launch_cluster<3>(c, a, smem); break;
-    case 4: launch_cluster<4>(c, a, smem); break;
-    case 5: launch_cluster<5>(c, a, smem); break;
-    case 6: launch_cluster<6>(c, a, smem); break;
-    case 7: launch_cluster<7>(c, a, smem); break;
-    case 8: launch_cluster<8>(c, a, smem); break;
-    case 10: launch_cluster<10>(c, a, smem); break;
-    case 12: launch_cluster<12>(c, a, smem); break;
-    case 14: launch_cluster<14>(c, a, smem); break;
-    default: launch_cluster<16>(c, a, smem); break;
+    case 1: launch_cluster<T, 1>(c, a, smem); break;
+    case 2: launch_cluster<T, 2>(c, a, smem); break;
+    case 3: launch_cluster<T, 3>(c, a, smem); break;
+    case 4: launch_cluster<T, 4>(c, a, smem); break;
+    case 5: launch_cluster<T, 5>(c, a, smem); break;
+    case 6: launch_cluster<T, 6>(c, a, smem); break;
+    case 7: launch_cluster<T, 7>(c, a, smem); break;
+    case 8: launch_cluster<T, 8>(c, a, smem); break;
+    default:
+      if constexpr (sizeof(T) == 8) {
+        switch (nr) {
+          case 10: launch_cluster<T, 10>(c, a, smem); break;
+          case 12: launch_cluster<T, 12>(c, a, smem); break;
+          case 14: launch_cluster<T, 14>(c, a, smem); break;
+          default: launch_cluster<T, 16>(c, a, smem); break;
+        }
+      }
   }
-  IPEPS_LAUNCH_CHECK();
-  c.count(KFam::Jacobi, 6.0 * double(m + k) * k * k / 2.0);
+  c.count(KFam::Jacobi, (sizeof(T) == 8 ? 6.0 : 24.0) * double(m + k) * k * k / 2.0);
+}
+
+}  // namespace
+
+bool jacobi_cluster_fits(int m, int k) { return fits(m, k, 1, kJMaxRowsPerLane); }
+bool jacobi_cluster_c_fits(int m, int k) { return fits(m, k, 2, 8); }
+
+void jacobi_svd_cluster(Ctx& c, double* X, int m, int k, int64_t ldx, double* J, int64_t ldj, double* S,
+                        int max_sweeps, double tol, int* d_sweeps) {
+  IPEPS_CHECK(jacobi_cluster_fits(m, k), "jacobi_svd_cluster: problem does not fit");
+  svd_cluster<double>(c, X, m, k, ldx, J, ldj, S, max_sweeps, tol, d_sweeps);
+}
+
+void jacobi_c_svd_cluster(Ctx& c, void* X, int m, int k, int64_t ldx, void* J, int64_t ldj, double* S, int max_sweeps,
+                          double tol, int* d_sweeps) {
+  IPEPS_CHECK(jacobi_cluster_c_fits(m, k), "jacobi_c_svd_cluster: problem does not fit");
+  svd_cluster<double2>(c, X, m, k, ldx, J, ldj, S, max_sweeps, tol, d_sweeps);
 }
 
 }  // namespace ipeps

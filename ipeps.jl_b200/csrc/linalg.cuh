@@ -41,13 +41,18 @@ bool trsm_fits(int k);
 // Rrow (optional): the same R packed row by row as written by chol_blocked.
 void trsm_right_upper(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const double* R, int64_t ldr,
                       double* Q, int64_t ldq, const double* Rrow = nullptr);
-// The same pass for k <= 160 (cholqr_fits): R in packed 8 x 8 blocks of
+// The same pass for k <= kCholqrMax (cholqr_fits): R in packed 8 x 8 blocks of
 // cholqr_packed(k) doubles (16-byte aligned), the diagonal blocks inverted.  G
 // receives R (strict lower triangle zeroed) when write_g.
-bool cholqr_fits(int k);
+constexpr int kCholqrMax = 192;
+inline bool cholqr_fits(int k) { return k >= 1 && k <= kCholqrMax; }
 int64_t cholqr_packed(int k);
 void chol_packed(Ctx& c, double* G, int k, int64_t ldg, double shift_factor, double* Rpk, bool write_g);
 void trsm_packed(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const double* Rpk, double* Q, int64_t ldq);
+// the pass of a complex sketch of k columns, 2 k <= kCholqrMax: R packed as the real
+// 2k x 2k factor (cholqr_packed(2 k) doubles)
+void chol_packed_c(Ctx& c, const void* G, int k, int64_t ldg, double shift_factor, double* Rpk);
+void trsm_packed_c(Ctx& c, const void* Y, int64_t ldy, int64_t N, int k, const double* Rpk, void* Q, int64_t ldq);
 // jacobi_svd with X held in shared memory and J formed from the logged
 // rotations when it fits; tol <= 0 means m * eps
 void jacobi_svd_auto(Ctx& c, double* X, int m, int k, int64_t ldx, double* J, int64_t ldj, double* S,
@@ -57,6 +62,10 @@ void jacobi_svd_auto(Ctx& c, double* X, int m, int k, int64_t ldx, double* J, in
 bool jacobi_cluster_fits(int m, int k);
 void jacobi_svd_cluster(Ctx& c, double* X, int m, int k, int64_t ldx, double* J, int64_t ldj, double* S,
                         int max_sweeps, double tol, int* d_sweeps);
+// complex128 X and J
+bool jacobi_cluster_c_fits(int m, int k);
+void jacobi_c_svd_cluster(Ctx& c, void* X, int m, int k, int64_t ldx, void* J, int64_t ldj, double* S, int max_sweeps,
+                          double tol, int* d_sweeps);
 // Complex (complex128) counterparts for complex iPEPS tensors, one CTA each;
 // complex_small_fits(m, k) says whether all three fit in shared memory.
 bool complex_small_fits(int m, int k);

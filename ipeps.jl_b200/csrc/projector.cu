@@ -260,12 +260,19 @@ Tensor orth_c(Ctx& c, const Tensor& Y0, int passes) {
   Tensor Y = Y0;
   Tensor G = c.alloc(DType::C128, {k, k});
   const double u = 1.1102230246251565e-16;
+  const bool packed = cholqr_fits(2 * k);
+  Tensor Rpk = packed ? c.alloc(DType::F64, {cholqr_packed(2 * k)}) : Tensor();
   for (int pass = 0; pass < passes; ++pass) {
     gemm(c, DType::C128, 'C', 'N', k, k, N, cplx(1), Y.data(), N, Y.data(), N, cplx(0), G.data(), k, true);
     const double sf = (pass == 0) ? 11.0 * (double(N) * k + double(k) * (k + 1)) * u : 0.0;
-    chol_c(c, G.data(), k, k, sf);
     Tensor Yn = c.alloc(DType::C128, {N, k});
-    trsm_c(c, Y.data(), N, N, k, G.data(), k, Yn.data(), N);
+    if (packed) {
+      chol_packed_c(c, G.data(), k, k, sf, Rpk.f64());
+      trsm_packed_c(c, Y.data(), N, N, k, Rpk.f64(), Yn.data(), N);
+    } else {
+      chol_c(c, G.data(), k, k, sf);
+      trsm_c(c, Y.data(), N, N, k, G.data(), k, Yn.data(), N);
+    }
     Y = Yn;
   }
   return Y;

@@ -110,7 +110,7 @@ Tensor apply_left_T(Ctx& c, const Tensor& X, const MatRef& R, char op, PlaneCach
 
 // Orthonormalise the columns of Y (N x k) by shifted CholeskyQR; if Rout is
 // non-null it receives R with Y = Q R.
-// passes (k <= 160): receives the packed R of each pass, Y = Q R_last ... R_first.
+// factors (cholqr_fits(k)): receives the packed R of each pass, Y = Q R_last ... R_first.
 Tensor orth(Ctx& c, const Tensor& Y, int passes, Tensor* Rout, std::vector<Tensor>* factors = nullptr);
 
 }  // namespace ipeps

@@ -5,7 +5,7 @@
 //                     column-parallel, the trailing update is a register-tiled SYRK.
 //   trsm_right_upper  Q = Y R^-1, two rows of Y per warp (the rows are independent), at
 //                     most one CTA per SM, R staged row-major in each CTA's shared memory.
-//                     (Both for k > 160; sketches of up to 160 columns: cholqr.cu.)
+//                     (Both for k > kCholqrMax; narrower sketches: cholqr.cu.)
 //   jacobi_svd_auto   one-sided Jacobi with only X in shared memory; every rotation is
 //                     logged, and J = product of the rotations is formed afterwards by a
 //                     row-parallel kernel (each row of J sees the same rotation sequence).
@@ -534,7 +534,7 @@ void launch_trsm(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const d
 
 }  // namespace
 
-bool chol_fits(int k) { return k > 160 && chol_smem_doubles(k) * 8 <= kSmemMax; }
+bool chol_fits(int k) { return k > kCholqrMax && chol_smem_doubles(k) * 8 <= kSmemMax; }
 
 void chol_blocked(Ctx& c, double* G, int k, int64_t ldg, double shift_factor, double* Rrow) {
   IPEPS_CHECK(chol_fits(k), "chol_blocked: k out of range");
@@ -545,7 +545,7 @@ void chol_blocked(Ctx& c, double* G, int k, int64_t ldg, double shift_factor, do
   c.count(KFam::SmallLinalg, double(k) * k * k / 3.0);
 }
 
-bool trsm_fits(int k) { return k > 160 && k <= 256 && trsm_smem_bytes(k, trsm_warps(k)) <= kSmemMax; }
+bool trsm_fits(int k) { return k > kCholqrMax && k <= 256 && trsm_smem_bytes(k, trsm_warps(k)) <= kSmemMax; }
 
 void trsm_right_upper(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const double* R, int64_t ldr, double* Q,
                       int64_t ldq, const double* Rrow) {
@@ -553,7 +553,6 @@ void trsm_right_upper(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, co
   if (N == 0) return;
   ProfScope ps(c, KFam::SmallLinalg);
   switch ((k + 31) / 32) {
-    case 6: launch_trsm<6>(c, Y, ldy, N, k, R, ldr, Rrow, Q, ldq); break;
     case 7: launch_trsm<7>(c, Y, ldy, N, k, R, ldr, Rrow, Q, ldq); break;
     default: launch_trsm<8>(c, Y, ldy, N, k, R, ldr, Rrow, Q, ldq); break;
   }

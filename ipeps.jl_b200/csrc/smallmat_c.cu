@@ -2,7 +2,8 @@
 // complex iPEPS tensors (e.g. the honeycomb models of src/model/*.jl, whose
 // environments are ComplexF64).  Same algorithms as the real kernels in
 // smallmat.cu, written for the modest sketch widths these models use
-// (k <= ~118, one CTA):
+// (k <= ~118, one CTA).  Up to 96 columns the CholeskyQR passes run on the real
+// kernels (cholqr.cu), from 16 columns the Jacobi SVD on a cluster.
 //
 //   chol_c           G = R^H R (G Hermitian), right-looking, one column per step
 //   trsm_c           Q = Y R^-1, one warp per row of Y
@@ -248,6 +249,11 @@ __global__ void __launch_bounds__(1024) jacobi_c_kernel(double2* Xg, int m, int 
   }
 }
 
+// Sketch width from which the Jacobi SVD runs on a cluster of 8 CTAs (jacobi_cluster.cu).
+// Five or six sweeps on one CTA against the cluster: 67 us and 84 us at k = 10, 128 and
+// 107 at k = 18, 385 and 184 at k = 46, 812 and 377 at k = 66, 1701 and 487 at k = 90.
+constexpr int kClusterJacobiMinKC = 16;
+
 constexpr int kApplyCRows = 8;
 
 // J = product of the logged unitary column transforms, one warp per row of J.
@@ -318,6 +324,10 @@ void trsm_c(Ctx& c, const void* Y, int64_t ldy, int64_t N, int k, const void* R,
 void jacobi_c_svd(Ctx& c, void* X, int m, int k, int64_t ldx, void* J, int64_t ldj, double* S, int max_sweeps,
                   double tol, int* d_sweeps) {
   IPEPS_CHECK(jacc_smem(m, k) <= kSmemMaxC, "jacobi_c_svd: sketch too wide for shared memory");
+  if (k >= kClusterJacobiMinKC && jacobi_cluster_c_fits(m, k)) {
+    jacobi_c_svd_cluster(c, X, m, k, ldx, J, ldj, S, max_sweeps, tol, d_sweeps);
+    return;
+  }
   if (tol <= 0) tol = double(m) * 2.220446049250313e-16;
   g_jacc_attr.ensure(jacobi_c_kernel, int(kSmemMaxC));
   const int kk = (k + 1) & ~1;

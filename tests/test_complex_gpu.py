@@ -115,3 +115,32 @@ def test_real_projector_rank_deficient(engine, pkg):
     R1 = U @ np.diag(np.sqrt(s)) @ rng.standard_normal((N, N)) * 0.1
     R2 = np.linalg.solve(rng.standard_normal((N, N)) * 0.1, np.diag(np.sqrt(s)) @ V.T)
     _check_projector(pkg, engine, R1, R2, chi)
+
+
+@pytest.mark.parametrize("n", [2, 9, 15, 16, 17, 33, 40, 63, 66, 80, 81, 96, 97])
+def test_projector_complex_block_edges(engine, pkg, n):
+    """Complex CholeskyQR (the real kernels at twice the width up to 96 columns) and Jacobi (a cluster from
+    16 columns) at the widths where they change: n x n corners, the sketch is the whole space, singular values
+    1 .. 1e-3.  Bars as in test_projector_jacobi_block_edges: 20 n eps in the values; for P1 P2 that times
+    s_1 / s_n (1e3) and the inverse relative gap of the truncated pair (n / 6.9)."""
+    rng = np.random.default_rng(n)
+    eps = np.finfo(float).eps
+    s = np.logspace(0, -3, n)
+    U, V, Z = (np.linalg.qr(_crandn(rng, n, n))[0] for _ in range(3))
+    R1, R2 = (U * np.sqrt(s)) @ Z, Z.conj().T @ (np.sqrt(s)[:, None] * V.conj().T)
+    P1, P2, got = pkg.get_projector(R1, R2, n - 1, engine=engine)
+    assert got.shape == (n - 1,)
+    assert np.abs(got - s[:-1]).max() <= 20 * n * eps
+    ref = Z.conj().T[:, :-1] @ Z[:-1]
+    assert np.abs(P1 @ P2 - ref).max() <= 20 * n * eps * 1e3 * max(1.0, n / 6.9)
+
+
+@pytest.mark.parametrize("n,rank", [(66, 5), (90, 20)])
+def test_projector_complex_rank_deficient(engine, pkg, n, rank):
+    rng = np.random.default_rng(n)
+    R1 = _crandn(rng, n, rank) @ _crandn(rng, rank, n)
+    R2 = _crandn(rng, n, rank) @ _crandn(rng, rank, n)
+    s_ref = np.linalg.svd(R1 @ R2, compute_uv=False)
+    P1, P2, s = pkg.get_projector(R1, R2, rank, engine=engine)
+    assert np.isfinite(P1).all() and np.isfinite(P2).all()
+    assert np.abs(s[:rank] - s_ref[:rank]).max() <= 20 * n * np.finfo(float).eps * s_ref[0]
