@@ -59,12 +59,13 @@ struct Ctx {
   // small device scalars (max-abs, traces, status words)
   std::shared_ptr<DBuf> scal;
   int* d_status = nullptr;
-  // tile configuration and K split of the FP64 GEMM by (m, n, k, upper): chosen
-  // from an estimate over all of them, so kept (bounded: emptied at 4096 shapes)
+  // tile configuration and K split of the FP64 GEMMs by (m, n, k, kind: 0 real, 1 to 3
+  // complex with both, the first, the second operand complex, 4 real upper triangle):
+  // chosen from an estimate over all of them, so kept (bounded: emptied at 4096 shapes)
   struct GemmPlan {
     int config = 0, S = 1, cs = 1;
   };
-  std::map<std::tuple<int64_t, int64_t, int64_t, bool>, GemmPlan> gemm_plans;
+  std::map<std::tuple<int64_t, int64_t, int64_t, int>, GemmPlan> gemm_plans;
   // per-kernel-family CUDA-event timing (enabled by ipeps_prof_enable)
   bool prof = false;
   // with prof: wall ms of the E+grad pullback's phases (checkpoint iterations,
@@ -159,7 +160,7 @@ Tensor clone(Ctx& c, const Tensor& in);
 void gemm(Ctx& c, DType dt, char opA, char opB, int64_t m, int64_t n, int64_t k,
           cuDoubleComplex alpha, const void* A, int64_t lda, const void* B, int64_t ldb,
           cuDoubleComplex beta, void* C, int64_t ldc, bool force_fp64 = false);
-// FP64 GEMM: DMMA for real operands, register-tiled SIMT for complex128
+// FP64 GEMM on the DMMA path: real, or complex128
 void gemm_f64(Ctx& c, DType dt, char opA, char opB, int64_t m, int64_t n, int64_t k,
               cuDoubleComplex alpha, const void* A, int64_t lda, const void* B, int64_t ldb,
               cuDoubleComplex beta, void* C, int64_t ldc);
@@ -168,6 +169,10 @@ void gemm_f64(Ctx& c, DType dt, char opA, char opB, int64_t m, int64_t n, int64_
 void gemm_f64_dmma(Ctx& c, char opA, char opB, int64_t m, int64_t n, int64_t k, double alpha, const double* A,
                    int64_t lda, const double* B, int64_t ldb, double beta, double* C, int64_t ldc,
                    bool upper = false);
+// complex128 GEMM on the DMMA path, op in {N, T, C}; one operand may be real (dtA or dtB F64)
+void gemm_c128_dmma(Ctx& c, char opA, DType dtA, char opB, DType dtB, int64_t m, int64_t n, int64_t k,
+                    cuDoubleComplex alpha, const void* A, int64_t lda, const void* B, int64_t ldb, cuDoubleComplex beta,
+                    void* C, int64_t ldc);
 // 3xTF32 tcgen05 GEMM for real operands (FP32-accumulated split products)
 // BF16 operands (rounded from FP32 while staged), FP32 accumulation and result; op in {N, T}
 void gemm_bf16(Ctx& c, char opA, char opB, int64_t m, int64_t n, int64_t k, float alpha, const float* A, int64_t lda,

@@ -26,11 +26,9 @@
 // Back-to-back launches, before -> now: 120 x 62 x 120 9.5 -> 6.3 us, 333 x 76 x
 // 333 14.5 -> 8.3, Gram 160 x 160 x 2500 26 -> 12.4 (upper triangle), 1024 x 128 x
 // 1024 25 -> 17, 2500 x 160 x 2500 113 -> 80, 2500 x 200 x 2500 140 -> 101.
-#include "ctx.cuh"
+#include "dmma.cuh"
 
-#include <algorithm>
 #include <atomic>
-#include <cmath>
 #include <iterator>
 #include <mutex>
 
@@ -39,123 +37,12 @@
 namespace ipeps {
 namespace {
 
-constexpr int kBK = 16;
-constexpr int kStages = 3;
-constexpr int kPad = 4;
-
-__device__ __forceinline__ unsigned su32(const void* p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ int64_t imin(int64_t a, int64_t b) { return a < b ? a : b; }
-__device__ __forceinline__ int64_t imax(int64_t a, int64_t b) { return a > b ? a : b; }
-
-template <int VEC>
-__device__ __forceinline__ void cp_async(double* dst, const double* src, int bytes) {
-  if constexpr (VEC == 2) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(su32(dst)), "l"(src), "r"(bytes));
-  } else {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(su32(dst)), "l"(src), "r"(bytes));
-  }
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
-
-__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
-
-// Shared-memory geometry of one operand tile (BMN rows of the m or n index).
-template <int BMN, bool KMAJ>
-struct Tile {
-  static constexpr int ld = KMAJ ? (kBK + kPad) : (BMN + kPad);  // doubles per stored row
-  static constexpr int size = KMAJ ? BMN * ld : kBK * ld;         // doubles per stage
-  // element (mn, k) of the tile
-  static __device__ __forceinline__ int at(int mn, int k) { return KMAJ ? mn * ld + k : k * ld + mn; }
-};
-
-// Copy the operand tile [mn0, mn0 + BMN) x [k0, k0 + 16) into shared memory.
-// Global layout: KMAJ: element (mn, k) at P[k + mn * ld]; else at P[mn + k * ld].
-template <int BMN, bool KMAJ, int VEC, int NT>
-__device__ __forceinline__ void load_tile(double* s, const double* __restrict__ P, int64_t ldp, int64_t MN,
-                                          int64_t mn0, int64_t k0, int64_t ke, int tid) {
-  using T = Tile<BMN, KMAJ>;
-  constexpr int inner = KMAJ ? kBK : BMN;  // contiguous extent
-  constexpr int outer = KMAJ ? BMN : kBK;
-  constexpr int chunks = inner / VEC * outer;
-#pragma unroll
-  for (int r = 0; r < (chunks + NT - 1) / NT; ++r) {
-    const int e = tid + r * NT;
-    if (chunks % NT != 0 && e >= chunks) break;
-    const int i = (e % (inner / VEC)) * VEC, o = e / (inner / VEC);
-    const int mn = KMAJ ? o : i, k = KMAJ ? i : o;
-    const int64_t gmn = mn0 + mn, gk = k0 + k;
-    int64_t valid;
-    const double* src;
-    if (KMAJ) {
-      valid = (gmn < MN) ? imin(VEC, imax(0, ke - gk)) : 0;
-      src = P + gk + gmn * ldp;
-    } else {
-      valid = (gk < ke) ? imin(VEC, imax(0, MN - gmn)) : 0;
-      src = P + gmn + gk * ldp;
-    }
-    if (valid == 0) src = P;  // any valid address; nothing is read
-    cp_async<VEC>(s + T::at(mn, k), src, int(valid) * 8);
-  }
-}
-
-// The same for a thread's chunks of successive tiles along k: one pointer that
-// moves with k, the chunks a fixed number of rows apart (the address arithmetic of
-// load_tile, per chunk and tile, cost the issue slots of ~10% of the products).
-template <int BMN, bool KMAJ, int VEC, int NT>
-struct Loader {
-  using T = Tile<BMN, KMAJ>;
-  static constexpr int inner = (KMAJ ? kBK : BMN) / VEC, outer = KMAJ ? BMN : kBK;
-  static constexpr bool regular = NT % inner == 0;
-  static constexpr int step = regular ? NT / inner : 1;  // rows between a thread's chunks
-  const double* P;
-  const double* p;
-  int64_t ldp, MN, mn0;
-  int i, o, mn_left;
-  __device__ __forceinline__ Loader(const double* P_, int64_t ld, int64_t MN_, int64_t mn0_, int64_t k0, int tid)
-      : P(P_), ldp(ld), MN(MN_), mn0(mn0_) {
-    i = (tid % inner) * VEC;
-    o = tid / inner;
-    mn_left = int(imin(MN - mn0, BMN));
-    p = KMAJ ? P + (k0 + i) + (mn0 + o) * ldp : P + (mn0 + i) + (k0 + o) * ldp;
-  }
-  // tile at k0 (its k's below ke) into s; then on to the next 16 k
-  __device__ __forceinline__ void next(double* s, int64_t k0, int64_t ke, int tid) {
-    if constexpr (!regular) {
-      load_tile<BMN, KMAJ, VEC, NT>(s, P, ldp, MN, mn0, k0, ke, tid);
-    } else {
-      const int k_left = int(imin(ke - k0, kBK));
-      const int in_left = (KMAJ ? k_left : mn_left) - i, out_left = KMAJ ? mn_left : k_left;
-      const int bytes = 8 * max(0, min(VEC, in_left));
-      double* d = s + (KMAJ ? T::at(o, i) : T::at(i, o));
-#pragma unroll
-      for (int r = 0; r < (outer + step - 1) / step; ++r) {
-        const int row = o + r * step;
-        if (outer % step != 0 && row >= outer) break;
-        const int n = row < out_left ? bytes : 0;
-        cp_async<VEC>(d + r * step * T::ld, n ? p + int64_t(r * step) * ldp : P, n);
-      }
-      p += KMAJ ? int64_t(kBK) : kBK * ldp;
-    }
-  }
-};
-
 // Warps: WGM x WGN over the tile, times KW over the 16 k of a stage (each of the
 // KW sums 16 / KW of them; the sums meet in shared memory at the end).
 template <int BM, int BN, int WGM, int WGN, int KW, bool AK, bool BK_>
 struct Geo {
   static constexpr int NT = WGM * WGN * KW * 32;
-  static constexpr int ring = kStages * (Tile<BM, AK>::size + Tile<BN, BK_>::size);  // doubles
+  static constexpr int ring = kStages * (Tile<double, BM, AK>::size + Tile<double, BN, BK_>::size);  // doubles
   static constexpr int sums = (KW > 1 ? KW - 1 : 1) * BM * BN;  // KW sums, then the tile for the cluster's sum
   static constexpr size_t smem = size_t(ring > sums ? ring : sums) * sizeof(double);
 };
@@ -175,8 +62,8 @@ __global__ void __launch_bounds__(WGM * WGN * KW * 32, MINB)
   constexpr int NT = GE::NT;
   constexpr int WM = BM / WGM, WN = BN / WGN;  // warp tile
   constexpr int TI = WM / 8, TJ = WN / 8;      // 8x8 DMMA tiles per warp
-  using TA = Tile<BM, AK>;
-  using TB = Tile<BN, BK_>;
+  using TA = Tile<double, BM, AK>;
+  using TB = Tile<double, BN, BK_>;
   extern __shared__ __align__(16) double smem[];
   double* sA = smem;
   double* sB = smem + kStages * TA::size;
@@ -198,8 +85,8 @@ __global__ void __launch_bounds__(WGM * WGN * KW * 32, MINB)
     for (int j = 0; j < TJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
   // B is consumed as (k, n): its "mn" index is n and it is k-contiguous when op(B) = N
-  Loader<BM, AK, VEC, NT> la(A, lda, M, m0, kb, tid);
-  Loader<BN, BK_, VEC, NT> lb(B, ldb, N, n0, kb, tid);
+  Loader<double, BM, AK, VEC, NT> la(A, lda, M, m0, kb, tid);
+  Loader<double, BN, BK_, VEC, NT> lb(B, ldb, N, n0, kb, tid);
 #pragma unroll
   for (int s = 0; s < kStages - 1; ++s) {
     if (s < nk) {
@@ -379,28 +266,6 @@ struct Split {
   int S = 1, cs = 1;
 };
 
-// CTAs of one kernel that run at the same time in clusters of cs, asked of the
-// driver once per kernel, cluster size and device: clusters need their SMs in one
-// GPC, so the larger ones leave some idle (128 x 80 tiles in clusters of 7: 40
-// clusters did not run at once on 148 SMs x 2, 117 us instead of 81).
-template <class K>
-int resident(K kern, int threads, size_t smem, int cs) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(1, 1, unsigned(cs));
-  cfg.blockDim = dim3(unsigned(threads));
-  cfg.dynamicSmemBytes = smem;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = 1;
-  at.val.clusterDim.y = 1;
-  at.val.clusterDim.z = unsigned(cs);
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  int n = 0;
-  IPEPS_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
-  return n * cs;
-}
-
 template <int BM, int BN, int WGM, int WGN, int KW, int MINB, bool AK, bool BK_, int VEC>
 void launch_cfg(Ctx& c, const Args& a, Split sp) {
   using GE = Geo<BM, BN, WGM, WGN, KW, AK, BK_>;
@@ -452,8 +317,6 @@ void launch_ops(Ctx& c, const Args& a, Split sp) {
 #undef IPEPS_DMMA_CASE
 }
 
-constexpr int kMaxCluster = 8;
-
 template <int BM, int BN, int WGM, int WGN, int KW, int MINB>
 int resident_cfg(int cs) {
   using GE = Geo<BM, BN, WGM, WGN, KW, true, true>;
@@ -468,8 +331,8 @@ int resident_cfg(int cs) {
 // 1024: 8.3 and 12.4), 64 x 32 for the sketches (2500 x 160 x 2500: 80 us, 64 x 64:
 // 90), 64 x 64 for large ones (4096^3: 4.06 ms, 128 x 80: 4.23), the 128-row tiles
 // for narrow outputs (a leg of D^2 d = 50: 128 x 64, 59.5 us at 250000 x 50 x 25,
-// 64 x 32: 81).  pipe: share of the FP64 pipe's rate that a full SM reaches, step:
-// cycles that one CTA alone needs per K step (see estimate).
+// 64 x 32: 81).  pipe, step: cycles of one K step (see split_cost; the
+// pipe at the share of its rate that a full SM reaches).
 struct Config {
   int bm, bn;
   double pipe, step;
@@ -477,12 +340,12 @@ struct Config {
   int (*resident)(int);
 };
 const Config kConfigs[] = {
-    {32, 32, 0.80, 520, launch_ops<32, 32, 1, 1, 4, 4>, resident_cfg<32, 32, 1, 1, 4, 4>},
-    {64, 32, 0.86, 830, launch_ops<64, 32, 2, 1, 2, 4>, resident_cfg<64, 32, 2, 1, 2, 4>},
-    {64, 64, 0.89, 1500, launch_ops<64, 64, 2, 2, 1, 3>, resident_cfg<64, 64, 2, 2, 1, 3>},
-    {128, 48, 0.80, 1900, launch_ops<128, 48, 8, 1, 1, 2>, resident_cfg<128, 48, 8, 1, 1, 2>},
-    {128, 64, 0.81, 2500, launch_ops<128, 64, 8, 1, 1, 2>, resident_cfg<128, 64, 8, 1, 1, 2>},
-    {128, 80, 0.81, 3150, launch_ops<128, 80, 8, 1, 1, 2>, resident_cfg<128, 80, 8, 1, 1, 2>},
+    {32, 32, 1024 / (4 * 0.80), 520, launch_ops<32, 32, 1, 1, 4, 4>, resident_cfg<32, 32, 1, 1, 4, 4>},
+    {64, 32, 2048 / (4 * 0.86), 830, launch_ops<64, 32, 2, 1, 2, 4>, resident_cfg<64, 32, 2, 1, 2, 4>},
+    {64, 64, 4096 / (4 * 0.89), 1500, launch_ops<64, 64, 2, 2, 1, 3>, resident_cfg<64, 64, 2, 2, 1, 3>},
+    {128, 48, 6144 / (4 * 0.80), 1900, launch_ops<128, 48, 8, 1, 1, 2>, resident_cfg<128, 48, 8, 1, 1, 2>},
+    {128, 64, 8192 / (4 * 0.81), 2500, launch_ops<128, 64, 8, 1, 1, 2>, resident_cfg<128, 64, 8, 1, 1, 2>},
+    {128, 80, 10240 / (4 * 0.81), 3150, launch_ops<128, 80, 8, 1, 1, 2>, resident_cfg<128, 80, 8, 1, 1, 2>},
 };
 constexpr int kNumConfigs = int(std::size(kConfigs));
 
@@ -501,46 +364,13 @@ const Residency& residency(int device) {
   return q;
 }
 
-// Estimated cycles of a configuration with S K chunks in clusters of cs: waves of
-// CTAs, each as long as its steps take on the fullest SM.  The constants are fitted
-// to a sweep of all configurations and splits over 151 shapes (D = 2 to 5, chi = 9 to
-// 100): the choice is 2.3% slower than the best of the sweep on average.
-double estimate(const Config& f, const Args& a, int sms, int slots, int S, int cs) {
-  const double gx = double((a.m + f.bm - 1) / f.bm), gy = double((a.n + f.bn - 1) / f.bn);
-  const double tiles = a.upper ? 0.5 * gx * gy + 0.5 * std::max(gx, gy) : gx * gy;
-  const double steps = std::ceil(std::ceil(double(a.k) / kBK) / S), ctas = tiles * S;
-  const double tile = f.bm * f.bn / (4.0 * f.pipe);  // one step of one CTA on the FP64 pipe of its SM
-  const double waves = std::floor(ctas / slots), rest = ctas - waves * slots;
-  const double full = std::max(1.0, double(slots) / sms);
-  // a cluster's CTAs share SMs sooner than the same number of single ones
-  const double part = std::min(full, std::ceil(rest / sms) * (cs > 1 ? 1.0 + 0.025 * (cs - 1) : 1.0));
-  double t = waves * (steps * std::max(full * tile, f.step) + 4100.0);
-  if (rest > 0) t += steps * std::max(part * tile, f.step) + 4100.0;
-  if (cs > 1) t = t * (cs > 2 && waves >= 1 ? 1.04 : 1.0) + (waves + 1) * (1300.0 + 0.43 * f.bm * f.bn);
-  if (S > cs) t += 7000.0 + (S / cs) * (106.0 + double(a.m) * double(a.n) * 16.0 / 9400.0);
-  return t;
-}
-
 Ctx::GemmPlan plan(Ctx& c, const Args& a) {
-  const auto key = std::make_tuple(a.m, a.n, a.k, a.upper);
+  const auto key = std::make_tuple(a.m, a.n, a.k, a.upper ? 4 : 0);
   const auto it = c.gemm_plans.find(key);
   if (it != c.gemm_plans.end()) return it->second;
   const Residency& res = residency(c.device);
-  Ctx::GemmPlan best;
-  double t = -1.0;
-  for (int f = 0; f < kNumConfigs; ++f)
-    for (int S = 1; S <= 1024; S = S < 8 ? S + 1 : 2 * S) {
-      if (S > 1 && int64_t(S) * 2 * kBK > a.k) break;
-      for (int cs : {std::min(S, kMaxCluster), 1}) {
-        if ((cs & (cs - 1)) != 0) continue;  // clusters of 3, 5, 6, 7 measured behind those of 2, 4, 8
-        if (cs == 1 && S > 1 && double(S) * double(a.m) * double(a.n) > 5e7) break;  // at most 400 MB of partial sums
-        const double e = estimate(kConfigs[f], a, c.sm_count, res.n[f][cs], S, cs);
-        if (t < 0 || e < t) {
-          best = {f, S, cs};
-          t = e;
-        }
-      }
-    }
+  const Ctx::GemmPlan best = best_split(kConfigs, kNumConfigs, [&](int f, int cs) { return res.n[f][cs]; }, c.sm_count,
+                                        a.m, a.n, a.k, 8, a.upper);
   if (c.gemm_plans.size() >= 4096) c.gemm_plans.clear();
   c.gemm_plans[key] = best;
   return best;

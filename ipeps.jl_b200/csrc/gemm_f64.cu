@@ -1,11 +1,8 @@
-// Complex128 GEMM for sm_100a (and the real FP64 kernel of the allocation-free
-// entry point): register-tiled SIMT FMA kernel.  Real FP64 products of the
-// engine go to the DMMA kernel (gemm_dmma.cu).  Tiles:
-//   real     64x64x16, 4x4 outputs per thread (allocation-free entry point)
-//   complex  64x64x8,  4x4 outputs per thread
-// Operands are staged through shared memory with one register prefetch stage.
-// Skinny problems (few output tiles, long K) use a deterministic split-K:
-// partial products go to a workspace and are summed in a fixed order.
+// Dispatch of the FP64 GEMMs (real: gemm_dmma.cu, complex128: gemm_zmma.cu), and the
+// real register-tiled FMA kernel of the allocation-free entry point: 64x64x16 tiles,
+// 4x4 outputs per thread, operands staged through shared memory with one register
+// prefetch stage, deterministic split-K for skinny problems (few output tiles, long
+// K): partial products go to a fixed scratch array and are summed in a fixed order.
 #include "ctx.cuh"
 
 #include <algorithm>
@@ -13,44 +10,20 @@
 namespace ipeps {
 namespace {
 
-__device__ __forceinline__ double cj(double x) { return x; }
-__device__ __forceinline__ cuDoubleComplex cj(cuDoubleComplex x) { return cuConj(x); }
-__device__ __forceinline__ void fma_acc(double& acc, double a, double b) { acc = fma(a, b, acc); }
-__device__ __forceinline__ void fma_acc(cuDoubleComplex& acc, cuDoubleComplex a, cuDoubleComplex b) {
-  acc.x = fma(a.x, b.x, acc.x);
-  acc.x = fma(-a.y, b.y, acc.x);
-  acc.y = fma(a.x, b.y, acc.y);
-  acc.y = fma(a.y, b.x, acc.y);
-}
-template <typename T> __device__ __forceinline__ T zero();
-template <> __device__ __forceinline__ double zero<double>() { return 0.0; }
-template <> __device__ __forceinline__ cuDoubleComplex zero<cuDoubleComplex>() {
-  return make_cuDoubleComplex(0, 0);
-}
-__device__ __forceinline__ double mulS(double a, cuDoubleComplex s) { return a * s.x; }
-__device__ __forceinline__ cuDoubleComplex mulS(cuDoubleComplex a, cuDoubleComplex s) {
-  return cuCmul(a, s);
-}
-__device__ __forceinline__ double addv(double a, double b) { return a + b; }
-__device__ __forceinline__ cuDoubleComplex addv(cuDoubleComplex a, cuDoubleComplex b) {
-  return cuCadd(a, b);
-}
-__device__ __forceinline__ bool is_zero(cuDoubleComplex s) { return s.x == 0.0 && s.y == 0.0; }
-
-// op codes: 0 = N, 1 = T, 2 = C (conjugate transpose)
-template <typename T, int BM, int BN, int BK, int TM, int TN>
+// op codes: 0 = N, 1 = T
+template <int BM, int BN, int BK, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
     gemm_kernel(int opA, int opB, int64_t M, int64_t N, int64_t K, int64_t kchunk,
-                cuDoubleComplex alpha, const T* __restrict__ A, int64_t lda,
-                const T* __restrict__ B, int64_t ldb, cuDoubleComplex beta, T* __restrict__ C,
-                int64_t ldc, T* __restrict__ partial) {
+                double alpha, const double* __restrict__ A, int64_t lda,
+                const double* __restrict__ B, int64_t ldb, double beta, double* __restrict__ C,
+                int64_t ldc, double* __restrict__ partial) {
   constexpr int NT = (BM / TM) * (BN / TN);
   constexpr int TX = BM / TM;  // threads along m
   constexpr int A_PER = BM * BK / NT;
   constexpr int B_PER = BN * BK / NT;
   static_assert(A_PER >= 1 && B_PER >= 1, "tile too small");
-  __shared__ T As[2][BK][BM + 1];
-  __shared__ T Bs[2][BK][BN + 1];
+  __shared__ double As[2][BK][BM + 1];
+  __shared__ double Bs[2][BK][BN + 1];
 
   const int tid = threadIdx.x;
   const int tx = tid % TX, ty = tid / TX;
@@ -59,13 +32,13 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
   const int64_t kb = int64_t(blockIdx.z) * kchunk;
   const int64_t ke = min(K, kb + kchunk);
 
-  T acc[TM][TN];
+  double acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = zero<T>();
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.0;
 
-  T ra[A_PER], rb[B_PER];
+  double ra[A_PER], rb[B_PER];
 
   auto load_a = [&](int64_t k0) {
 #pragma unroll
@@ -75,10 +48,9 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
       if (opA == 0) { mi = e % BM; ki = e / BM; }
       else { ki = e % BK; mi = e / BK; }
       int64_t gm = m0 + mi, gk = k0 + ki;
-      T v = zero<T>();
+      double v = 0.0;
       if (gm < M && gk < ke) {
         v = (opA == 0) ? A[gm + gk * lda] : A[gk + gm * lda];
-        if (opA == 2) v = cj(v);
       }
       ra[r] = v;
     }
@@ -91,10 +63,9 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
       if (opB == 0) { ki = e % BK; ni = e / BK; }
       else { ni = e % BN; ki = e / BN; }
       int64_t gn = n0 + ni, gk = k0 + ki;
-      T v = zero<T>();
+      double v = 0.0;
       if (gn < N && gk < ke) {
         v = (opB == 0) ? B[gk + gn * ldb] : B[gn + gk * ldb];
-        if (opB == 2) v = cj(v);
       }
       rb[r] = v;
     }
@@ -133,7 +104,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
     }
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
-      T a[TM], b[TN];
+      double a[TM], b[TN];
 #pragma unroll
       for (int i = 0; i < TM; ++i) a[i] = As[buf][kk][tx + i * TX];
 #pragma unroll
@@ -141,7 +112,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) fma_acc(acc[i][j], a[i], b[j]);
+        for (int j = 0; j < TN; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
     }
     if (more) {
       store(buf ^ 1);
@@ -162,25 +133,24 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
       if (partial) {
         partial[int64_t(blockIdx.z) * M * N + gm + gn * M] = acc[i][j];
       } else {
-        T v = mulS(acc[i][j], alpha);
-        if (!is_zero(beta)) v = addv(v, mulS(C[gm + gn * ldc], beta));
+        double v = acc[i][j] * alpha;
+        if (beta != 0.0) v += C[gm + gn * ldc] * beta;
         C[gm + gn * ldc] = v;
       }
     }
   }
 }
 
-template <typename T>
-__global__ void splitk_reduce(int64_t M, int64_t N, int S, const T* __restrict__ partial,
-                              cuDoubleComplex alpha, cuDoubleComplex beta, T* __restrict__ C,
+__global__ void splitk_reduce(int64_t M, int64_t N, int S, const double* __restrict__ partial,
+                              double alpha, double beta, double* __restrict__ C,
                               int64_t ldc) {
   int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= M * N) return;
   int64_t gm = idx % M, gn = idx / M;
-  T s = partial[idx];
-  for (int z = 1; z < S; ++z) s = addv(s, partial[int64_t(z) * M * N + idx]);
-  T v = mulS(s, alpha);
-  if (!is_zero(beta)) v = addv(v, mulS(C[gm + gn * ldc], beta));
+  double s = partial[idx];
+  for (int z = 1; z < S; ++z) s += partial[int64_t(z) * M * N + idx];
+  double v = s * alpha;
+  if (beta != 0.0) v += C[gm + gn * ldc] * beta;
   C[gm + gn * ldc] = v;
 }
 
@@ -191,44 +161,6 @@ int opcode(char o) {
     case 'C': case 'c': return 2;
   }
   throw Error(kEInval, "gemm: bad op");
-}
-
-template <typename T, int BM, int BN, int BK, int TM, int TN>
-void launch(Ctx& c, int oa, int ob, int64_t m, int64_t n, int64_t k, cuDoubleComplex alpha,
-            const void* A, int64_t lda, const void* B, int64_t ldb, cuDoubleComplex beta, void* C,
-            int64_t ldc) {
-  constexpr int NT = (BM / TM) * (BN / TN);
-  int64_t gx = (m + BM - 1) / BM, gy = (n + BN - 1) / BN;
-  IPEPS_CHECK(gy <= 65535, "gemm: n too large for grid");
-  int64_t tiles = gx * gy;
-  int S = 1;
-  // split K when the output grid covers well under two waves and K is long
-  const int64_t target = 2LL * c.sm_count;
-  if (tiles < target && k >= 8 * BK * 2) {
-    int64_t want = (target + tiles - 1) / tiles;
-    int64_t maxs = k / (8 * BK);
-    S = int(std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, maxs), 64)));
-  }
-  int64_t kchunk = (k + S - 1) / S;
-  kchunk = ((kchunk + BK - 1) / BK) * BK;
-  S = int((k + kchunk - 1) / kchunk);
-  if (S < 1) S = 1;
-  ProfScope ps(c, KFam::GemmF64);
-  T* partial = nullptr;
-  if (S > 1) partial = static_cast<T*>(c.workspace(size_t(S) * m * n * sizeof(T)));
-  dim3 grid{unsigned(gx), unsigned(gy), unsigned(S)};
-  gemm_kernel<T, BM, BN, BK, TM, TN><<<grid, NT, 0, c.stream>>>(
-      oa, ob, m, n, k, kchunk, alpha, static_cast<const T*>(A), lda, static_cast<const T*>(B),
-      ldb, beta, static_cast<T*>(C), ldc, partial);
-  IPEPS_LAUNCH_CHECK();
-  c.count(KFam::GemmF64, (sizeof(T) == 8 ? 2.0 : 8.0) * double(m) * double(n) * double(k));
-  if (S > 1) {
-    int64_t tot = m * n;
-    splitk_reduce<T><<<unsigned((tot + 255) / 256), 256, 0, c.stream>>>(
-        m, n, S, partial, alpha, beta, static_cast<T*>(C), ldc);
-    IPEPS_LAUNCH_CHECK();
-    c.count(KFam::Reduce, 0, double(S + 2) * tot * sizeof(T));
-  }
 }
 
 }  // namespace
@@ -244,8 +176,7 @@ void gemm_f64(Ctx& c, DType dt, char opA, char opB, int64_t m, int64_t n, int64_
     gemm_f64_dmma(c, opA, opB, m, n, k, alpha.x, static_cast<const double*>(A), lda, static_cast<const double*>(B),
                   ldb, beta.x, static_cast<double*>(C), ldc);
   } else {
-    launch<cuDoubleComplex, 64, 64, 8, 4, 4>(c, oa, ob, m, n, k, alpha, A, lda, B, ldb, beta, C,
-                                             ldc);
+    gemm_c128_dmma(c, opA, dt, opB, dt, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
   }
 }
 
@@ -344,14 +275,13 @@ extern "C" int ipeps_gemm_f64_noalloc(char opA, char opB, int64_t m, int64_t n, 
   kchunk = ((kchunk + BK - 1) / BK) * BK;
   S = (k + kchunk - 1) / kchunk;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const cuDoubleComplex a = make_cuDoubleComplex(alpha, 0), b = make_cuDoubleComplex(beta, 0);
   dim3 grid{unsigned(gx), unsigned(gy), unsigned(S)};
-  gemm_kernel<double, BM, BN, BK, TM, TN><<<grid, NT, 0, st>>>(oa, ob, m, n, k, kchunk, a, A, lda, B, ldb, b, C, ldc,
+  gemm_kernel<BM, BN, BK, TM, TN><<<grid, NT, 0, st>>>(oa, ob, m, n, k, kchunk, alpha, A, lda, B, ldb, beta, C, ldc,
                                                                 S > 1 ? scratch : nullptr);
   if (cudaGetLastError() != cudaSuccess) return IPEPS_ECUDA;
   if (S > 1) {
     const int64_t tot = m * n;
-    splitk_reduce<double><<<unsigned((tot + 255) / 256), 256, 0, st>>>(m, n, int(S), scratch, a, b, C, ldc);
+    splitk_reduce<<<unsigned((tot + 255) / 256), 256, 0, st>>>(m, n, int(S), scratch, alpha, beta, C, ldc);
     if (cudaGetLastError() != cudaSuccess) return IPEPS_ECUDA;
   }
   return IPEPS_OK;
