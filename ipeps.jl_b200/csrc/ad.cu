@@ -332,30 +332,90 @@ void Tape::backward() {
   ops_.clear();
 }
 
-AV ad_tcon(Tape& tp, const AV& a, const std::vector<int>& la, const AV& b, const std::vector<int>& lb) {
-  Ctx& c = tp.ctx();
-  AV out{tcon(c, a.t, la, b.t, lb), -1};
-  if (a.id < 0 && b.id < 0) return out;
-  out.id = tp.newid();
-  const int nout = out.t.nd;
-  // dA = tcon(dC, lcA, B, lbA): output in A's leg order; B's free labels are summed
-  std::vector<int> lcA(nout), lbA(lb.size()), lcB(nout), laB(la.size());
-  for (int j = 0; j < nout; ++j) {
-    const int l = -(j + 1);
-    const int p = findl(la, l), q = findl(lb, l);
-    lcA[j] = (p >= 0) ? -(p + 1) : 1000 + (j + 1);
-    lcB[j] = (q >= 0) ? -(q + 1) : 2000 + (j + 1);
+namespace {
+
+__global__ void real_part_kernel(const double2* x, double* y, int64_t n) {
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+    y[i] = x[i].x;
+}
+
+// the cotangent of a real variable from a possibly complex one: its real part
+Tensor real_of(Ctx& c, const Tensor& x) {
+  if (x.empty() || x.dt == DType::F64) return x;
+  Tensor y = c.alloc(DType::F64, x.shape());
+  const int64_t n = x.numel();
+  const unsigned g = unsigned(std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, int64_t(c.sm_count) * 8)));
+  real_part_kernel<<<g, 256, 0, c.stream>>>(static_cast<const double2*>(x.data()), y.f64(), n);
+  IPEPS_LAUNCH_CHECK();
+  return y;
+}
+
+// labels of dA = tcon(dC, lcA, B, lbA) (output in A's leg order, B's free labels
+// summed) and of dB = tcon(A, laB, dC, lcB)
+struct BackLabels {
+  std::vector<int> lcA, lbA, lcB, laB;
+  BackLabels(int nout, const std::vector<int>& la, const std::vector<int>& lb)
+      : lcA(nout), lbA(lb.size()), lcB(nout), laB(la.size()) {
+    for (int j = 0; j < nout; ++j) {
+      const int l = -(j + 1);
+      const int p = findl(la, l), q = findl(lb, l);
+      lcA[j] = (p >= 0) ? -(p + 1) : 1000 + (j + 1);
+      lcB[j] = (q >= 0) ? -(q + 1) : 2000 + (j + 1);
+    }
+    for (size_t q = 0; q < lb.size(); ++q) lbA[q] = (lb[q] > 0) ? -(findl(la, lb[q]) + 1) : 1000 - lb[q];
+    for (size_t p = 0; p < la.size(); ++p) laB[p] = (la[p] > 0) ? -(findl(lb, la[p]) + 1) : 2000 - la[p];
   }
-  for (size_t q = 0; q < lb.size(); ++q) lbA[q] = (lb[q] > 0) ? -(findl(la, lb[q]) + 1) : 1000 - lb[q];
-  for (size_t p = 0; p < la.size(); ++p) laB[p] = (la[p] > 0) ? -(findl(lb, la[p]) + 1) : 2000 - la[p];
-  Tensor at = a.t, bt = b.t;
-  const int ia = a.id, ib = b.id, io = out.id;
-  tp.push([&tp, at, bt, ia, ib, io, lcA, lbA, lcB, laB]() {
+};
+
+}  // namespace
+
+AV ad_tcon(Tape& tp, const AV& a, const std::vector<int>& la, const AV& b, const std::vector<int>& lb) {
+  Contraction p(a.t, la, b.t, lb);
+  return ad_tcon_sum(tp, p, {{a, b}}, la, lb);
+}
+
+AV ad_tcon_sum(Tape& tp, Contraction& p, const std::vector<std::pair<AV, AV>>& terms, const std::vector<int>& la,
+               const std::vector<int>& lb) {
+  Ctx& c = tp.ctx();
+  Tensor raw;
+  bool var = false;
+  for (const auto& t : terms) {
+    p.add(c, raw, t.first.t, t.second.t);
+    var = var || t.first.id >= 0 || t.second.id >= 0;
+  }
+  AV out{p.finish(c, raw), -1};
+  if (!var) return out;
+  out.id = tp.newid();
+  const int io = out.id;
+  BackLabels bl(out.t.nd, la, lb);
+  tp.push([&tp, terms, io, bl]() {
     const Tensor& g = tp.grad(io);
     if (g.empty()) return;
     Ctx& c = tp.ctx();
-    if (ia >= 0) tp.acc(ia, tcon(c, g, lcA, bt.dt == DType::C128 ? conj(c, bt) : bt, lbA));
-    if (ib >= 0) tp.acc(ib, tcon(c, at.dt == DType::C128 ? conj(c, at) : at, laB, g, lcB));
+    const AV &a0 = terms[0].first, &b0 = terms[0].second;
+    Contraction pa(g, bl.lcA, b0.t, bl.lbA), pb(a0.t, bl.laB, g, bl.lcB);
+    // one product of the sum may be real where the sum is complex: its cotangent is the real part
+    Tensor gr;
+    auto cot = [&](const Tensor& x, const Tensor& y) {
+      if (g.dt == DType::F64 || x.dt == DType::C128 || y.dt == DType::C128) return g;
+      if (gr.empty()) gr = real_of(c, g);
+      return gr;
+    };
+    auto cj = [&](const Tensor& x) { return x.dt == DType::C128 ? conj(c, x) : x; };
+    for (const auto& t : terms) {
+      const AV &a = t.first, &b = t.second;
+      const Tensor gt = cot(a.t, b.t);
+      Tensor raw;
+      if (a.id >= 0) {
+        pa.add(c, raw, gt, cj(b.t));
+        tp.acc(a.id, pa.finish(c, raw));
+      }
+      raw = Tensor();
+      if (b.id >= 0) {
+        pb.add(c, raw, cj(a.t), gt);
+        tp.acc(b.id, pb.finish(c, raw));
+      }
+    }
   });
   return out;
 }
@@ -751,22 +811,6 @@ struct IterCk {
 }  // namespace
 
 namespace {
-
-__global__ void real_part_kernel(const double2* x, double* y, int64_t n) {
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-    y[i] = x[i].x;
-}
-
-// the cotangent of a real variable from a possibly complex one: its real part
-Tensor real_of(Ctx& c, const Tensor& x) {
-  if (x.empty() || x.dt == DType::F64) return x;
-  Tensor y = c.alloc(DType::F64, x.shape());
-  const int64_t n = x.numel();
-  const unsigned g = unsigned(std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, int64_t(c.sm_count) * 8)));
-  real_part_kernel<<<g, 256, 0, c.stream>>>(static_cast<const double2*>(x.data()), y.f64(), n);
-  IPEPS_LAUNCH_CHECK();
-  return y;
-}
 
 std::complex<double> scalar_host(Ctx& c, const Tensor& t) {
   double h[2] = {0, 0};

@@ -41,6 +41,9 @@ class Tape {
 };
 
 AV ad_tcon(Tape& tp, const AV& a, const std::vector<int>& la, const AV& b, const std::vector<int>& lb);
+// the sum of the products of `terms`, all of the contraction p (labels la, lb)
+AV ad_tcon_sum(Tape& tp, Contraction& p, const std::vector<std::pair<AV, AV>>& terms, const std::vector<int>& la,
+               const std::vector<int>& lb);
 AV ad_reshape(Tape& tp, const AV& a, const std::vector<int64_t>& s);
 AV ad_permute(Tape& tp, const AV& a, const std::vector<int>& perm);
 AV ad_renorm(Tape& tp, const AV& a);

@@ -15,42 +15,20 @@
 namespace ipeps {
 
 // ------------------------------------------------------------ nested algebra
-namespace {
-
-void add_into(Ctx& c, Tensor& acc, const Tensor& t) {
-  if (t.empty()) return;
-  if (acc.empty()) {
-    acc = t;
-    return;
-  }
-  if (acc.dt == DType::F64 && t.dt == DType::C128) acc = to_complex(c, acc);
-  axpy(c, cplx(1), t, acc);  // real into complex handled by axpy_rc
-}
-
-}  // namespace
-
 // nested_tensor.jl:77-92 (product rule), emptyT.jl:24-26 (EmptyT absorbs)
 NT ntcon(Ctx& c, const NT& A, const std::vector<int>& la, const NT& B, const std::vector<int>& lb) {
   if (!A.nested && !B.nested) return NT(tcon(c, A.c[0], la, B.c[0], lb));
   NT r;
   r.nested = true;
-  if (A.nested && B.nested) {
-    static const int pairs[4][4][2] = {{{0, 0}, {-1, -1}, {-1, -1}, {-1, -1}},
-                                       {{0, 1}, {1, 0}, {-1, -1}, {-1, -1}},
-                                       {{0, 2}, {2, 0}, {-1, -1}, {-1, -1}},
-                                       {{0, 3}, {3, 0}, {1, 2}, {2, 1}}};
-    for (int o = 0; o < 4; ++o)
-      for (int p = 0; p < 4; ++p) {
-        int i = pairs[o][p][0], j = pairs[o][p][1];
-        if (i < 0 || !A.has(i) || !B.has(j)) continue;
-        add_into(c, r.c[o], tcon(c, A.c[i], la, B.c[j], lb));
-      }
-  } else if (A.nested) {
-    for (int i = 0; i < 4; ++i)
-      if (A.has(i)) r.c[i] = tcon(c, A.c[i], la, B.c[0], lb);
-  } else {
-    for (int i = 0; i < 4; ++i)
-      if (B.has(i)) r.c[i] = tcon(c, A.c[0], la, B.c[i], lb);
+  Contraction p(A.c[0], la, B.c[0], lb);
+  for (int o = 0; o < 4; ++o) {
+    Tensor raw;
+    for (const auto& ij : kNestedPairs[o]) {
+      const int i = ij[0], j = ij[1];
+      if (i < 0 || !(A.nested || i == 0) || !(B.nested || j == 0) || !A.has(i) || !B.has(j)) continue;
+      p.add(c, raw, A.c[i], B.c[j]);
+    }
+    if (!raw.empty()) r.c[o] = p.finish(c, raw);
   }
   return r;
 }

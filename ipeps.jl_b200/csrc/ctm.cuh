@@ -18,6 +18,11 @@ struct NT {
   bool has(int i) const { return !c[i].empty(); }
 };
 
+// component pairs of a product of nested tensors (nested_tensor.jl:77-92); -1: none
+constexpr int kNestedPairs[4][4][2] = {{{0, 0}, {-1, -1}, {-1, -1}, {-1, -1}},
+                                       {{0, 1}, {1, 0}, {-1, -1}, {-1, -1}},
+                                       {{0, 2}, {2, 0}, {-1, -1}, {-1, -1}},
+                                       {{0, 3}, {3, 0}, {1, 2}, {2, 1}}};
 NT ntcon(Ctx& c, const NT& A, const std::vector<int>& la, const NT& B, const std::vector<int>& lb);
 NT nreshape(const NT& A, const std::vector<int64_t>& s);
 NT npermute(Ctx& c, const NT& A, const std::vector<int>& perm);

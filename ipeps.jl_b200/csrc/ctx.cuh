@@ -207,9 +207,33 @@ Tensor matmul(Ctx& c, const Tensor& A, char opA, const Tensor& B, char opB);
 // are summed, negative labels -1,-2,... give the output order).
 Tensor tcon(Ctx& c, const Tensor& A, const std::vector<int>& la, const Tensor& B,
             const std::vector<int>& lb);
-// out += tcon(...) (out must have the output shape)
-void tcon_acc(Ctx& c, Tensor& out, const Tensor& A, const std::vector<int>& la, const Tensor& B,
-              const std::vector<int>& lb);
+// The plan of one tcon for operands of given shapes and labels, for sums of products
+// of the same contraction (the components of nested tensors): each operand is
+// permuted once however many products it enters, the products are added by the GEMM
+// in the layout it writes, and the sum is permuted once at the end.
+class Contraction {
+ public:
+  Contraction(const Tensor& A, const std::vector<int>& la, const Tensor& B, const std::vector<int>& lb);
+  // raw += A B (raw is allocated by the first product)
+  void add(Ctx& c, Tensor& raw, const Tensor& A, const Tensor& B);
+  // the sum in output order
+  Tensor finish(Ctx& c, const Tensor& raw) const;
+
+  struct Side {
+    std::vector<int> perm;  // empty: used as it stands
+    char op = 'N';
+    int64_t ld = 1;
+    std::vector<std::pair<Tensor, Tensor>> done;  // operands permuted so far (kept alive by the plan)
+  };
+
+ private:
+  static Tensor prepared(Ctx& c, Side& s, const Tensor& X);
+  Side a_, b_;
+  bool swapped_ = false;
+  int64_t m_ = 1, n_ = 1, k_ = 1;
+  std::vector<int64_t> odims_, raw_dims_;
+  std::vector<int> final_;  // permutation of the product to output order; empty: none
+};
 
 // ------------------------------------------------------------ reductions
 // d_out[0] = max |x| (device scalar)

@@ -42,28 +42,6 @@ Tensor as_dtype(Ctx& c, const Tensor& g, DType dt) {
   return dt == DType::F64 ? real_part(c, g) : to_complex(c, g);
 }
 
-AV ad_add(Tape& tp, const AV& a, const AV& b) {
-  Ctx& c = tp.ctx();
-  if (a.t.empty()) return b;
-  if (b.t.empty()) return a;
-  DType dt = (a.t.dt == DType::C128 || b.t.dt == DType::C128) ? DType::C128 : DType::F64;
-  AV out{clone(c, a.t.dt == dt ? a.t : to_complex(c, a.t)), -1};
-  axpy(c, cplx(1), b.t, out.t);
-  if (a.id < 0 && b.id < 0) return out;
-  out.id = tp.newid();
-  const int ia = a.id, ib = b.id, io = out.id;
-  const DType da = a.t.dt, db = b.t.dt;
-  const std::vector<int64_t> sa = a.t.shape(), sb = b.t.shape();
-  tp.push([&tp, ia, ib, io, da, db, sa, sb]() {
-    const Tensor& g = tp.grad(io);
-    if (g.empty()) return;
-    Ctx& c = tp.ctx();
-    if (ia >= 0) tp.acc(ia, as_dtype(c, g, da).reshape(sa));
-    if (ib >= 0) tp.acc(ib, as_dtype(c, g, db).reshape(sb));
-  });
-  return out;
-}
-
 // y = s x (s complex constant); dx = conj(s) dy
 AV ad_scale_c(Tape& tp, const AV& a, double re, double im) {
   Ctx& c = tp.ctx();
@@ -130,23 +108,15 @@ struct NADPolicy {
       return r;
     }
     r.nested = true;
-    if (a.nested && b.nested) {  // nested_tensor.jl:77-88
-      static const int pairs[4][4][2] = {{{0, 0}, {-1, -1}, {-1, -1}, {-1, -1}},
-                                         {{0, 1}, {1, 0}, {-1, -1}, {-1, -1}},
-                                         {{0, 2}, {2, 0}, {-1, -1}, {-1, -1}},
-                                         {{0, 3}, {3, 0}, {1, 2}, {2, 1}}};
-      for (int o = 0; o < 4; ++o)
-        for (int p = 0; p < 4; ++p) {
-          const int i = pairs[o][p][0], j = pairs[o][p][1];
-          if (i < 0 || !a.has(i) || !b.has(j)) continue;
-          r.c[o] = ad_add(tp, r.c[o], ad_tcon(tp, a.c[i], la, b.c[j], lb));
-        }
-    } else if (a.nested) {
-      for (int i = 0; i < 4; ++i)
-        if (a.has(i)) r.c[i] = ad_tcon(tp, a.c[i], la, b.c[0], lb);
-    } else {
-      for (int i = 0; i < 4; ++i)
-        if (b.has(i)) r.c[i] = ad_tcon(tp, a.c[0], la, b.c[i], lb);
+    Contraction p(a.c[0].t, la, b.c[0].t, lb);
+    for (int o = 0; o < 4; ++o) {  // nested_tensor.jl:77-92
+      std::vector<std::pair<AV, AV>> terms;
+      for (const auto& ij : kNestedPairs[o]) {
+        const int i = ij[0], j = ij[1];
+        if (i < 0 || !(a.nested || i == 0) || !(b.nested || j == 0) || !a.has(i) || !b.has(j)) continue;
+        terms.emplace_back(a.c[i], b.c[j]);
+      }
+      if (!terms.empty()) r.c[o] = ad_tcon_sum(tp, p, terms, la, lb);
     }
     return r;
   }

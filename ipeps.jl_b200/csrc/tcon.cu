@@ -19,11 +19,6 @@
 namespace ipeps {
 namespace {
 
-struct Plan {
-  bool swap = false;  // compute with roles (A,B) swapped
-  std::vector<int> fa, fb, kk;  // label lists
-};
-
 // position of each label in a label list
 int find(const std::vector<int>& l, int x) {
   for (size_t i = 0; i < l.size(); ++i)
@@ -49,28 +44,6 @@ std::vector<int> strip_units(const std::vector<int>& labels, const std::map<int,
   return r;
 }
 
-struct Operand {
-  Tensor t;     // possibly permuted copy
-  char op;      // 'N' or 'T'
-  int64_t ld;
-};
-
-// Bring X (labels lx) into a GEMM operand whose logical matrix is
-// [rows, cols] where rows/cols are label lists.
-Operand prepare(Ctx& c, const Tensor& X, const std::vector<int>& lx, const std::vector<int>& rows,
-                const std::vector<int>& cols, const std::map<int, int64_t>& ext) {
-  int64_t nr = 1, nc = 1;
-  for (int l : rows) nr *= ext.at(l);
-  for (int l : cols) nc *= ext.at(l);
-  auto sx = strip_units(lx, ext), sr = strip_units(rows, ext), scl = strip_units(cols, ext);
-  if (ordered_as(sx, sr, scl)) return {X, 'N', std::max<int64_t>(nr, 1)};
-  if (ordered_as(sx, scl, sr)) return {X, 'T', std::max<int64_t>(nc, 1)};
-  std::vector<int> perm;
-  for (int l : rows) perm.push_back(find(lx, l));
-  for (int l : cols) perm.push_back(find(lx, l));
-  return {permute(c, X, perm), 'N', std::max<int64_t>(nr, 1)};
-}
-
 int64_t permute_cost(const std::vector<int>& lx, const std::vector<int>& r, const std::vector<int>& col,
                      const std::map<int, int64_t>& ext, int64_t numel) {
   auto sx = strip_units(lx, ext), sr = strip_units(r, ext), sc = strip_units(col, ext);
@@ -78,8 +51,39 @@ int64_t permute_cost(const std::vector<int>& lx, const std::vector<int>& r, cons
   return numel;
 }
 
-void contract(Ctx& c, const Tensor& A, const std::vector<int>& la, const Tensor& B,
-              const std::vector<int>& lb, Tensor* out, bool accumulate) {
+// How an operand with labels lx becomes a GEMM operand whose logical matrix is [rows, cols].
+Contraction::Side plan_side(const std::vector<int>& lx, const std::vector<int>& rows, const std::vector<int>& cols,
+                            const std::map<int, int64_t>& ext) {
+  int64_t nr = 1, nc = 1;
+  for (int l : rows) nr *= ext.at(l);
+  for (int l : cols) nc *= ext.at(l);
+  auto sx = strip_units(lx, ext), sr = strip_units(rows, ext), scl = strip_units(cols, ext);
+  Contraction::Side s;
+  if (ordered_as(sx, sr, scl)) {
+    s.ld = std::max<int64_t>(nr, 1);
+  } else if (ordered_as(sx, scl, sr)) {
+    s.op = 'T';
+    s.ld = std::max<int64_t>(nc, 1);
+  } else {
+    for (int l : rows) s.perm.push_back(find(lx, l));
+    for (int l : cols) s.perm.push_back(find(lx, l));
+    s.ld = std::max<int64_t>(nr, 1);
+  }
+  return s;
+}
+
+// op(A) op(B) of real and complex operands; the result is complex when either is
+void gemm_any(Ctx& c, char opA, const Tensor& A, int64_t lda, char opB, const Tensor& B, int64_t ldb, int64_t m,
+              int64_t n, int64_t k, double beta, void* C, int64_t ldc) {
+  if (A.dt == B.dt)
+    gemm(c, A.dt, opA, opB, m, n, k, cplx(1), A.data(), lda, B.data(), ldb, cplx(beta), C, ldc);
+  else
+    gemm_c128_dmma(c, opA, A.dt, opB, B.dt, m, n, k, cplx(1), A.data(), lda, B.data(), ldb, cplx(beta), C, ldc);
+}
+
+}  // namespace
+
+Contraction::Contraction(const Tensor& A, const std::vector<int>& la, const Tensor& B, const std::vector<int>& lb) {
   IPEPS_CHECK(int(la.size()) == A.nd, "tcon: label count != rank of A " + shape_str(A));
   IPEPS_CHECK(int(lb.size()) == B.nd, "tcon: label count != rank of B " + shape_str(B));
   std::map<int, int64_t> ext;
@@ -103,89 +107,84 @@ void contract(Ctx& c, const Tensor& A, const std::vector<int>& la, const Tensor&
   by_out(fa);
   by_out(fb);
   const int nout = int(fa.size() + fb.size());
-  std::vector<int64_t> odims(nout);
+  odims_.resize(nout);
   for (int i = 0; i < nout; ++i) {
     auto it = ext.find(-(i + 1));
     IPEPS_CHECK(it != ext.end(), "tcon: output labels must be -1..-n");
-    odims[i] = it->second;
+    odims_[i] = it->second;
   }
   // output arrangement
   auto pos = [](int l) { return -l - 1; };
   int maxa = -1, mina = 1 << 30, maxb = -1, minb = 1 << 30;
   for (int l : fa) { maxa = std::max(maxa, pos(l)); mina = std::min(mina, pos(l)); }
   for (int l : fb) { maxb = std::max(maxb, pos(l)); minb = std::min(minb, pos(l)); }
-  bool direct = fb.empty() || fa.empty() || maxa < minb;
-  bool swapped = !direct && maxb < mina;
+  const bool direct = fb.empty() || fa.empty() || maxa < minb;
+  swapped_ = !direct && maxb < mina;
   // summed-label order: from A or from B
   int64_t costA = permute_cost(la, fa, kA, ext, A.numel()) + permute_cost(lb, kA, fb, ext, B.numel());
   int64_t costB = permute_cost(la, fa, kB, ext, A.numel()) + permute_cost(lb, kB, fb, ext, B.numel());
   const std::vector<int>& kk = (costB < costA) ? kB : kA;
-
-  int64_t m = 1, n = 1, k = 1;
-  for (int l : fa) m *= ext[l];
-  for (int l : fb) n *= ext[l];
-  for (int l : kk) k *= ext[l];
-
-  DType dt = (A.dt == DType::C128 || B.dt == DType::C128) ? DType::C128 : DType::F64;
-  Tensor Ac = A, Bc = B;
-  if (A.dt != dt) Ac = to_complex(c, A);
-  if (B.dt != dt) Bc = to_complex(c, B);
-
-  Tensor res;
-  bool need_final_perm = !(direct || swapped);
-  if (accumulate) {
-    IPEPS_CHECK(out && !out->empty() && out->numel() == m * n && out->dt == dt, "tcon_acc: bad output");
+  for (int l : fa) m_ *= ext[l];
+  for (int l : fb) n_ *= ext[l];
+  for (int l : kk) k_ *= ext[l];
+  if (!swapped_) {
+    a_ = plan_side(la, fa, kk, ext);
+    b_ = plan_side(lb, kk, fb, ext);
+  } else {  // C^T = B^T A^T : rows = fb, cols = fa
+    a_ = plan_side(la, kk, fa, ext);
+    b_ = plan_side(lb, fb, kk, ext);
   }
-  if (!need_final_perm && accumulate) res = *out;
-  else if (!need_final_perm && out && !out->empty() && out->dt == dt && out->numel() == m * n) res = *out;
-  else res = c.alloc(dt, direct || swapped ? odims : std::vector<int64_t>{m, n});
-
-  if (k == 0 || m * n == 0) {
-    if (!accumulate) IPEPS_CUDA(cudaMemsetAsync(res.data(), 0, res.bytes(), c.stream));
-  } else if (!swapped) {
-    Operand oa = prepare(c, Ac, la, fa, kk, ext);
-    Operand ob = prepare(c, Bc, lb, kk, fb, ext);
-    gemm(c, dt, oa.op, ob.op, m, n, k, cplx(1), oa.t.data(), oa.ld, ob.t.data(), ob.ld,
-         cplx(accumulate && !need_final_perm ? 1.0 : 0.0), res.data(), m);
-  } else {
-    // C^T = B^T A^T : rows = fb, cols = fa
-    Operand ob = prepare(c, Bc, lb, fb, kk, ext);
-    Operand oa = prepare(c, Ac, la, kk, fa, ext);
-    gemm(c, dt, ob.op, oa.op, n, m, k, cplx(1), ob.t.data(), ob.ld, oa.t.data(), oa.ld,
-         cplx(accumulate ? 1.0 : 0.0), res.data(), n);
-  }
-  if (need_final_perm) {
-    // res is [fa..., fb...] -> output order
+  if (!(direct || swapped_)) {
+    // the product is [fa..., fb...] -> output order
     std::vector<int> cur(fa);
     cur.insert(cur.end(), fb.begin(), fb.end());
-    std::vector<int64_t> cd;
-    for (int l : cur) cd.push_back(ext[l]);
-    Tensor r2 = res.reshape(cd);
-    std::vector<int> perm(nout);
-    for (int i = 0; i < nout; ++i) perm[i] = find(cur, -(i + 1));
-    Tensor p = permute(c, r2, perm);
-    if (accumulate) axpy(c, cplx(1), p, *out);
-    else *out = p;
-    return;
-  }
-  if (!accumulate) {
-    res = res.reshape(odims);
-    *out = res;
+    for (int l : cur) raw_dims_.push_back(ext[l]);
+    final_.resize(nout);
+    for (int i = 0; i < nout; ++i) final_[i] = find(cur, -(i + 1));
   }
 }
 
-}  // namespace
+Tensor Contraction::prepared(Ctx& c, Side& s, const Tensor& X) {
+  if (s.perm.empty()) return X;
+  for (const auto& q : s.done)
+    if (q.first.buf == X.buf && q.first.offset == X.offset && q.first.dt == X.dt) return q.second;
+  Tensor p = permute(c, X, s.perm);
+  s.done.emplace_back(X, p);
+  return p;
+}
+
+void Contraction::add(Ctx& c, Tensor& raw, const Tensor& A, const Tensor& B) {
+  const DType dt = (A.dt == DType::C128 || B.dt == DType::C128) ? DType::C128 : DType::F64;
+  if (!raw.empty() && raw.dt == DType::F64 && dt == DType::C128) raw = to_complex(c, raw);
+  if (!raw.empty() && raw.dt == DType::C128 && dt == DType::F64) {
+    Tensor t;
+    add(c, t, A, B);
+    axpy(c, cplx(1), t, raw);
+    return;
+  }
+  const double beta = raw.empty() ? 0.0 : 1.0;
+  if (raw.empty()) raw = c.alloc(dt, final_.empty() ? odims_ : raw_dims_);
+  if (k_ == 0 || m_ * n_ == 0) {
+    if (beta == 0.0) IPEPS_CUDA(cudaMemsetAsync(raw.data(), 0, raw.bytes(), c.stream));
+    return;
+  }
+  const Tensor a = prepared(c, a_, A), b = prepared(c, b_, B);
+  if (!swapped_)
+    gemm_any(c, a_.op, a, a_.ld, b_.op, b, b_.ld, m_, n_, k_, beta, raw.data(), m_);
+  else
+    gemm_any(c, b_.op, b, b_.ld, a_.op, a, a_.ld, n_, m_, k_, beta, raw.data(), n_);
+}
+
+Tensor Contraction::finish(Ctx& c, const Tensor& raw) const {
+  return final_.empty() ? raw : permute(c, raw, final_);
+}
 
 Tensor tcon(Ctx& c, const Tensor& A, const std::vector<int>& la, const Tensor& B,
             const std::vector<int>& lb) {
-  Tensor out;
-  contract(c, A, la, B, lb, &out, false);
-  return out;
-}
-
-void tcon_acc(Ctx& c, Tensor& out, const Tensor& A, const std::vector<int>& la, const Tensor& B,
-              const std::vector<int>& lb) {
-  contract(c, A, la, B, lb, &out, true);
+  Contraction p(A, la, B, lb);
+  Tensor raw;
+  p.add(c, raw, A, B);
+  return p.finish(c, raw);
 }
 
 Tensor matmul(Ctx& c, const Tensor& A, char opA, const Tensor& B, char opB) {
@@ -196,11 +195,9 @@ Tensor matmul(Ctx& c, const Tensor& A, char opA, const Tensor& B, char opB) {
   int64_t n = (opB == 'N') ? B.dims[1] : B.dims[0];
   IPEPS_CHECK(ka == kb, "matmul: inner dimension mismatch " + shape_str(A) + " " + shape_str(B));
   DType dt = (A.dt == DType::C128 || B.dt == DType::C128) ? DType::C128 : DType::F64;
-  Tensor Ac = A.dt == dt ? A : to_complex(c, A);
-  Tensor Bc = B.dt == dt ? B : to_complex(c, B);
   Tensor C = c.alloc(dt, {m, n});
-  gemm(c, dt, opA, opB, m, n, ka, cplx(1), Ac.data(), std::max<int64_t>(Ac.dims[0], 1), Bc.data(),
-       std::max<int64_t>(Bc.dims[0], 1), cplx(0), C.data(), std::max<int64_t>(m, 1));
+  gemm_any(c, opA, A, std::max<int64_t>(A.dims[0], 1), opB, B, std::max<int64_t>(B.dims[0], 1), m, n, ka, 0.0,
+           C.data(), std::max<int64_t>(m, 1));
   return C;
 }
 
