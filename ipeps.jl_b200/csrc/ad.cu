@@ -27,6 +27,7 @@ __device__ __forceinline__ double wsum(double v) {
 
 // out[0] = sum x*y (deterministic: fixed grid, then one block)
 __global__ void dot_partial_kernel(const double* x, const double* y, int64_t n, double* part) {
+  pdl_wait();
   double s = 0;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     s = fma(x[i], y[i], s);
@@ -42,6 +43,7 @@ __global__ void dot_partial_kernel(const double* x, const double* y, int64_t n, 
 }
 
 __global__ void sum_kernel(const double* part, int n, double* out) {
+  pdl_wait();
   double s = 0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += part[i];
   s = wsum(s);
@@ -57,6 +59,7 @@ __global__ void sum_kernel(const double* part, int n, double* out) {
 
 // smallest index with |x_i| == m
 __global__ void argmax_kernel(const double* x, int64_t n, const double* m, unsigned long long* idx) {
+  pdl_wait();
   const double mv = *m;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     if (fabs(x[i]) == mv) atomicMin(idx, static_cast<unsigned long long>(i));
@@ -65,6 +68,7 @@ __global__ void argmax_kernel(const double* x, int64_t n, const double* m, unsig
 // dx = dy/m - (dot/m^2) sign(x_k) e_k
 __global__ void renorm_back_kernel(const double* dy, const double* x, int64_t n, const double* m,
                                    const unsigned long long* idx, const double* dot, double* dx) {
+  pdl_wait();
   const double mv = *m, inv = 1.0 / mv;
   const int64_t k = int64_t(*idx);
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
@@ -77,6 +81,7 @@ __global__ void renorm_back_kernel(const double* dy, const double* x, int64_t n,
 // X[:, j] *= f(s[j]); mode 0: s, 1: 1/sqrt(s), 2: sqrt(s), 3: 1/s.  The inverse
 // of a kept s of exactly 0 is taken as 0 (its projector column is zero).
 __global__ void colscale_kernel(double* X, int64_t ld, int64_t m, int ncols, const double* s, int mode) {
+  pdl_wait();
   const int64_t tot = m * ncols;
   for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < tot; t += int64_t(gridDim.x) * blockDim.x) {
     const int64_t i = t % m;
@@ -89,6 +94,7 @@ __global__ void colscale_kernel(double* X, int64_t ld, int64_t m, int ncols, con
 
 // out (N x n) = transpose of in (n x N) with columns scaled by 1/sqrt(s)
 __global__ void transpose_scale_kernel(const double* in, int n, int64_t N, const double* s, double* out) {
+  pdl_wait();
   const int64_t tot = int64_t(n) * N;
   for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < tot; t += int64_t(gridDim.x) * blockDim.x) {
     const int64_t a = t % N;
@@ -100,6 +106,7 @@ __global__ void transpose_scale_kernel(const double* in, int n, int64_t N, const
 // dS_i = -1/(2 s_i) (sum_a dP1[a,i] P1[a,i] + sum_j dP2[i,j] P2[i,j]); one warp per i
 __global__ void dS_kernel(int n, int64_t N, const double* dP1, const double* P1, const double* dP2, const double* P2,
                           const double* s, double* dS) {
+  pdl_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= n) return;
   const int i = warp;
@@ -118,6 +125,7 @@ __device__ __forceinline__ double Fb(double x, double eta) { return x / (x * x +
 // J = F o C1, K = F o C2, F_ij = f(s_j^2 - s_i^2)
 __global__ void att_kernel(int n, const double* C1, const double* C2, const double* s, const double* dS, double eta,
                            double* A) {
+  pdl_wait();
   const int64_t tot = int64_t(n) * n;
   for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < tot; t += int64_t(gridDim.x) * blockDim.x) {
     const int i = int(t % n), j = int(t / n);
@@ -132,6 +140,7 @@ __global__ void att_kernel(int n, const double* C1, const double* C2, const doub
 // G[a,i] = f(s_t[i]^2 - s_in[a]^2) C[a,i]  (a in-sketch discarded, i kept)
 __global__ void fin_kernel(int nin, int n, const double* C, const double* s_in, const double* s_t, double eta,
                            double* G) {
+  pdl_wait();
   const int64_t tot = int64_t(nin) * n;
   for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < tot; t += int64_t(gridDim.x) * blockDim.x) {
     const int a = int(t % nin), i = int(t / nin);
@@ -171,6 +180,7 @@ __device__ __forceinline__ double cheb_coef(double si, double eta, double b, int
 // X[:, i] += a_m(i) T[:, i]
 __global__ void cheb_acc_kernel(double* X, const double* T, int64_t N, int n, const double* s, double eta, double b,
                                 int m) {
+  pdl_wait();
   const int64_t tot = N * n;
   for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < tot; t += int64_t(gridDim.x) * blockDim.x) {
     const int i = int(t / N);
@@ -179,6 +189,7 @@ __global__ void cheb_acc_kernel(double* X, const double* T, int64_t N, int n, co
 }
 
 __global__ void cheb_coef_max_kernel(const double* s, int n, double eta, double b, int m, double* out) {
+  pdl_wait();
   double mx = 0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) mx = fmax(mx, fabs(cheb_coef(s[i], eta, b, m)));
   for (int o = 16; o; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -190,6 +201,7 @@ __global__ void cheb_coef_max_kernel(const double* s, int n, double eta, double 
 __global__ void resolvent_check_kernel(const double* X, const double* BX, const double* BBX, const double* Y,
                                        const double* BY, const double* s, double eta, int64_t N, int n, double* res,
                                        double* rhs) {
+  pdl_wait();
   const int64_t tot = N * n;
   for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < tot; t += int64_t(gridDim.x) * blockDim.x) {
     const double s2 = s[t / N] * s[t / N];
@@ -201,6 +213,7 @@ __global__ void resolvent_check_kernel(const double* X, const double* BX, const 
 
 // out[i] = sum_j X[i + j N]
 __global__ void rowsum_kernel(const double* X, int64_t N, int n, double* out) {
+  pdl_wait();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < N; i += int64_t(gridDim.x) * blockDim.x) {
     double a = 0;
     for (int j = 0; j < n; ++j) a += X[i + j * N];
@@ -210,6 +223,7 @@ __global__ void rowsum_kernel(const double* X, int64_t N, int n, double* out) {
 
 // y = alpha * x + beta * y (elementwise over n doubles)
 __global__ void axpby_kernel(double alpha, const double* x, double beta, double* y, int64_t n) {
+  pdl_wait();
   for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += int64_t(gridDim.x) * blockDim.x)
     y[t] = fma(alpha, x[t], beta * y[t]);
 }
@@ -224,8 +238,8 @@ double dot_host(Ctx& c, const Tensor& x, const Tensor& y) {
   const int blocks = int(std::min<int64_t>((n + 255) / 256, 1024));
   double* part = static_cast<double*>(c.workspace(size_t(std::max(blocks, 1)) * 8 + 64));
   double* out = reinterpret_cast<double*>(c.scal->p) + 32;
-  dot_partial_kernel<<<std::max(blocks, 1), 256, 0, c.stream>>>(x.f64(), y.f64(), n, part);
-  sum_kernel<<<1, 256, 0, c.stream>>>(part, std::max(blocks, 1), out);
+  launch(c.stream, dot_partial_kernel, std::max(blocks, 1), 256, 0, x.f64(), y.f64(), n, part);
+  launch(c.stream, sum_kernel, 1, 256, 0, part, std::max(blocks, 1), out);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Reduce, 2.0 * n, 16.0 * n);
   double h = 0;
@@ -239,14 +253,14 @@ void dot_dev(Ctx& c, const Tensor& x, const Tensor& y, double* out) {
   const int64_t n = x.numel();
   const int blocks = int(std::min<int64_t>((n + 255) / 256, 1024));
   double* part = static_cast<double*>(c.workspace(size_t(std::max(blocks, 1)) * 8 + 64));
-  dot_partial_kernel<<<std::max(blocks, 1), 256, 0, c.stream>>>(x.f64(), y.f64(), n, part);
-  sum_kernel<<<1, 256, 0, c.stream>>>(part, std::max(blocks, 1), out);
+  launch(c.stream, dot_partial_kernel, std::max(blocks, 1), 256, 0, x.f64(), y.f64(), n, part);
+  launch(c.stream, sum_kernel, 1, 256, 0, part, std::max(blocks, 1), out);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Reduce, 2.0 * n, 16.0 * n);
 }
 
 void colscale(Ctx& c, Tensor& X, const double* s, int ncols, int mode) {
-  colscale_kernel<<<gridn(c, X.dims[0] * ncols), 256, 0, c.stream>>>(X.f64(), X.dims[0], X.dims[0], ncols, s, mode);
+  launch(c.stream, colscale_kernel, gridn(c, X.dims[0] * ncols), 256, 0, X.f64(), X.dims[0], X.dims[0], ncols, s, mode);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Elementwise, 0, 16.0 * X.dims[0] * ncols);
 }
@@ -335,6 +349,7 @@ void Tape::backward() {
 namespace {
 
 __global__ void real_part_kernel(const double2* x, double* y, int64_t n) {
+  pdl_wait();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     y[i] = x[i].x;
 }
@@ -345,7 +360,7 @@ Tensor real_of(Ctx& c, const Tensor& x) {
   Tensor y = c.alloc(DType::F64, x.shape());
   const int64_t n = x.numel();
   const unsigned g = unsigned(std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, int64_t(c.sm_count) * 8)));
-  real_part_kernel<<<g, 256, 0, c.stream>>>(static_cast<const double2*>(x.data()), y.f64(), n);
+  launch(c.stream, real_part_kernel, g, 256, 0, static_cast<const double2*>(x.data()), y.f64(), n);
   IPEPS_LAUNCH_CHECK();
   return y;
 }
@@ -458,7 +473,7 @@ AV ad_renorm(Tape& tp, const AV& a) {
   unsigned long long* d_k = reinterpret_cast<unsigned long long*>(d_m + 1);
   IPEPS_CUDA(cudaMemsetAsync(d_k, 0xff, 8, c.stream));
   const int64_t n = a.t.numel();
-  argmax_kernel<<<gridn(c, n), 256, 0, c.stream>>>(a.t.f64(), n, d_m, d_k);
+  launch(c.stream, argmax_kernel, gridn(c, n), 256, 0, a.t.f64(), n, d_m, d_k);
   IPEPS_LAUNCH_CHECK();
   AV out{clone(c, a.t), -1};
   scale_inv(c, out.t, d_m);
@@ -474,12 +489,11 @@ AV ad_renorm(Tape& tp, const AV& a) {
     const int blocks = int(std::min<int64_t>((n + 255) / 256, 1024));
     double* part = static_cast<double*>(c.workspace(size_t(std::max(blocks, 1)) * 8 + 64));
     Tensor dot = c.alloc(DType::F64, {1});
-    dot_partial_kernel<<<std::max(blocks, 1), 256, 0, c.stream>>>(g.f64(), xt.f64(), n, part);
-    sum_kernel<<<1, 256, 0, c.stream>>>(part, std::max(blocks, 1), dot.f64());
+    launch(c.stream, dot_partial_kernel, std::max(blocks, 1), 256, 0, g.f64(), xt.f64(), n, part);
+    launch(c.stream, sum_kernel, 1, 256, 0, part, std::max(blocks, 1), dot.f64());
     Tensor dx = c.alloc(DType::F64, xt.shape());
-    renorm_back_kernel<<<gridn(c, n), 256, 0, c.stream>>>(
-        g.f64(), xt.f64(), n, mk.f64(), reinterpret_cast<const unsigned long long*>(mk.f64() + 1), dot.f64(),
-        dx.f64());
+    launch(c.stream, renorm_back_kernel, gridn(c, n), 256, 0, g.f64(), xt.f64(), n, mk.f64(),
+           reinterpret_cast<const unsigned long long*>(mk.f64() + 1), dot.f64(), dx.f64());
     IPEPS_LAUNCH_CHECK();
     c.count(KFam::Elementwise, 0, 24.0 * n);
     tp.acc(ia, dx);
@@ -521,14 +535,14 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
   colscale(c, dVt, s.f64(), n, 1);
   // dS
   Tensor dS = c.alloc(DType::F64, {n});
-  dS_kernel<<<(n * 32 + 255) / 256, 256, 0, c.stream>>>(n, K1, dP1.f64(), P1.f64(), dP2.f64(), P2.f64(), s.f64(),
-                                                         dS.f64());
+  launch(c.stream, dS_kernel, (n * 32 + 255) / 256, 256, 0, n, K1, dP1.f64(), P1.f64(), dP2.f64(), P2.f64(), s.f64(),
+         dS.f64());
   IPEPS_LAUNCH_CHECK();
   // kept x kept block
   Tensor C1 = mm(c, Ut, 'T', dUt, 'N', true), C2 = mm(c, Vt, 'T', dVt, 'N', true);
   Tensor Att = c.alloc(DType::F64, {n, n});
-  att_kernel<<<gridn(c, int64_t(n) * n), 256, 0, c.stream>>>(n, C1.f64(), C2.f64(), s.f64(), dS.f64(), kSvdEta,
-                                                             Att.f64());
+  launch(c.stream, att_kernel, gridn(c, int64_t(n) * n), 256, 0, n, C1.f64(), C2.f64(), s.f64(), dS.f64(), kSvdEta,
+         Att.f64());
   IPEPS_LAUNCH_CHECK();
   // W1 = V_t A_tt^T ; Acol, Bcol accumulate the discarded couplings
   Tensor W1 = mm(c, Vt, 'N', Att, 'T', true);
@@ -541,10 +555,10 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
     Tensor sin = vec_view(pr.Sr, n, nin);
     Tensor Cu = mm(c, Uin, 'T', dUt, 'N', true), Cv = mm(c, Vin, 'T', dVt, 'N', true);
     Tensor Gu = c.alloc(DType::F64, {nin, n}), Gv = c.alloc(DType::F64, {nin, n});
-    fin_kernel<<<gridn(c, int64_t(nin) * n), 256, 0, c.stream>>>(nin, n, Cu.f64(), sin.f64(), s.f64(), kSvdEta,
-                                                                 Gu.f64());
-    fin_kernel<<<gridn(c, int64_t(nin) * n), 256, 0, c.stream>>>(nin, n, Cv.f64(), sin.f64(), s.f64(), kSvdEta,
-                                                                 Gv.f64());
+    launch(c.stream, fin_kernel, gridn(c, int64_t(nin) * n), 256, 0, nin, n, Cu.f64(), sin.f64(), s.f64(), kSvdEta,
+           Gu.f64());
+    launch(c.stream, fin_kernel, gridn(c, int64_t(nin) * n), 256, 0, nin, n, Cv.f64(), sin.f64(), s.f64(), kSvdEta,
+           Gv.f64());
     IPEPS_LAUNCH_CHECK();
     // Acol += V_in diag(s_in) G_u ; Bcol += U_in diag(s_in) G_v
     Tensor sGu = clone(c, Gu), sGv = clone(c, Gv);
@@ -609,7 +623,7 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
       double est = 0;
       {
         Tensor t = c.alloc(DType::F64, {N1, 1});
-        rowsum_kernel<<<gridn(c, N1), 256, 0, c.stream>>>(Yu0.f64(), N1, n, t.f64());
+        launch(c.stream, rowsum_kernel, gridn(c, N1), 256, 0, Yu0.f64(), N1, n, t.f64());
         IPEPS_LAUNCH_CHECK();
         double nt = std::sqrt(dot_host(c, t, t));
         for (int it = 0; it < 6 && nt > 0; ++it) {
@@ -637,8 +651,9 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
       Tensor W1 = c.alloc(DType::F64, {N2, 2 * int64_t(n)}), W2 = c.alloc(DType::F64, {N1, 2 * int64_t(n)});
       Tensor BYu, BYv;
       auto next_T = [&](Tensor& B, const Tensor& T, const Tensor& Tprev, int m) {
-        axpby_kernel<<<gridn(c, B.numel()), 256, 0, c.stream>>>(-1.0, T.f64(), 2.0 / b, B.f64(), B.numel());
-        if (m > 0) axpby_kernel<<<gridn(c, B.numel()), 256, 0, c.stream>>>(-1.0, Tprev.f64(), 2.0, B.f64(), B.numel());
+        launch(c.stream, axpby_kernel, gridn(c, B.numel()), 256, 0, -1.0, T.f64(), 2.0 / b, B.f64(), B.numel());
+        if (m > 0) launch(c.stream, axpby_kernel, gridn(c, B.numel()), 256, 0, -1.0, Tprev.f64(), 2.0, B.f64(),
+                          B.numel());
         IPEPS_LAUNCH_CHECK();
       };
       auto apply_B = [&](const Tensor& Tu, const Tensor& Tv, const Tensor& Pu, const Tensor& Pv, int m, Tensor* Bu,
@@ -662,8 +677,8 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
         auto B = [&](const Tensor& T) { return u_side ? Bu_of(T) : Bv_of(T); };
         const Tensor BX = B(X), BBX = B(BX);
         Tensor res = c.alloc(DType::F64, X.shape()), rhs = c.alloc(DType::F64, X.shape());
-        resolvent_check_kernel<<<gridn(c, X.numel()), 256, 0, c.stream>>>(
-            X.f64(), BX.f64(), BBX.f64(), Y.f64(), BY.f64(), s.f64(), kSvdEta, X.dims[0], n, res.f64(), rhs.f64());
+        launch(c.stream, resolvent_check_kernel, gridn(c, X.numel()), 256, 0, X.f64(), BX.f64(), BBX.f64(), Y.f64(),
+               BY.f64(), s.f64(), kSvdEta, X.dims[0], n, res.f64(), rhs.f64());
         IPEPS_LAUNCH_CHECK();
         const double nr = dot_host(c, rhs, rhs);
         return nr > 0 ? std::sqrt(dot_host(c, res, res) / nr) : 0.0;
@@ -678,14 +693,16 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
         gemm(c, DType::F64, 'N', 'N', N1, n, N2, cplx(1), MP.data(), N1, Tv.data(), N2, cplx(0),
              cols(W2, n, n).data(), N1, true);
         for (int m = 0; m < kMaxTerms; ++m) {
-          cheb_acc_kernel<<<gridn(c, N1 * n), 256, 0, c.stream>>>(Xu.f64(), Tu.f64(), N1, n, s.f64(), kSvdEta, b, m);
-          cheb_acc_kernel<<<gridn(c, N2 * n), 256, 0, c.stream>>>(Xv.f64(), Tv.f64(), N2, n, s.f64(), kSvdEta, b, m);
+          launch(c.stream, cheb_acc_kernel, gridn(c, N1 * n), 256, 0, Xu.f64(), Tu.f64(), N1, n, s.f64(), kSvdEta, b,
+                 m);
+          launch(c.stream, cheb_acc_kernel, gridn(c, N2 * n), 256, 0, Xv.f64(), Tv.f64(), N2, n, s.f64(), kSvdEta, b,
+                 m);
           IPEPS_LAUNCH_CHECK();
           c.series_terms++;
           // the stopping tests read back five device scalars every kCheckEvery terms
           // (one host round trip instead of five per term)
           if (m % kCheckEvery == kCheckEvery - 1 || m == kMaxTerms - 1) {
-            cheb_coef_max_kernel<<<1, 32, 0, c.stream>>>(s.f64(), n, kSvdEta, b, m + 1, d_cmax);
+            launch(c.stream, cheb_coef_max_kernel, 1, 32, 0, s.f64(), n, kSvdEta, b, m + 1, d_cmax);
             IPEPS_LAUNCH_CHECK();
             dot_dev(c, Tu, Tu, d_cmax + 1);
             dot_dev(c, Tv, Tv, d_cmax + 2);
@@ -747,7 +764,7 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
   // dR1 = U_t [ (R2 W1)^T + S^-1/2 dP2 ] + Bcol (R2 V_t)^T,   R2 V_t = P1 S^1/2
   Tensor Z = Rapply(c, R2t, t2, 'N', W1);
   Tensor dP2T = c.alloc(DType::F64, {K1, n});
-  transpose_scale_kernel<<<gridn(c, K1 * n), 256, 0, c.stream>>>(dP2.f64(), n, K1, s.f64(), dP2T.f64());
+  launch(c.stream, transpose_scale_kernel, gridn(c, K1 * n), 256, 0, dP2.f64(), n, K1, s.f64(), dP2T.f64());
   IPEPS_LAUNCH_CHECK();
   axpy(c, cplx(1), dP2T, Z);
   Tensor BcolS = clone(c, Bcol);

@@ -83,6 +83,7 @@ __host__ __device__ __forceinline__ int col_base(int I, int nb) { return I * nb 
 template <bool CX>
 __global__ void __launch_bounds__(kCpThreads, 1)
     chol_panel_kernel(double* G, int k, int64_t ldg, double shift_factor, double2* __restrict__ Rpk, int write_g) {
+  pdl_wait();
   extern __shared__ __align__(16) double2 S[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int nb = (k + 7) >> 3, nblk = nb * (nb + 1) / 2;
@@ -290,6 +291,7 @@ template <int NB, bool CX>
 __global__ void __launch_bounds__(kTpThreads) trsm_panel_kernel(const double* __restrict__ Y, int64_t ldy, int64_t N,
                                                                 int k, int warps, const double2* __restrict__ Rpk,
                                                                 double* __restrict__ Q, int64_t ldq) {
+  pdl_wait();
   extern __shared__ __align__(16) double2 Rs[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int nb = (k + 7) >> 3, n2 = nb * (nb + 1) / 2 * 32;
@@ -352,8 +354,8 @@ template <bool CX>
 void launch_chol(Ctx& c, double* G, int k, int64_t ldg, double shift_factor, double* Rpk, bool write_g) {
   static SmemAttrOnce attr;
   attr.ensure(chol_panel_kernel<CX>, int(size_t(cholqr_packed(kCholqrMax)) * 8));
-  chol_panel_kernel<CX><<<1, kCpThreads, size_t(cholqr_packed(k)) * 8, c.stream>>>(
-      G, k, ldg, shift_factor, reinterpret_cast<double2*>(Rpk), write_g);
+  launch(c.stream, chol_panel_kernel<CX>, 1, kCpThreads, size_t(cholqr_packed(k)) * 8, G, k, ldg, shift_factor,
+         reinterpret_cast<double2*>(Rpk), write_g);
   IPEPS_LAUNCH_CHECK();
 }
 
@@ -366,8 +368,8 @@ void launch_trsm(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const d
   // eight rows per warp; one CTA per SM as long as eight warps hold its rows (R is staged once per CTA)
   const int64_t groups = (N + 7) / 8;
   const int64_t warps = std::min<int64_t>(kTpThreads / 32, (groups + c.sm_count - 1) / c.sm_count);
-  trsm_panel_kernel<NB, CX><<<unsigned((groups + warps - 1) / warps), kTpThreads, smem, c.stream>>>(
-      Y, ldy, N, k, int(warps), reinterpret_cast<const double2*>(Rpk), Q, ldq);
+  launch(c.stream, trsm_panel_kernel<NB, CX>, unsigned((groups + warps - 1) / warps), kTpThreads, smem, Y, ldy, N, k,
+         int(warps), reinterpret_cast<const double2*>(Rpk), Q, ldq);
   IPEPS_LAUNCH_CHECK();
 }
 

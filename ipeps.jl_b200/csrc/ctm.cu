@@ -340,6 +340,7 @@ namespace {
 
 // out[0..1] = tr(H rho) (complex), out[2..3] = tr(rho) (complex); FP64
 __global__ void dm_trace_kernel(const double* rho, int rho_complex, const double2* H, int n, double* out) {
+  pdl_wait();
   double hr = 0, hi = 0, tr = 0, ti = 0;
   for (int t = threadIdx.x; t < n * n; t += 32) {
     int i = t % n, j = t / n;  // tr(H rho) = sum_ij H[i,j] rho[j,i]
@@ -373,8 +374,8 @@ std::vector<Traces> dm_traces(Ctx& c, const std::vector<std::pair<Tensor, Tensor
     const Tensor& H = items[i].second;
     int d2 = int(rho.dims[0]);
     IPEPS_CHECK(H.dims[0] == d2 && H.dt == DType::C128, "dm_traces: H must be complex d^2 x d^2");
-    dm_trace_kernel<<<1, 32, 0, c.stream>>>(rho.f64(), rho.dt == DType::C128, static_cast<const double2*>(H.data()),
-                                            d2, d_out + 4 * i);
+    launch(c.stream, dm_trace_kernel, 1, 32, 0, rho.f64(), rho.dt == DType::C128,
+           static_cast<const double2*>(H.data()), d2, d_out + 4 * i);
     IPEPS_LAUNCH_CHECK();
     c.count(KFam::Reduce);
   }

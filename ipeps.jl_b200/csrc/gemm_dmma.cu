@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(WGM * WGN * KW * 32, MINB)
     dmma_gemm_kernel(int64_t M, int64_t N, int64_t K, int64_t kchunk, double alpha, const double* __restrict__ A,
                      int64_t lda, const double* __restrict__ B, int64_t ldb, double beta, double* __restrict__ C,
                      int64_t ldc, double* __restrict__ partial, int cs, int upper) {
+  pdl_wait();
   using GE = Geo<BM, BN, WGM, WGN, KW, AK, BK_>;
   constexpr int NT = GE::NT;
   constexpr int WM = BM / WGM, WN = BN / WGN;  // warp tile
@@ -219,6 +220,7 @@ __global__ void __launch_bounds__(WGM * WGN * KW * 32, MINB)
 // thread with 16-byte loads; the general case one element per thread.
 __global__ void dmma_splitk_reduce(int64_t M, int64_t N, int S, const double* __restrict__ partial, double alpha,
                                    double beta, double* __restrict__ C, int64_t ldc) {
+  pdl_wait();
   const int64_t tot = M * N;
   if (ldc == M && (tot & 1) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
     const int64_t i2 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, idx = 2 * i2;
@@ -279,26 +281,15 @@ void launch_cfg(Ctx& c, const Args& a, Split sp) {
   const int cz = sp.S / sp.cs;
   double* partial = nullptr;
   if (cz > 1) partial = static_cast<double*>(c.workspace(size_t(cz) * a.m * a.n * sizeof(double)));
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(unsigned(gx), unsigned(gy), unsigned(sp.S));
-  cfg.blockDim = dim3(GE::NT);
-  cfg.dynamicSmemBytes = GE::smem;
-  cfg.stream = c.stream;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = 1;
-  at.val.clusterDim.y = 1;
-  at.val.clusterDim.z = unsigned(sp.cs);
-  cfg.attrs = &at;
-  cfg.numAttrs = sp.cs > 1 ? 1 : 0;
-  IPEPS_CUDA(cudaLaunchKernelEx(&cfg, kern, a.m, a.n, a.k, kchunk, a.alpha, a.A, a.lda, a.B, a.ldb, a.beta, a.C, a.ldc,
-                                partial, sp.cs, int(a.upper)));
+  launch_clusters(c.stream, kern, dim3(unsigned(gx), unsigned(gy), unsigned(sp.S)), GE::NT, GE::smem,
+                  dim3(1, 1, unsigned(sp.cs)), a.m, a.n, a.k, kchunk, a.alpha, a.A, a.lda, a.B, a.ldb, a.beta, a.C,
+                  a.ldc, partial, sp.cs, int(a.upper));
   if (cz > 1) {
     const int64_t tot = a.m * a.n;
     const bool pairs = a.ldc == a.m && (tot & 1) == 0 && (reinterpret_cast<uintptr_t>(a.C) & 15) == 0;
     const int64_t threads = pairs ? tot / 2 : tot;
-    dmma_splitk_reduce<<<unsigned((threads + 255) / 256), 256, 0, c.stream>>>(a.m, a.n, cz, partial, a.alpha, a.beta,
-                                                                              a.C, a.ldc);
+    launch(c.stream, dmma_splitk_reduce, unsigned((threads + 255) / 256), 256, 0, a.m, a.n, cz, partial, a.alpha,
+           a.beta, a.C, a.ldc);
     IPEPS_LAUNCH_CHECK();
     c.count(KFam::Reduce, 0, double(cz + 2) * tot * sizeof(double));
   }

@@ -55,6 +55,7 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
 // k contiguous: X(r, k) = X[k + r*ld]; each thread converts 4 consecutive k
 __global__ void split_kc_kernel(const double* __restrict__ X, int64_t ld, int64_t rows, int64_t K, int64_t Kp,
                                 float* __restrict__ P) {
+  pdl_wait();
   const int64_t q = Kp / 4;
   const int64_t n = rows * q;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
@@ -74,6 +75,7 @@ __global__ void split_kc_kernel(const double* __restrict__ X, int64_t ld, int64_
 // rows contiguous: X(r, k) = X[r + k*ld]; 32 x 32 tiles through shared memory
 __global__ void split_tr_kernel(const double* __restrict__ X, int64_t ld, int64_t rows, int64_t K, int64_t Kp,
                                 float* __restrict__ P) {
+  pdl_wait();
   __shared__ double t[32][33];
   const int64_t r0 = int64_t(blockIdx.x) * 32, k0 = int64_t(blockIdx.y) * 32;
   const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
@@ -142,6 +144,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
 
 __global__ void __launch_bounds__(NTHREADS, 1)
     tf32x3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, Args a) {
+  pdl_wait();
   extern __shared__ unsigned char smem_raw[];
   char* smem = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int BN = a.BN, S = a.stages;
@@ -336,6 +339,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // C = alpha * sum_z partial[z] + beta * C, FP64 sums of the FP32 partials
 __global__ void splitk_reduce_kernel(int M, int N, int S, const float* __restrict__ partial, double alpha,
                                      double beta, double* __restrict__ C, int64_t ldc) {
+  pdl_wait();
   const int64_t tot = int64_t(M) * N;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < tot; i += int64_t(gridDim.x) * blockDim.x) {
     double s = 0;
@@ -412,11 +416,11 @@ Planes split_kmajor(Ctx& c, const double* X, int64_t ld, bool kcontig, int64_t r
   if (kcontig) {
     const int64_t n = rows * (p.Kp / 4);
     const int grid = int(std::min<int64_t>((n + 255) / 256, int64_t(c.sm_count) * 16));
-    split_kc_kernel<<<grid, 256, 0, c.stream>>>(X, ld, rows, K, p.Kp, P);
+    launch(c.stream, split_kc_kernel, grid, 256, 0, X, ld, rows, K, p.Kp, P);
   } else {
     IPEPS_CHECK(p.Kp / 32 <= 65535, "split_kmajor: K too large for the grid");
     dim3 grid{unsigned((rows + 31) / 32), unsigned(p.Kp / 32)};
-    split_tr_kernel<<<grid, dim3{32, 8}, 0, c.stream>>>(X, ld, rows, K, p.Kp, P);
+    launch(c.stream, split_tr_kernel, grid, dim3(32, 8), 0, X, ld, rows, K, p.Kp, P);
   }
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Permute, 0, double(rows) * K * 8 + double(rows) * p.Kp * 8);
@@ -463,13 +467,13 @@ void gemm_tf32x3_planes(Ctx& c, const Planes& PA, const Planes& PB, int64_t m, i
   const CUtensorMap mA = plane_map(PA, BM), mB = plane_map(PB, BN);
   const int grid = std::min(a.units, c.sm_count);
   ProfScope ps(c, KFam::GemmTF32x3);
-  tf32x3_kernel<<<grid, NTHREADS, smem, c.stream>>>(mA, mB, a);
+  launch(c.stream, tf32x3_kernel, grid, NTHREADS, smem, mA, mB, a);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::GemmTF32x3, 2.0 * double(m) * double(n) * double(k));
   if (S > 1) {
     const int64_t tot = m * n;
     const int rg = int(std::min<int64_t>((tot + 255) / 256, int64_t(c.sm_count) * 8));
-    splitk_reduce_kernel<<<rg, 256, 0, c.stream>>>(int(m), int(n), S, a.partial, alpha, beta, C, ldc);
+    launch(c.stream, splitk_reduce_kernel, rg, 256, 0, int(m), int(n), S, a.partial, alpha, beta, C, ldc);
     IPEPS_LAUNCH_CHECK();
     c.count(KFam::Reduce, 0, double(S) * tot * 4 + double(beta != 0.0 ? 2 : 1) * tot * 8);
   }

@@ -50,6 +50,7 @@ __global__ void __launch_bounds__(WGM * WGN * KW * 32)
     zmma_gemm_kernel(int64_t M, int64_t N, int64_t K, int64_t kchunk, double2 alpha, const EA* __restrict__ A,
                      int64_t lda, double sa, const EB* __restrict__ B, int64_t ldb, double sb, double2 beta,
                      double2* __restrict__ C, int64_t ldc, double2* __restrict__ partial, int cs) {
+  pdl_wait();
   using GE = Geo<BM, BN, WGM, WGN, KW, EA, EB, AK, BK_>;
   constexpr bool CA = std::is_same_v<EA, double2>, CB = std::is_same_v<EB, double2>;
   constexpr int NT = GE::NT;
@@ -218,6 +219,7 @@ __global__ void __launch_bounds__(WGM * WGN * KW * 32)
 // sum of the clusters' partial products, in split order
 __global__ void zmma_splitk_reduce(int64_t M, int64_t N, int S, const double2* __restrict__ partial, double2 alpha,
                                    double2 beta, double2* __restrict__ C, int64_t ldc) {
+  pdl_wait();
   const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, tot = M * N;
   if (idx >= tot) return;
   double2 v = partial[idx];
@@ -256,24 +258,13 @@ void launch_cfg(Ctx& c, const Args& a, int S, int cs) {
   const int cz = S / cs;
   double2* partial = nullptr;
   if (cz > 1) partial = static_cast<double2*>(c.workspace(size_t(cz) * a.m * a.n * sizeof(double2)));
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(unsigned(gx), unsigned(gy), unsigned(S));
-  cfg.blockDim = dim3(GE::NT);
-  cfg.dynamicSmemBytes = GE::smem;
-  cfg.stream = c.stream;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = 1;
-  at.val.clusterDim.y = 1;
-  at.val.clusterDim.z = unsigned(cs);
-  cfg.attrs = &at;
-  cfg.numAttrs = cs > 1 ? 1 : 0;
-  IPEPS_CUDA(cudaLaunchKernelEx(&cfg, kern, a.m, a.n, a.k, kchunk, a.alpha, static_cast<const EA*>(a.A), a.lda, a.sa,
-                                static_cast<const EB*>(a.B), a.ldb, a.sb, a.beta, a.C, a.ldc, partial, cs));
+  launch_clusters(c.stream, kern, dim3(unsigned(gx), unsigned(gy), unsigned(S)), GE::NT, GE::smem,
+                  dim3(1, 1, unsigned(cs)), a.m, a.n, a.k, kchunk, a.alpha, static_cast<const EA*>(a.A), a.lda, a.sa,
+                  static_cast<const EB*>(a.B), a.ldb, a.sb, a.beta, a.C, a.ldc, partial, cs);
   if (cz > 1) {
     const int64_t tot = a.m * a.n;
-    zmma_splitk_reduce<<<unsigned((tot + 255) / 256), 256, 0, c.stream>>>(a.m, a.n, cz, partial, a.alpha, a.beta, a.C,
-                                                                          a.ldc);
+    launch(c.stream, zmma_splitk_reduce, unsigned((tot + 255) / 256), 256, 0, a.m, a.n, cz, partial, a.alpha, a.beta,
+           a.C, a.ldc);
     IPEPS_LAUNCH_CHECK();
     c.count(KFam::Reduce, 0, double(cz + 2) * tot * sizeof(double2));
   }

@@ -19,6 +19,7 @@ namespace ipeps {
 namespace {
 
 __global__ void real_part_kernel(const double2* x, double* y, int64_t n) {
+  pdl_wait();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     y[i] = x[i].x;
 }
@@ -30,8 +31,8 @@ unsigned gridn(Ctx& c, int64_t n) {
 Tensor real_part(Ctx& c, const Tensor& x) {
   if (x.dt == DType::F64) return x;
   Tensor y = c.alloc(DType::F64, x.shape());
-  real_part_kernel<<<gridn(c, x.numel()), 256, 0, c.stream>>>(static_cast<const double2*>(x.data()), y.f64(),
-                                                              x.numel());
+  launch(c.stream, real_part_kernel, gridn(c, x.numel()), 256, 0, static_cast<const double2*>(x.data()), y.f64(),
+         x.numel());
   IPEPS_LAUNCH_CHECK();
   return y;
 }

@@ -185,6 +185,7 @@ __device__ __forceinline__ void store_col(const T (&u)[NR], T* x, int lane) {
 // k = 62 244 -> 128 us, k = 98 587 -> 288, k = 128 588 -> 336, k = 160 888 -> 556.
 template <class T, int NR>
 __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) jacobi_cluster_kernel(JcArgs a) {
+  pdl_wait();
   extern __shared__ __align__(16) double jsm[];
   cg::cluster_group cluster = cg::this_cluster();
   constexpr int H = 32 * NR;
@@ -342,7 +343,7 @@ template <class T, int NR>
 void launch_cluster(Ctx& c, const JcArgs& a, size_t smem) {
   static SmemAttrOnce attr;
   attr.ensure(jacobi_cluster_kernel<T, NR>, int(kJSmemMax));
-  jacobi_cluster_kernel<T, NR><<<kJP, kJWarps * 32, smem, c.stream>>>(a);
+  launch(c.stream, jacobi_cluster_kernel<T, NR>, kJP, kJWarps * 32, smem, a);
   IPEPS_LAUNCH_CHECK();
 }
 

@@ -19,6 +19,7 @@ constexpr int kThreads = 1024;
 // residual of size ~0 instead of blowing up).  shift is added to the diagonal.
 __global__ void __launch_bounds__(kThreads) chol_kernel(double* G, int k, int64_t ldg, double shift,
                                                         int* status) {
+  pdl_wait();
   __shared__ double s_piv;
   __shared__ double s_tr;
   if (threadIdx.x == 0) {
@@ -61,6 +62,7 @@ __global__ void __launch_bounds__(kThreads) chol_kernel(double* G, int k, int64_
 // X[i, j] = -(sum_{l=i+1..j} R[i,l] X[l,j]) / R[i,i], X[i,i] = 1/R[i,i].
 __global__ void __launch_bounds__(kThreads) triinv_kernel(const double* R, int k, int64_t ldr, double* X,
                                                           int64_t ldx) {
+  pdl_wait();
   for (int64_t t = threadIdx.x; t < int64_t(k) * k; t += blockDim.x) {
     int i = int(t % k), j = int(t / k);
     X[i + j * ldx] = (i == j) ? 1.0 / R[i + i * ldr] : 0.0;
@@ -88,6 +90,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 __global__ void __launch_bounds__(kThreads) jacobi_kernel(double* X, int m, int k, int64_t ldx, double* J,
                                                           int64_t ldj, double* S, int max_sweeps, double tol,
                                                           int* status, int* sweeps_out) {
+  pdl_wait();
   __shared__ double s_off;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   for (int64_t t = threadIdx.x; t < int64_t(k) * k; t += blockDim.x) {
@@ -159,6 +162,7 @@ __global__ void __launch_bounds__(kThreads) jacobi_kernel(double* X, int m, int 
 // Descending sort of S (length k <= 4096) with permutation; ties keep the
 // later index first (the reference reverses an ascending stable sortperm).
 __global__ void sort_desc_kernel(const double* S, int k, double* S_out, int* perm) {
+  pdl_wait();
   extern __shared__ unsigned char sm_raw[];
   double* v = reinterpret_cast<double*>(sm_raw);
   // (a NaN sorts last: perm stays a permutation, the gathers that use it stay in range)
@@ -180,6 +184,7 @@ __global__ void sort_desc_kernel(const double* S, int k, double* S_out, int* per
 // out[:, j] = in[:, perm[j]] * (scale ? scale[j] : 1), j < ncols
 __global__ void gather_cols_kernel(const double* in, int64_t ldi, int64_t m, const int* perm, int ncols,
                                    const double* scale_v, int scale_mode, double* out, int64_t ldo) {
+  pdl_wait();
   int64_t tot = m * ncols;
   for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < tot; t += int64_t(gridDim.x) * blockDim.x) {
     int64_t i = t % m;
@@ -193,6 +198,7 @@ __global__ void gather_cols_kernel(const double* in, int64_t ldi, int64_t m, con
 
 // y[:, j] *= f(s[j]), f: 1 -> 1/sqrt(s)
 __global__ void scale_cols_kernel(double* X, int64_t ldx, int64_t m, int ncols, const double* s, int mode) {
+  pdl_wait();
   int64_t tot = m * ncols;
   for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < tot; t += int64_t(gridDim.x) * blockDim.x) {
     int64_t i = t % m;
@@ -205,6 +211,7 @@ __global__ void scale_cols_kernel(double* X, int64_t ldx, int64_t m, int ncols, 
 }
 
 __global__ void scale_rows_kernel(double* X, int64_t ldx, int64_t m, int64_t ncols, const double* s, int mode) {
+  pdl_wait();
   int64_t tot = m * ncols;
   for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < tot; t += int64_t(gridDim.x) * blockDim.x) {
     int64_t i = t % m, j = t / m;
@@ -215,6 +222,7 @@ __global__ void scale_rows_kernel(double* X, int64_t ldx, int64_t m, int64_t nco
 
 // trace of G (k x k) -> out
 __global__ void trace_kernel(const double* G, int k, int64_t ldg, double* out) {
+  pdl_wait();
   double s = 0;
   for (int i = threadIdx.x; i < k; i += blockDim.x) s += G[i + i * ldg];
   s = warp_sum(s);
@@ -229,6 +237,7 @@ __global__ void trace_kernel(const double* G, int k, int64_t ldg, double* out) {
 }
 
 __global__ void shift_diag_kernel(double* G, int k, int64_t ldg, const double* tr, double factor) {
+  pdl_wait();
   const double sft = factor * (*tr);
   for (int i = threadIdx.x; i < k; i += blockDim.x) G[i + i * ldg] += sft;
 }
@@ -241,24 +250,24 @@ unsigned grid_for(Ctx& c, int64_t n) {
 
 void chol_upper(Ctx& c, double* G, int k, int64_t ldg, const double* d_trace_shift, double shift_factor) {
   if (d_trace_shift) {
-    shift_diag_kernel<<<1, 256, 0, c.stream>>>(G, k, ldg, d_trace_shift, shift_factor);
+    launch(c.stream, shift_diag_kernel, 1, 256, 0, G, k, ldg, d_trace_shift, shift_factor);
     IPEPS_LAUNCH_CHECK();
   }
   ProfScope ps(c, KFam::SmallLinalg);
-  chol_kernel<<<1, kThreads, 0, c.stream>>>(G, k, ldg, 0.0, c.d_status);
+  launch(c.stream, chol_kernel, 1, kThreads, 0, G, k, ldg, 0.0, c.d_status);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::SmallLinalg, double(k) * k * k / 3.0);
 }
 
 void triinv_upper(Ctx& c, const double* R, int k, int64_t ldr, double* X, int64_t ldx) {
   ProfScope ps(c, KFam::SmallLinalg);
-  triinv_kernel<<<1, kThreads, 0, c.stream>>>(R, k, ldr, X, ldx);
+  launch(c.stream, triinv_kernel, 1, kThreads, 0, R, k, ldr, X, ldx);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::SmallLinalg, double(k) * k * k / 3.0);
 }
 
 void trace(Ctx& c, const double* G, int k, int64_t ldg, double* d_out) {
-  trace_kernel<<<1, 256, 0, c.stream>>>(G, k, ldg, d_out);
+  launch(c.stream, trace_kernel, 1, 256, 0, G, k, ldg, d_out);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Reduce);
 }
@@ -266,34 +275,34 @@ void trace(Ctx& c, const double* G, int k, int64_t ldg, double* d_out) {
 void jacobi_svd(Ctx& c, double* X, int m, int k, int64_t ldx, double* J, int64_t ldj, double* S,
                 int max_sweeps, double tol, int* d_sweeps) {
   ProfScope ps(c, KFam::Jacobi);
-  jacobi_kernel<<<1, kThreads, 0, c.stream>>>(X, m, k, ldx, J, ldj, S, max_sweeps, tol, c.d_status, d_sweeps);
+  launch(c.stream, jacobi_kernel, 1, kThreads, 0, X, m, k, ldx, J, ldj, S, max_sweeps, tol, c.d_status, d_sweeps);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Jacobi, 6.0 * double(m + k) * k * k / 2.0);
 }
 
 void sort_desc(Ctx& c, const double* S, int k, double* S_out, int* perm) {
   IPEPS_CHECK(k <= 4096, "sort_desc: k too large");
-  sort_desc_kernel<<<1, 1024, size_t(k) * sizeof(double), c.stream>>>(S, k, S_out, perm);
+  launch(c.stream, sort_desc_kernel, 1, 1024, size_t(k) * sizeof(double), S, k, S_out, perm);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::SmallLinalg);
 }
 
 void gather_cols(Ctx& c, const double* in, int64_t ldi, int64_t m, const int* perm, int ncols,
                  const double* scale_v, int scale_mode, double* out, int64_t ldo) {
-  gather_cols_kernel<<<grid_for(c, m * ncols), 256, 0, c.stream>>>(in, ldi, m, perm, ncols, scale_v, scale_mode,
-                                                                   out, ldo);
+  launch(c.stream, gather_cols_kernel, grid_for(c, m * ncols), 256, 0, in, ldi, m, perm, ncols, scale_v, scale_mode,
+         out, ldo);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Elementwise, 0, 16.0 * m * ncols);
 }
 
 void scale_cols(Ctx& c, double* X, int64_t ldx, int64_t m, int ncols, const double* s, int mode) {
-  scale_cols_kernel<<<grid_for(c, m * ncols), 256, 0, c.stream>>>(X, ldx, m, ncols, s, mode);
+  launch(c.stream, scale_cols_kernel, grid_for(c, m * ncols), 256, 0, X, ldx, m, ncols, s, mode);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Elementwise, 0, 16.0 * m * ncols);
 }
 
 void scale_rows(Ctx& c, double* X, int64_t ldx, int64_t m, int64_t ncols, const double* s, int mode) {
-  scale_rows_kernel<<<grid_for(c, m * ncols), 256, 0, c.stream>>>(X, ldx, m, ncols, s, mode);
+  launch(c.stream, scale_rows_kernel, grid_for(c, m * ncols), 256, 0, X, ldx, m, ncols, s, mode);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Elementwise, 0, 16.0 * m * ncols);
 }

@@ -124,6 +124,7 @@ struct PermArgs {
 
 template <typename T>
 __global__ void permute_simple(PermArgs a, int64_t total, const T* __restrict__ in, T* __restrict__ out) {
+  pdl_wait();
   for (int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
        idx += int64_t(gridDim.x) * blockDim.x) {
     int64_t r = idx, off = 0;
@@ -160,6 +161,7 @@ constexpr int64_t kPermChunk = 2048;
 // short row).
 template <typename T, bool SMALL>
 __global__ void permute_rows(RowArgs a, int64_t rows, int64_t nchunk, const T* __restrict__ in, T* __restrict__ out) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
   const int64_t units = rows * nchunk;
@@ -217,6 +219,7 @@ struct TileArgs {
 
 template <typename T>
 __global__ void permute_tiled(TileArgs a, const T* __restrict__ in, T* __restrict__ out) {
+  pdl_wait();
   __shared__ T tile[32][33];
   const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
   const int64_t x0 = int64_t(blockIdx.x) * 32, y0 = int64_t(blockIdx.y) * 32;
@@ -269,9 +272,9 @@ void permute_impl(Ctx& c, const Tensor& in, const std::vector<int>& perm, Tensor
     bool small = rows * nchunk <= int64_t(UINT32_MAX);
     for (int i = 0; i < a.nd; ++i) small = small && a.odims[i] <= int64_t(UINT32_MAX);
     if (small)
-      permute_rows<T, true><<<unsigned(std::max<int64_t>(blocks, 1)), 256, 0, c.stream>>>(a, rows, nchunk, ip, op);
+      launch(c.stream, permute_rows<T, true>, unsigned(std::max<int64_t>(blocks, 1)), 256, 0, a, rows, nchunk, ip, op);
     else
-      permute_rows<T, false><<<unsigned(std::max<int64_t>(blocks, 1)), 256, 0, c.stream>>>(a, rows, nchunk, ip, op);
+      launch(c.stream, permute_rows<T, false>, unsigned(std::max<int64_t>(blocks, 1)), 256, 0, a, rows, nchunk, ip, op);
   } else if (perm[0] == 0 || in.dims[0] == 1 || out.dims[0] == 1) {
     PermArgs a{};
     a.nd = nd;
@@ -280,7 +283,7 @@ void permute_impl(Ctx& c, const Tensor& in, const std::vector<int>& perm, Tensor
       a.istride[i] = istr[perm[i]];
     }
     int64_t blocks = std::min<int64_t>((total + 255) / 256, int64_t(c.sm_count) * 16);
-    permute_simple<T><<<unsigned(std::max<int64_t>(blocks, 1)), 256, 0, c.stream>>>(a, total, ip, op);
+    launch(c.stream, permute_simple<T>, unsigned(std::max<int64_t>(blocks, 1)), 256, 0, a, total, ip, op);
   } else {
     const int q = perm[0];
     int p = 0;
@@ -307,7 +310,7 @@ void permute_impl(Ctx& c, const Tensor& in, const std::vector<int>& perm, Tensor
     dim3 grid(unsigned((a.n0 + 31) / 32), unsigned((a.nq + 31) / 32),
               unsigned(std::min<int64_t>(a.rest_total, 65535)));
     IPEPS_CHECK(grid.x <= 2147483647u && grid.y <= 65535u, "permute: grid too large");
-    permute_tiled<T><<<grid, dim3(32, 8), 0, c.stream>>>(a, ip, op);
+    launch(c.stream, permute_tiled<T>, grid, dim3(32, 8), 0, a, ip, op);
   }
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Permute, 0, 2.0 * double(total) * sizeof(T));
@@ -389,6 +392,7 @@ __device__ __forceinline__ double absval(double2 x) { return hypot(x.x, x.y); }
 
 template <typename T>
 __global__ void maxabs_kernel(const T* __restrict__ x, int64_t n, unsigned long long* out) {
+  pdl_wait();
   double m = 0.0;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     m = fmax(m, absval(x[i]));
@@ -405,12 +409,14 @@ __global__ void maxabs_kernel(const T* __restrict__ x, int64_t n, unsigned long 
 }
 
 __global__ void scale_inv_kernel(double* __restrict__ x, int64_t n, const double* __restrict__ s) {
+  pdl_wait();
   const double inv = 1.0 / s[0];
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     x[i] *= inv;
 }
 
 __global__ void scale_c_kernel(double2* __restrict__ x, int64_t n, double2 s) {
+  pdl_wait();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
     double2 v = x[i];
     x[i] = make_double2(v.x * s.x - v.y * s.y, v.x * s.y + v.y * s.x);
@@ -418,16 +424,19 @@ __global__ void scale_c_kernel(double2* __restrict__ x, int64_t n, double2 s) {
 }
 
 __global__ void scale_r_kernel(double* __restrict__ x, int64_t n, double s) {
+  pdl_wait();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     x[i] *= s;
 }
 
 __global__ void axpy_r_kernel(double a, const double* __restrict__ x, double* __restrict__ y, int64_t n) {
+  pdl_wait();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     y[i] = fma(a, x[i], y[i]);
 }
 
 __global__ void axpy_c_kernel(double2 a, const double2* __restrict__ x, double2* __restrict__ y, int64_t n) {
+  pdl_wait();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
     double2 v = x[i], w = y[i];
     w.x += a.x * v.x - a.y * v.y;
@@ -437,6 +446,7 @@ __global__ void axpy_c_kernel(double2 a, const double2* __restrict__ x, double2*
 }
 
 __global__ void axpy_rc_kernel(double2 a, const double* __restrict__ x, double2* __restrict__ y, int64_t n) {
+  pdl_wait();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
     double v = x[i];
     double2 w = y[i];
@@ -447,6 +457,7 @@ __global__ void axpy_rc_kernel(double2 a, const double* __restrict__ x, double2*
 }
 
 __global__ void conj_kernel(const double2* __restrict__ x, double2* __restrict__ y, int64_t n) {
+  pdl_wait();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
     double2 v = x[i];
     y[i] = make_double2(v.x, -v.y);
@@ -454,13 +465,18 @@ __global__ void conj_kernel(const double2* __restrict__ x, double2* __restrict__
 }
 
 __global__ void to_complex_kernel(const double* __restrict__ x, double2* __restrict__ y, int64_t n) {
+  pdl_wait();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     y[i] = make_double2(x[i], 0.0);
 }
 
-__global__ void flag_status_kernel(int* status, int bits) { atomicOr(status, bits); }
+__global__ void flag_status_kernel(int* status, int bits) {
+  pdl_wait();
+  atomicOr(status, bits);
+}
 
 __global__ void finite_kernel(const double* __restrict__ x, int64_t n, int* status) {
+  pdl_wait();
   bool bad = false;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     bad |= !isfinite(x[i]);
@@ -476,6 +492,7 @@ __device__ __forceinline__ uint64_t splitmix(uint64_t z) {
 }
 
 __global__ void randn_kernel(double* __restrict__ x, int64_t n, uint64_t seed) {
+  pdl_wait();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
     uint64_t a = splitmix(seed ^ (2 * uint64_t(i)));
     uint64_t b = splitmix(seed ^ (2 * uint64_t(i) + 1));
@@ -495,17 +512,18 @@ void maxabs(Ctx& c, const Tensor& x, double* d_out) {
   IPEPS_CUDA(cudaMemsetAsync(d_out, 0, sizeof(double), c.stream));
   const int64_t n = x.numel();
   if (x.dt == DType::F64)
-    maxabs_kernel<double><<<grid_for(c, n), 256, 0, c.stream>>>(x.f64(), n, reinterpret_cast<unsigned long long*>(d_out));
+    launch(c.stream, maxabs_kernel<double>, grid_for(c, n), 256, 0, x.f64(), n,
+           reinterpret_cast<unsigned long long*>(d_out));
   else
-    maxabs_kernel<double2><<<grid_for(c, n), 256, 0, c.stream>>>(static_cast<const double2*>(x.data()), n,
-                                                                  reinterpret_cast<unsigned long long*>(d_out));
+    launch(c.stream, maxabs_kernel<double2>, grid_for(c, n), 256, 0, static_cast<const double2*>(x.data()), n,
+           reinterpret_cast<unsigned long long*>(d_out));
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Reduce, 0, double(x.bytes()));
 }
 
 void scale_inv(Ctx& c, Tensor& x, const double* d_s) {
   const int64_t n = x.numel() * (x.dt == DType::F64 ? 1 : 2);
-  scale_inv_kernel<<<grid_for(c, n), 256, 0, c.stream>>>(x.f64(), n, d_s);
+  launch(c.stream, scale_inv_kernel, grid_for(c, n), 256, 0, x.f64(), n, d_s);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Elementwise, 0, 2.0 * double(x.bytes()));
 }
@@ -514,9 +532,10 @@ void scale(Ctx& c, Tensor& x, cuDoubleComplex s) {
   const int64_t n = x.numel();
   if (x.dt == DType::F64) {
     IPEPS_CHECK(s.y == 0.0, "scale: complex factor on real tensor");
-    scale_r_kernel<<<grid_for(c, n), 256, 0, c.stream>>>(x.f64(), n, s.x);
+    launch(c.stream, scale_r_kernel, grid_for(c, n), 256, 0, x.f64(), n, s.x);
   } else {
-    scale_c_kernel<<<grid_for(c, n), 256, 0, c.stream>>>(static_cast<double2*>(x.data()), n, make_double2(s.x, s.y));
+    launch(c.stream, scale_c_kernel, grid_for(c, n), 256, 0, static_cast<double2*>(x.data()), n,
+           make_double2(s.x, s.y));
   }
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Elementwise, 0, 2.0 * double(x.bytes()));
@@ -527,12 +546,13 @@ void axpy(Ctx& c, cuDoubleComplex a, const Tensor& x, Tensor& y) {
   const int64_t n = x.numel();
   if (y.dt == DType::F64) {
     IPEPS_CHECK(x.dt == DType::F64 && a.y == 0.0, "axpy: complex into real");
-    axpy_r_kernel<<<grid_for(c, n), 256, 0, c.stream>>>(a.x, x.f64(), y.f64(), n);
+    launch(c.stream, axpy_r_kernel, grid_for(c, n), 256, 0, a.x, x.f64(), y.f64(), n);
   } else if (x.dt == DType::C128) {
-    axpy_c_kernel<<<grid_for(c, n), 256, 0, c.stream>>>(make_double2(a.x, a.y), static_cast<const double2*>(x.data()),
-                                                         static_cast<double2*>(y.data()), n);
+    launch(c.stream, axpy_c_kernel, grid_for(c, n), 256, 0, make_double2(a.x, a.y),
+           static_cast<const double2*>(x.data()), static_cast<double2*>(y.data()), n);
   } else {
-    axpy_rc_kernel<<<grid_for(c, n), 256, 0, c.stream>>>(make_double2(a.x, a.y), x.f64(), static_cast<double2*>(y.data()), n);
+    launch(c.stream, axpy_rc_kernel, grid_for(c, n), 256, 0, make_double2(a.x, a.y), x.f64(),
+           static_cast<double2*>(y.data()), n);
   }
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Elementwise, 0, 3.0 * double(y.bytes()));
@@ -541,8 +561,8 @@ void axpy(Ctx& c, cuDoubleComplex a, const Tensor& x, Tensor& y) {
 Tensor conj(Ctx& c, const Tensor& x) {
   if (x.dt == DType::F64) return clone(c, x);
   Tensor y = c.alloc(x.dt, x.shape());
-  conj_kernel<<<grid_for(c, x.numel()), 256, 0, c.stream>>>(static_cast<const double2*>(x.data()),
-                                                           static_cast<double2*>(y.data()), x.numel());
+  launch(c.stream, conj_kernel, grid_for(c, x.numel()), 256, 0, static_cast<const double2*>(x.data()),
+         static_cast<double2*>(y.data()), x.numel());
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Elementwise, 0, 2.0 * double(x.bytes()));
   return y;
@@ -551,7 +571,8 @@ Tensor conj(Ctx& c, const Tensor& x) {
 Tensor to_complex(Ctx& c, const Tensor& x) {
   if (x.dt == DType::C128) return x;
   Tensor y = c.alloc(DType::C128, x.shape());
-  to_complex_kernel<<<grid_for(c, x.numel()), 256, 0, c.stream>>>(x.f64(), static_cast<double2*>(y.data()), x.numel());
+  launch(c.stream, to_complex_kernel, grid_for(c, x.numel()), 256, 0, x.f64(), static_cast<double2*>(y.data()),
+         x.numel());
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Elementwise, 0, 3.0 * double(x.bytes()));
   return y;
@@ -559,13 +580,13 @@ Tensor to_complex(Ctx& c, const Tensor& x) {
 
 void check_finite(Ctx& c, const Tensor& x) {
   const int64_t n = x.numel() * (x.dt == DType::F64 ? 1 : 2);
-  finite_kernel<<<grid_for(c, n), 256, 0, c.stream>>>(x.f64(), n, c.d_status);
+  launch(c.stream, finite_kernel, grid_for(c, n), 256, 0, x.f64(), n, c.d_status);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Reduce, 0, double(x.bytes()));
 }
 
 void flag_status(Ctx& c, int bits) {
-  flag_status_kernel<<<1, 1, 0, c.stream>>>(c.d_status, bits);
+  launch(c.stream, flag_status_kernel, 1, 1, 0, c.d_status, bits);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Reduce);
 }
@@ -573,7 +594,7 @@ void flag_status(Ctx& c, int bits) {
 void randn(Ctx& c, Tensor& x) {
   const int64_t n = x.numel() * (x.dt == DType::F64 ? 1 : 2);
   uint64_t seed = c.rng_seed * 0x2545F4914F6CDD1DULL + (c.rng_counter++);
-  randn_kernel<<<grid_for(c, n), 256, 0, c.stream>>>(x.f64(), n, seed);
+  launch(c.stream, randn_kernel, grid_for(c, n), 256, 0, x.f64(), n, seed);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Elementwise, 0, double(x.bytes()));
 }

@@ -158,6 +158,7 @@ namespace {
 
 // out[j] = ||X[:, j]|| for j < nc (FP64, one warp per column)
 __global__ void colnorms_kernel(const double* X, int64_t m, int nc, double* out) {
+  pdl_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= nc) return;
   double s = 0;
@@ -168,6 +169,7 @@ __global__ void colnorms_kernel(const double* X, int64_t m, int nc, double* out)
 
 // max over columns j < nc of ||X[:, j]|| (FP64, one warp per column)
 __global__ void colnorm_max_kernel(const double* X, int64_t m, int nc, unsigned long long* out) {
+  pdl_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= nc) return;
   double s = 0;
@@ -178,6 +180,7 @@ __global__ void colnorm_max_kernel(const double* X, int64_t m, int nc, unsigned 
 
 // y -= f norm^2 x
 __global__ void sub_shift_kernel(double f, const double* norm, const double* x, double* y, int64_t n) {
+  pdl_wait();
   const double a = -f * norm[0] * norm[0];
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     y[i] = fma(a, x[i], y[i]);
@@ -220,7 +223,7 @@ struct RealOps {
     }
     const int64_t n = W.numel();
     const unsigned grid = unsigned(std::min<int64_t>((n + 255) / 256, int64_t(c.sm_count) * 8));
-    sub_shift_kernel<<<grid, 256, 0, c.stream>>>(f, norm, T.f64(), W.f64(), n);
+    launch(c.stream, sub_shift_kernel, grid, 256, 0, f, norm, T.f64(), W.f64(), n);
     IPEPS_LAUNCH_CHECK();
     c.count(KFam::Elementwise, 0, 24.0 * n);
     return orth_(W, inter);
@@ -339,7 +342,7 @@ Sketch sketch_pass(Ctx& c, Ops& o, const Tensor& Om, int q, const SvdParams& sp,
   Tensor Z = Om, Y = o.M(Om);
   double* norm = reinterpret_cast<double*>(c.scal->p) + 56;
   if (b > 0 && q > 0) {
-    colnorms_kernel<<<1, 32, 0, c.stream>>>(Y.f64(), o.N1(), 1, norm);
+    launch(c.stream, colnorms_kernel, 1, 32, 0, Y.f64(), o.N1(), 1, norm);
     IPEPS_LAUNCH_CHECK();
   }
   for (int it = 0; it < q; ++it) {
@@ -528,8 +531,8 @@ ProjResult projector_impl(Ctx& c, Ops& o, int chi, const SvdParams& sp, ProjCach
     gather_cols(c, sk.X.f64(), w * k, w * k, d_perm, nr, nullptr, 0, Us.f64(), w * k);  // W = Ux S
     gemm(c, dt, 'N', 'N', N1, nr, k, cplx(-1), sk.Q.data(), N1, Us.data(), k, cplx(1), Res.data(), N1, true);
     IPEPS_CUDA(cudaMemsetAsync(d_res, 0, 8, c.stream));
-    colnorm_max_kernel<<<(nr * 32 + 255) / 256, 256, 0, c.stream>>>(Res.f64(), w * N1, nr,
-                                                                    reinterpret_cast<unsigned long long*>(d_res));
+    launch(c.stream, colnorm_max_kernel, (nr * 32 + 255) / 256, 256, 0, Res.f64(), w * N1, nr,
+           reinterpret_cast<unsigned long long*>(d_res));
     IPEPS_LAUNCH_CHECK();
     double res = 0;
     IPEPS_CUDA(cudaMemcpyAsync(&res, d_res, 8, cudaMemcpyDeviceToHost, c.stream));
@@ -609,7 +612,7 @@ ProjResult projector_impl(Ctx& c, Ops& o, int chi, const SvdParams& sp, ProjCach
       gather_cols(c, sk.X.f64(), k, k, d_perm, rr, nullptr, 0, Wall.f64(), k);
       gemm(c, dt, 'N', 'N', N1, rr, k, cplx(-1), sk.Q.data(), N1, Wall.data(), k, cplx(1), Res.data(), N1, true);
       Tensor rn = c.alloc(DType::F64, {rr});
-      colnorms_kernel<<<(rr * 32 + 255) / 256, 256, 0, c.stream>>>(Res.f64(), N1, rr, rn.f64());
+      launch(c.stream, colnorms_kernel, (rr * 32 + 255) / 256, 256, 0, Res.f64(), N1, rr, rn.f64());
       IPEPS_LAUNCH_CHECK();
       std::vector<double> rh(rr);
       IPEPS_CUDA(cudaMemcpyAsync(rh.data(), rn.data(), size_t(rr) * 8, cudaMemcpyDeviceToHost, c.stream));

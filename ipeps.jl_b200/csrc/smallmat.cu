@@ -43,6 +43,7 @@ size_t chol_smem_doubles(int k) {
 // the row-parallel triangular solve stages with contiguous copies).
 __global__ void __launch_bounds__(kCholThreads) chol_blocked_kernel(double* G, int k, int64_t ldg,
                                                                     double shift_factor, double* Rrow) {
+  pdl_wait();
   extern __shared__ __align__(16) double sm[];
   const int npk = ((k * (k + 1)) / 2 + 1) & ~1;
   double* P = sm;                                     // packed upper triangle
@@ -215,6 +216,7 @@ template <int NS>
 __global__ void __launch_bounds__(512, 1) trsm_rows_kernel(const double* Y, int64_t ldy, int64_t N, int k,
                                                            const double* R, int64_t ldr, const double* Rrow,
                                                            double* Q, int64_t ldq) {
+  pdl_wait();
   extern __shared__ __align__(16) double sm[];
   const int kp = k | 1;
   const int nthr = blockDim.x, nwarp = nthr >> 5, rows = nwarp * kTrsmRPW;
@@ -341,6 +343,7 @@ template <int NV>
 __global__ void __launch_bounds__(kJacThreads) jacobi_log_kernel(double* Xg, int m, int k, int64_t ldx, double2* rot,
                                                                  int max_sweeps, double tol, double* S, int* status,
                                                                  int* sweeps_out) {
+  pdl_wait();
   extern __shared__ __align__(16) double X[];
   constexpr int mp = 16 * NV;
   double* nrm = X + int64_t(mp) * k;
@@ -455,6 +458,7 @@ size_t apply_smem_bytes(int k) {
 // applied.
 __global__ void __launch_bounds__(kApplyRows * 32) jacobi_apply_kernel(const double2* rot, int k, const int* d_sweeps,
                                                                      double* J, int64_t ldj) {
+  pdl_wait();
   extern __shared__ __align__(16) double sm2[];
   const int kk = (k + 1) & ~1, np = kk / 2;
   double2* logb = reinterpret_cast<double2*>(sm2);  // 2 x kChunk x np
@@ -516,7 +520,8 @@ template <int NV>
 void launch_jacobi(Ctx& c, double* X, int m, int k, int64_t ldx, double2* rot, int max_sweeps, double tol, double* S,
                    int* d_sweeps, size_t smem) {
   g_jlog_attr[NV].ensure(jacobi_log_kernel<NV>, int(kSmemMax));
-  jacobi_log_kernel<NV><<<1, kJacThreads, smem, c.stream>>>(X, m, k, ldx, rot, max_sweeps, tol, S, c.d_status, d_sweeps);
+  launch(c.stream, jacobi_log_kernel<NV>, 1, kJacThreads, smem, X, m, k, ldx, rot, max_sweeps, tol, S, c.d_status,
+         d_sweeps);
   IPEPS_LAUNCH_CHECK();
 }
 
@@ -528,7 +533,7 @@ void launch_trsm(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const d
   g_trsm_attr[NS].ensure(trsm_rows_kernel<NS>, int(kSmemMax));
   const int64_t rows = int64_t(warps) * kTrsmRPW;
   const unsigned grid = unsigned(std::min<int64_t>((N + rows - 1) / rows, std::max(c.sm_count, 1)));
-  trsm_rows_kernel<NS><<<grid, warps * 32, smem, c.stream>>>(Y, ldy, N, k, R, ldr, Rrow, Q, ldq);
+  launch(c.stream, trsm_rows_kernel<NS>, grid, warps * 32, smem, Y, ldy, N, k, R, ldr, Rrow, Q, ldq);
   IPEPS_LAUNCH_CHECK();
 }
 
@@ -540,7 +545,7 @@ void chol_blocked(Ctx& c, double* G, int k, int64_t ldg, double shift_factor, do
   IPEPS_CHECK(chol_fits(k), "chol_blocked: k out of range");
   ProfScope ps(c, KFam::SmallLinalg);
   g_chol_attr.ensure(chol_blocked_kernel, int(kSmemMax));
-  chol_blocked_kernel<<<1, kCholThreads, chol_smem_doubles(k) * 8, c.stream>>>(G, k, ldg, shift_factor, Rrow);
+  launch(c.stream, chol_blocked_kernel, 1, kCholThreads, chol_smem_doubles(k) * 8, G, k, ldg, shift_factor, Rrow);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::SmallLinalg, double(k) * k * k / 3.0);
 }
@@ -589,7 +594,7 @@ void jacobi_svd_auto(Ctx& c, double* X, int m, int k, int64_t ldx, double* J, in
     ProfScope ps(c, KFam::Jacobi);
     g_apply_attr.ensure(jacobi_apply_kernel, int(kSmemMax));
     const unsigned grid = unsigned((k + kApplyRows - 1) / kApplyRows);
-    jacobi_apply_kernel<<<grid, kApplyRows * 32, apply_smem_bytes(k), c.stream>>>(rp, k, d_sweeps, J, ldj);
+    launch(c.stream, jacobi_apply_kernel, grid, kApplyRows * 32, apply_smem_bytes(k), rp, k, d_sweeps, J, ldj);
     IPEPS_LAUNCH_CHECK();
     c.count(KFam::Jacobi, 6.0 * double(k) * k * k / 2.0);
   }

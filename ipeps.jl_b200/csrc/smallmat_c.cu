@@ -34,6 +34,7 @@ constexpr int kCholCThreads = 256;
 // Guarded Cholesky of a Hermitian positive semi-definite G (upper triangle
 // read): the same shift and pivot guard as the real kernel.  G <- R.
 __global__ void __launch_bounds__(kCholCThreads) chol_c_kernel(double2* G, int k, int64_t ldg, double shift_factor) {
+  pdl_wait();
   extern __shared__ __align__(16) double2 Pc[];
   double2* rowj = Pc + (k * (k + 1)) / 2;
   __shared__ double s_red[kCholCThreads / 32];
@@ -93,6 +94,7 @@ constexpr int kTrsmCRows = 8;
 __global__ void __launch_bounds__(kTrsmCRows * 32) trsm_c_kernel(const double2* Y, int64_t ldy, int64_t N, int k,
                                                                  const double2* R, int64_t ldr, double2* Q,
                                                                  int64_t ldq) {
+  pdl_wait();
   extern __shared__ __align__(16) double2 smc[];
   double2* Rs = smc;                                                // column-major packed upper, k(k+1)/2
   double2* rows = Rs + (k * (k + 1)) / 2;                           // kTrsmCRows x k
@@ -155,6 +157,7 @@ __device__ __forceinline__ double hsum16c(double v) {
 __global__ void __launch_bounds__(1024) jacobi_c_kernel(double2* Xg, int m, int k, int64_t ldx, double2* rot,
                                                         int max_sweeps, double tol, double* S, int* status,
                                                         int* sweeps_out) {
+  pdl_wait();
   extern __shared__ __align__(16) double2 Xc[];
   double* nrm = reinterpret_cast<double*>(Xc + int64_t(m) * k);
   __shared__ int s_rot;
@@ -260,6 +263,7 @@ constexpr int kApplyCRows = 8;
 __global__ void __launch_bounds__(kApplyCRows * 32) jacobi_c_apply_kernel(const double2* rot, int k,
                                                                          const int* d_sweeps, double2* J,
                                                                          int64_t ldj) {
+  pdl_wait();
   extern __shared__ __align__(16) double2 rowc[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = blockIdx.x * kApplyCRows + warp;
@@ -303,7 +307,7 @@ void chol_c(Ctx& c, void* G, int k, int64_t ldg, double shift_factor) {
   IPEPS_CHECK(cholc_smem(k) <= kSmemMaxC, "chol_c: k too large for shared memory");
   g_cholc_attr.ensure(chol_c_kernel, int(kSmemMaxC));
   ProfScope ps(c, KFam::SmallLinalg);
-  chol_c_kernel<<<1, kCholCThreads, cholc_smem(k), c.stream>>>(static_cast<double2*>(G), k, ldg, shift_factor);
+  launch(c.stream, chol_c_kernel, 1, kCholCThreads, cholc_smem(k), static_cast<double2*>(G), k, ldg, shift_factor);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::SmallLinalg, 8.0 * double(k) * k * k / 6.0);
 }
@@ -314,9 +318,8 @@ void trsm_c(Ctx& c, const void* Y, int64_t ldy, int64_t N, int k, const void* R,
   g_trsmc_attr.ensure(trsm_c_kernel, int(kSmemMaxC));
   ProfScope ps(c, KFam::SmallLinalg);
   const unsigned grid = unsigned((N + kTrsmCRows - 1) / kTrsmCRows);
-  trsm_c_kernel<<<grid, kTrsmCRows * 32, trsmc_smem(k), c.stream>>>(static_cast<const double2*>(Y), ldy, N, k,
-                                                                    static_cast<const double2*>(R), ldr,
-                                                                    static_cast<double2*>(Q), ldq);
+  launch(c.stream, trsm_c_kernel, grid, kTrsmCRows * 32, trsmc_smem(k), static_cast<const double2*>(Y), ldy, N, k,
+         static_cast<const double2*>(R), ldr, static_cast<double2*>(Q), ldq);
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::SmallLinalg, 4.0 * double(N) * k * k);
 }
@@ -336,8 +339,8 @@ void jacobi_c_svd(Ctx& c, void* X, int m, int k, int64_t ldx, void* J, int64_t l
   double2* rp = reinterpret_cast<double2*>(rot.data());
   {
     ProfScope ps(c, KFam::Jacobi);
-    jacobi_c_kernel<<<1, 1024, jacc_smem(m, k), c.stream>>>(static_cast<double2*>(X), m, k, ldx, rp, max_sweeps, tol,
-                                                            S, c.d_status, d_sweeps);
+    launch(c.stream, jacobi_c_kernel, 1, 1024, jacc_smem(m, k), static_cast<double2*>(X), m, k, ldx, rp, max_sweeps,
+           tol, S, c.d_status, d_sweeps);
     IPEPS_LAUNCH_CHECK();
     c.count(KFam::Jacobi, 24.0 * double(m) * k * k / 2.0);
   }
@@ -346,7 +349,8 @@ void jacobi_c_svd(Ctx& c, void* X, int m, int k, int64_t ldx, void* J, int64_t l
     const size_t smem = size_t(kApplyCRows) * k * 16;
     g_appc_attr.ensure(jacobi_c_apply_kernel, int(kSmemMaxC));
     const unsigned grid = unsigned((k + kApplyCRows - 1) / kApplyCRows);
-    jacobi_c_apply_kernel<<<grid, kApplyCRows * 32, smem, c.stream>>>(rp, k, d_sweeps, static_cast<double2*>(J), ldj);
+    launch(c.stream, jacobi_c_apply_kernel, grid, kApplyCRows * 32, smem, rp, k, d_sweeps, static_cast<double2*>(J),
+           ldj);
     IPEPS_LAUNCH_CHECK();
     c.count(KFam::Jacobi, 24.0 * double(k) * k * k / 2.0);
   }
