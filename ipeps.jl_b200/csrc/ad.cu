@@ -42,8 +42,10 @@ __global__ void dot_partial_kernel(const double* x, const double* y, int64_t n, 
   }
 }
 
+// out[y] = sum of the n entries of part's row y, one block per row
 __global__ void sum_kernel(const double* part, int n, double* out) {
   pdl_wait();
+  part += int64_t(blockIdx.x) * n;
   double s = 0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += part[i];
   s = wsum(s);
@@ -53,7 +55,7 @@ __global__ void sum_kernel(const double* part, int n, double* out) {
   if (threadIdx.x == 0) {
     double t = 0;
     for (int w = 0; w < int(blockDim.x >> 5); ++w) t += sm[w];
-    *out = t;
+    out[blockIdx.x] = t;
   }
 }
 
@@ -177,23 +179,53 @@ __device__ __forceinline__ double cheb_coef(double si, double eta, double b, int
   return (m == 0 ? 1.0 : 2.0) * (2.0 / b) * re;
 }
 
-// X[:, i] += a_m(i) T[:, i]
-__global__ void cheb_acc_kernel(double* X, const double* T, int64_t N, int n, const double* s, double eta, double b,
-                                int m) {
+// coef[i + m n] = a_m(i) and cmax[m] = max_i |a_m(i)|, block m.  (The transcendental
+// functions of a coefficient cost more than an element's update: one evaluation per
+// column and term, not per element.)
+__global__ void cheb_table_kernel(const double* s, int n, double eta, double b, double* cmax, double* coef) {
   pdl_wait();
-  const int64_t tot = N * n;
-  for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < tot; t += int64_t(gridDim.x) * blockDim.x) {
-    const int i = int(t / N);
-    X[t] = fma(cheb_coef(s[i], eta, b, m), T[t], X[t]);
+  const int m = blockIdx.x;
+  double mx = 0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const double v = cheb_coef(s[i], eta, b, m);
+    coef[i + int64_t(m) * n] = v;
+    mx = fmax(mx, fabs(v));
+  }
+  for (int o = 16; o; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  __shared__ double sm[32];
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < int(blockDim.x >> 5); ++w) mx = fmax(mx, sm[w]);
+    cmax[m] = mx;
   }
 }
 
-__global__ void cheb_coef_max_kernel(const double* s, int n, double eta, double b, int m, double* out) {
+// X = a_0 Y (N x n, coefficients per column)
+__global__ void cheb_start_kernel(const double* Y, int64_t N, const double* coef, double* X) {
   pdl_wait();
-  double mx = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) mx = fmax(mx, fabs(cheb_coef(s[i], eta, b, m)));
-  for (int o = 16; o; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if (threadIdx.x == 0) *out = mx;
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  const int64_t t = i + int64_t(blockIdx.y) * N;
+  X[t] = coef[blockIdx.y] * Y[t];
+}
+
+// One term in one pass: Z = B T_m becomes T_{m+1} = 2 (2/b B T_m - T_m) - T_{m-1}
+// (without P: T_1 = 2/b B T_0 - T_0, and B T_0 is kept in BY), a copy goes to `out` (which
+// may be P) and X += a_{m+1} T_{m+1}.
+__global__ void cheb_step_kernel(double* Z, const double* T, const double* P, double* out, double* X, int64_t N,
+                                 const double* coef, double scale, double* BY) {
+  pdl_wait();
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  const int64_t t = i + int64_t(blockIdx.y) * N;
+  const double z = Z[t];
+  double v = fma(-1.0, T[t], scale * z);
+  if (P) v = fma(-1.0, P[t], 2.0 * v);
+  else BY[t] = z;
+  Z[t] = v;
+  out[t] = v;
+  X[t] = fma(coef[blockIdx.y], v, X[t]);
 }
 
 // Check of X[:, i] = f(s_i^2 - B) Y[:, i] through (x^2 + eta) f(x) = x:
@@ -221,11 +253,28 @@ __global__ void rowsum_kernel(const double* X, int64_t N, int n, double* out) {
   }
 }
 
-// y = alpha * x + beta * y (elementwise over n doubles)
-__global__ void axpby_kernel(double alpha, const double* x, double beta, double* y, int64_t n) {
+// sums of squares of several arrays at once: blocks (x, array), then one block per array
+constexpr int kMaxSums = 9;
+struct SumsArgs {
+  const double* p[kMaxSums];
+  int64_t n[kMaxSums];
+};
+__global__ void sumsq_partial_kernel(SumsArgs a, double* part) {
   pdl_wait();
-  for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += int64_t(gridDim.x) * blockDim.x)
-    y[t] = fma(alpha, x[t], beta * y[t]);
+  const double* x = a.p[blockIdx.y];
+  const int64_t n = a.n[blockIdx.y];
+  double s = 0;
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+    s = fma(x[i], x[i], s);
+  s = wsum(s);
+  __shared__ double sm[32];
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0;
+    for (int w = 0; w < int(blockDim.x >> 5); ++w) t += sm[w];
+    part[blockIdx.x + gridDim.x * blockIdx.y] = t;
+  }
 }
 
 }  // namespace
@@ -233,30 +282,24 @@ __global__ void axpby_kernel(double alpha, const double* x, double beta, double*
 // ------------------------------------------------------------------ helpers
 namespace {
 
-double dot_host(Ctx& c, const Tensor& x, const Tensor& y) {
-  const int64_t n = x.numel();
-  const int blocks = int(std::min<int64_t>((n + 255) / 256, 1024));
-  double* part = static_cast<double*>(c.workspace(size_t(std::max(blocks, 1)) * 8 + 64));
-  double* out = reinterpret_cast<double*>(c.scal->p) + 32;
-  launch(c.stream, dot_partial_kernel, std::max(blocks, 1), 256, 0, x.f64(), y.f64(), n, part);
-  launch(c.stream, sum_kernel, 1, 256, 0, part, std::max(blocks, 1), out);
+// out[k] = sum of the squares of x[k], on the device
+void sumsq_dev(Ctx& c, std::initializer_list<Tensor> xs, double* out) {
+  SumsArgs a{};
+  int na = 0;
+  int64_t longest = 1, total = 0;
+  IPEPS_CHECK(xs.size() <= kMaxSums, "sumsq_dev: too many arrays");
+  for (const Tensor& x : xs) {
+    a.p[na] = x.f64();
+    a.n[na++] = x.numel();
+    longest = std::max(longest, x.numel());
+    total += x.numel();
+  }
+  const int blocks = int(std::min<int64_t>((longest + 255) / 256, 1024));
+  double* part = static_cast<double*>(c.workspace(size_t(blocks) * na * 8 + 64));
+  launch(c.stream, sumsq_partial_kernel, dim3(unsigned(blocks), unsigned(na)), 256, 0, a, part);
+  launch(c.stream, sum_kernel, na, 256, 0, part, blocks, out);
   IPEPS_LAUNCH_CHECK();
-  c.count(KFam::Reduce, 2.0 * n, 16.0 * n);
-  double h = 0;
-  IPEPS_CUDA(cudaMemcpyAsync(&h, out, 8, cudaMemcpyDeviceToHost, c.stream));
-  c.sync();
-  return h;
-}
-
-// *out = sum x*y on the device (stream ordered, no host round trip)
-void dot_dev(Ctx& c, const Tensor& x, const Tensor& y, double* out) {
-  const int64_t n = x.numel();
-  const int blocks = int(std::min<int64_t>((n + 255) / 256, 1024));
-  double* part = static_cast<double*>(c.workspace(size_t(std::max(blocks, 1)) * 8 + 64));
-  launch(c.stream, dot_partial_kernel, std::max(blocks, 1), 256, 0, x.f64(), y.f64(), n, part);
-  launch(c.stream, sum_kernel, 1, 256, 0, part, std::max(blocks, 1), out);
-  IPEPS_LAUNCH_CHECK();
-  c.count(KFam::Reduce, 2.0 * n, 16.0 * n);
+  c.count(KFam::Reduce, 2.0 * total, 8.0 * total);
 }
 
 void colscale(Ctx& c, Tensor& X, const double* s, int ncols, int mode) {
@@ -585,12 +628,10 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
   {
     Tensor Ur = pr.Ur, Vr = pr.Vr;
     const Tensor Yu0 = project_out(c, Ur, dUt), Yv0 = project_out(c, Vr, dVt);
-    double* d_cmax = reinterpret_cast<double*>(c.scal->p) + 40;
     constexpr int kMaxTerms = 160;
     constexpr double kTol = 1e-11;
     constexpr double kCheckTol = 1e-10;
     constexpr int kCheckEvery = 4;
-    const double ny0 = std::sqrt(dot_host(c, Yu0, Yu0) + dot_host(c, Yv0, Yv0));
     Tensor Xu = c.zeros(DType::F64, {N1, n}), Xv = c.zeros(DType::F64, {N2, n});
     // M = R1 R2 formed once (N1 x N2): each application of M M^T or M^T M is
     // then two products instead of four
@@ -612,28 +653,35 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
       gemm(c, DType::F64, 'N', 'T', N1, N2, rr, cplx(-1), C2.data(), N1, Vr.data(), N2, cplx(1), MP.data(), N1,
            true);
     }
-    auto Bu_of = [&](const Tensor& T) { return mm(c, MP, 'N', mm(c, MP, 'T', T, 'N', true), 'N', true); };
-    auto Bv_of = [&](const Tensor& T) { return mm(c, MP, 'T', mm(c, MP, 'N', T, 'N', true), 'N', true); };
+    // b: above the sketch's s_next^2 and a power-iteration estimate of the
+    // top of B (six steps on the sum of the u-side cotangent columns), kept
+    // below the smallest kept s_n^2 so that every resolvent's pole lies outside
+    // [0, b].  All norms come back in one transfer.
+    constexpr int kPower = 6;
+    double h[2 + kPower + 1];
+    {
+      Tensor t = c.alloc(DType::F64, {N1, kPower + 1}), u = c.alloc(DType::F64, {N2}),
+             hd = c.alloc(DType::F64, {2 + kPower + 1});
+      launch(c.stream, rowsum_kernel, gridn(c, N1), 256, 0, Yu0.f64(), N1, n, t.f64());
+      IPEPS_LAUNCH_CHECK();
+      auto col = [&](int j) { return cols(t, j, 1); };
+      for (int it = 0; it < kPower; ++it) {
+        gemm(c, DType::F64, 'T', 'N', N2, 1, N1, cplx(1), MP.data(), N1, col(it).data(), N1, cplx(0), u.data(), N2,
+             true);
+        gemm(c, DType::F64, 'N', 'N', N1, 1, N2, cplx(1), MP.data(), N1, u.data(), N2, cplx(0), col(it + 1).data(),
+             N1, true);
+      }
+      static_assert(kPower == 6 && 2 + kPower + 1 <= kMaxSums);
+      sumsq_dev(c, {Yu0, Yv0, col(0), col(1), col(2), col(3), col(4), col(5), col(6)}, hd.f64());
+      IPEPS_CUDA(cudaMemcpyAsync(h, hd.data(), sizeof(h), cudaMemcpyDeviceToHost, c.stream));
+      c.sync();
+    }
+    const double ny0 = std::sqrt(h[0] + h[1]);
     bool series_done = (ny0 == 0.0);
     if (!series_done) {
-      // b: above the sketch's s_next^2 and a power-iteration estimate of the
-      // top of B (six steps on the sum of the u-side cotangent columns), kept
-      // below the smallest kept s_n^2 so that every resolvent's pole lies outside [0, b]
       const double lam = pr.s_next * pr.s_next, sn2 = pr.sr_host[n - 1] * pr.sr_host[n - 1];
       double est = 0;
-      {
-        Tensor t = c.alloc(DType::F64, {N1, 1});
-        launch(c.stream, rowsum_kernel, gridn(c, N1), 256, 0, Yu0.f64(), N1, n, t.f64());
-        IPEPS_LAUNCH_CHECK();
-        double nt = std::sqrt(dot_host(c, t, t));
-        for (int it = 0; it < 6 && nt > 0; ++it) {
-          Tensor bt = Bu_of(t);
-          const double nb = std::sqrt(dot_host(c, bt, bt));
-          est = nb / nt;
-          t = bt;
-          nt = nb;
-        }
-      }
+      for (int it = 0; it < kPower && h[2 + it] > 0; ++it) est = std::sqrt(h[3 + it]) / std::sqrt(h[2 + it]);
       // b is at least the rounding level of B (~eps s_1^2): below it the
       // recursion would amplify rounding noise.  Kept s_n^2 under that floor
       // are far inside the broadening (f(x) ~ x / eta there, the pole
@@ -649,86 +697,102 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
       // next term (with M_P in place of M).  B~ T = (2/b) B T - T,
       // T_{m+1} = 2 B~ T_m - T_{m-1}.
       Tensor W1 = c.alloc(DType::F64, {N2, 2 * int64_t(n)}), W2 = c.alloc(DType::F64, {N1, 2 * int64_t(n)});
-      Tensor BYu, BYv;
-      auto next_T = [&](Tensor& B, const Tensor& T, const Tensor& Tprev, int m) {
-        launch(c.stream, axpby_kernel, gridn(c, B.numel()), 256, 0, -1.0, T.f64(), 2.0 / b, B.f64(), B.numel());
-        if (m > 0) launch(c.stream, axpby_kernel, gridn(c, B.numel()), 256, 0, -1.0, Tprev.f64(), 2.0, B.f64(),
-                          B.numel());
-        IPEPS_LAUNCH_CHECK();
-      };
-      auto apply_B = [&](const Tensor& Tu, const Tensor& Tv, const Tensor& Pu, const Tensor& Pv, int m, Tensor* Bu,
-                         Tensor* Bv) {
-        IPEPS_CUDA(cudaMemcpyAsync(W2.data(), Tu.data(), size_t(N1) * n * 8, cudaMemcpyDeviceToDevice, c.stream));
+      Tensor BYu = c.alloc(DType::F64, {N1, n}), BYv = c.alloc(DType::F64, {N2, n});
+      // two vectors of the recursion per side (the older one is overwritten by the next)
+      Tensor Ku[2] = {c.alloc(DType::F64, {N1, n}), c.alloc(DType::F64, {N1, n})};
+      Tensor Kv[2] = {c.alloc(DType::F64, {N2, n}), c.alloc(DType::F64, {N2, n})};
+      // sums of squares, cmax per term, coefficients per term and column
+      Tensor tab = c.alloc(DType::F64, {4 + (kMaxTerms + 1) * int64_t(n + 1)});
+      double *d_sums = tab.f64(), *d_cmax = d_sums + 4, *d_coef = d_cmax + kMaxTerms + 1;
+      double sums[4 + kMaxTerms + 1];  // the host's copy of the first two
+      IPEPS_CHECK(n <= 65535, "projector adjoint: too many columns for the grid");
+      const dim3 gu(unsigned((N1 + 255) / 256), unsigned(n)), gv(unsigned((N2 + 255) / 256), unsigned(n));
+      // W1 = M^T W2 and W2 = M W1 (with M_P in place of M)
+      auto down = [&]() {
         gemm(c, DType::F64, 'T', 'N', N2, 2 * n, N1, cplx(1), MP.data(), N1, W2.data(), N1, cplx(0), W1.data(), N2,
              true);
-        // the next v-side vector in place (it feeds the second product), and a copy to keep
-        Tensor zv = cols(W1, n, n);
-        if (m == 0) BYv = clone(c, zv);  // B Y_0 on the v side, for the resolvent check
-        next_T(zv, Tv, Pv, m);
-        *Bv = clone(c, zv);
+      };
+      auto up = [&]() {
         gemm(c, DType::F64, 'N', 'N', N1, 2 * n, N2, cplx(1), MP.data(), N1, W1.data(), N2, cplx(0), W2.data(), N1,
              true);
-        *Bu = clone(c, cols(W2, 0, n));
-        if (m == 0) BYu = clone(c, *Bu);  // B Y_0 on the u side
-        next_T(*Bu, Tu, Pu, m);
       };
-      // relative residual of ((s_i^2 - B)^2 + eta) X_i = (s_i^2 - B) Y_i over all columns of one side
-      auto check = [&](const Tensor& X, const Tensor& Y, const Tensor& BY, bool u_side) {
-        auto B = [&](const Tensor& T) { return u_side ? Bu_of(T) : Bv_of(T); };
-        const Tensor BX = B(X), BBX = B(BX);
-        Tensor res = c.alloc(DType::F64, X.shape()), rhs = c.alloc(DType::F64, X.shape());
-        launch(c.stream, resolvent_check_kernel, gridn(c, X.numel()), 256, 0, X.f64(), BX.f64(), BBX.f64(), Y.f64(),
-               BY.f64(), s.f64(), kSvdEta, X.dims[0], n, res.f64(), rhs.f64());
+      // W2 = [A | M V]
+      auto fill = [&](const Tensor& A, const Tensor& V) {
+        IPEPS_CUDA(cudaMemcpyAsync(W2.data(), A.data(), size_t(N1) * n * 8, cudaMemcpyDeviceToDevice, c.stream));
+        gemm(c, DType::F64, 'N', 'N', N1, n, N2, cplx(1), MP.data(), N1, V.data(), N2, cplx(0),
+             cols(W2, n, n).data(), N1, true);
+      };
+      // the larger of both sides' relative residuals of ((s_i^2 - B)^2 + eta) X_i = (s_i^2 - B) Y_i
+      auto check = [&]() {
+        fill(Xu, Xv);
+        down();  // [M^T Xu | B Xv]
+        Tensor BXv = clone(c, cols(W1, n, n));
+        up();  // [B Xu | M B Xv]
+        Tensor BXu = clone(c, cols(W2, 0, n));
+        down();  // [M^T B Xu | B B Xv]
+        gemm(c, DType::F64, 'N', 'N', N1, n, N2, cplx(1), MP.data(), N1, W1.data(), N2, cplx(0), W2.data(), N1, true);
+        Tensor ru = c.alloc(DType::F64, {N1, n}), qu = c.alloc(DType::F64, {N1, n});
+        Tensor rv = c.alloc(DType::F64, {N2, n}), qv = c.alloc(DType::F64, {N2, n});
+        launch(c.stream, resolvent_check_kernel, gridn(c, N1 * n), 256, 0, Xu.f64(), BXu.f64(), W2.f64(), Yu0.f64(),
+               BYu.f64(), s.f64(), kSvdEta, N1, n, ru.f64(), qu.f64());
+        launch(c.stream, resolvent_check_kernel, gridn(c, N2 * n), 256, 0, Xv.f64(), BXv.f64(),
+               cols(W1, n, n).f64(), Yv0.f64(), BYv.f64(), s.f64(), kSvdEta, N2, n, rv.f64(), qv.f64());
         IPEPS_LAUNCH_CHECK();
-        const double nr = dot_host(c, rhs, rhs);
-        return nr > 0 ? std::sqrt(dot_host(c, res, res) / nr) : 0.0;
+        sumsq_dev(c, {ru, qu, rv, qv}, d_sums);
+        IPEPS_CUDA(cudaMemcpyAsync(sums, d_sums, 4 * 8, cudaMemcpyDeviceToHost, c.stream));
+        c.sync();
+        auto rel = [](double r, double q) { return q > 0 ? std::sqrt(r / q) : 0.0; };
+        const double u = rel(sums[0], sums[1]), v = rel(sums[2], sums[3]);
+        return u <= v || std::isnan(v) ? v : u;
       };
       for (int attempt = 0; attempt < 6; ++attempt) {
-        Xu = c.zeros(DType::F64, {N1, n});
-        Xv = c.zeros(DType::F64, {N2, n});
-        Tensor Pu = Yu0, Pv = Yv0;  // T_{m-1}
+        launch(c.stream, cheb_table_kernel, kMaxTerms + 1, 128, 0, s.f64(), n, kSvdEta, b, d_cmax, d_coef);
+        launch(c.stream, cheb_start_kernel, gu, 256, 0, Yu0.f64(), N1, d_coef, Xu.f64());
+        launch(c.stream, cheb_start_kernel, gv, 256, 0, Yv0.f64(), N2, d_coef, Xv.f64());
+        IPEPS_LAUNCH_CHECK();
         Tensor Tu = Yu0, Tv = Yv0;  // T_m
         bool blew_up = false, converged = false;
-        // M_P T_v of the first term, in the second half of W2
-        gemm(c, DType::F64, 'N', 'N', N1, n, N2, cplx(1), MP.data(), N1, Tv.data(), N2, cplx(0),
-             cols(W2, n, n).data(), N1, true);
+        fill(Tu, Tv);
+        // The stopping tests read the sums of squares back, at some of the terms
+        // kCheckEvery - 1, 2 kCheckEvery - 1, ...: at the first of them, then where the
+        // coefficients' tail has fallen far enough for the |X| seen last.
+        int next = kCheckEvery - 1;
         for (int m = 0; m < kMaxTerms; ++m) {
-          launch(c.stream, cheb_acc_kernel, gridn(c, N1 * n), 256, 0, Xu.f64(), Tu.f64(), N1, n, s.f64(), kSvdEta, b,
-                 m);
-          launch(c.stream, cheb_acc_kernel, gridn(c, N2 * n), 256, 0, Xv.f64(), Tv.f64(), N2, n, s.f64(), kSvdEta, b,
-                 m);
-          IPEPS_LAUNCH_CHECK();
           c.series_terms++;
-          // the stopping tests read back five device scalars every kCheckEvery terms
-          // (one host round trip instead of five per term)
-          if (m % kCheckEvery == kCheckEvery - 1 || m == kMaxTerms - 1) {
-            launch(c.stream, cheb_coef_max_kernel, 1, 32, 0, s.f64(), n, kSvdEta, b, m + 1, d_cmax);
-            IPEPS_LAUNCH_CHECK();
-            dot_dev(c, Tu, Tu, d_cmax + 1);
-            dot_dev(c, Tv, Tv, d_cmax + 2);
-            dot_dev(c, Xu, Xu, d_cmax + 3);
-            dot_dev(c, Xv, Xv, d_cmax + 4);
-            double h[5];
-            IPEPS_CUDA(cudaMemcpyAsync(h, d_cmax, sizeof(h), cudaMemcpyDeviceToHost, c.stream));
+          if (m == next || m == kMaxTerms - 1) {
+            const bool first = m == kCheckEvery - 1;
+            sumsq_dev(c, {Tu, Tv, Xu, Xv}, d_sums);
+            IPEPS_CUDA(cudaMemcpyAsync(sums, d_sums, first ? sizeof(sums) : 4 * 8, cudaMemcpyDeviceToHost, c.stream));
             c.sync();
-            if (std::sqrt(h[1] + h[2]) > 8.0 * ny0) {
+            if (!(std::sqrt(sums[0] + sums[1]) <= 8.0 * ny0)) {
               blew_up = true;  // spectrum beyond b
               break;
             }
             // |T_m| <= |T_0| on [0, b]: the remaining terms are bounded by the coefficient tail
-            if (h[0] * ny0 <= kTol * std::sqrt(h[3] + h[4])) {
+            const double* cmax = sums + 4;
+            const double bound = kTol * std::sqrt(sums[2] + sums[3]);
+            if (cmax[m + 1] * ny0 <= bound) {
               converged = true;
               break;
             }
+            do next += kCheckEvery;
+            while (next < kMaxTerms && cmax[next + 1] * ny0 > bound);
           }
-          Tensor Bu, Bv;
-          apply_B(Tu, Tv, Pu, Pv, m, &Bu, &Bv);
-          Pu = Tu;
-          Pv = Tv;
-          Tu = Bu;
-          Tv = Bv;
+          Tensor &nu = Ku[m & 1], &nv = Kv[m & 1];
+          const double* pu = m > 1 ? nu.f64() : m > 0 ? Yu0.f64() : nullptr;  // T_{m-1}
+          const double* pv = m > 1 ? nv.f64() : m > 0 ? Yv0.f64() : nullptr;
+          const double* coef = d_coef + int64_t(m + 1) * n;
+          down();  // [M^T T_u | B T_v]
+          launch(c.stream, cheb_step_kernel, gv, 256, 0, cols(W1, n, n).f64(), Tv.f64(), pv, nv.f64(), Xv.f64(), N2,
+                 coef, 2.0 / b, BYv.f64());
+          up();  // [B T_u | M T_v']
+          launch(c.stream, cheb_step_kernel, gu, 256, 0, W2.f64(), Tu.f64(), pu, nu.f64(), Xu.f64(), N1, coef,
+                 2.0 / b, BYu.f64());
+          IPEPS_LAUNCH_CHECK();
+          Tu = nu;
+          Tv = nv;
         }
-        if (converged && std::max(check(Xu, Yu0, BYu, true), check(Xv, Yv0, BYv, false)) <= kCheckTol) {
+        if (converged && check() <= kCheckTol) {
           series_done = true;
           break;
         }
