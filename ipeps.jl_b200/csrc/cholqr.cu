@@ -77,52 +77,12 @@ __host__ __device__ __forceinline__ int col_base(int I, int nb) { return I * nb 
 // its time fetching instructions (55 us at k = 160).
 // The contract is that of chol_blocked: shift_factor * trace is added to the
 // diagonal, a pivot at or below 1e-32 trace leaves R[j][j] = 1 and row j zero.
-// CX: G is complex Hermitian of k / 2 columns, taken as the real symmetric matrix of
-// its 2 x 2 blocks [[re, -im], [im, re]].  The factor of that is the same form of the
-// complex factor (the Cholesky factor is unique), so the real kernels do the work.
-template <bool CX>
-__global__ void __launch_bounds__(kCpThreads, 1)
-    chol_panel_kernel(double* G, int k, int64_t ldg, double shift_factor, double2* __restrict__ Rpk, int write_g) {
-  pdl_wait();
-  extern __shared__ __align__(16) double2 S[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int nb = (k + 7) >> 3, nblk = nb * (nb + 1) / 2;
-
-  // G's upper triangle (columns from k on: the identity)
-  {
-    constexpr int U = 7;  // blocks in flight per warp
-    int J = 0, first = 0;
-    for (int b0 = warp; b0 < nblk; b0 += U * kCpWarps) {
-      double2 v[U];
-#pragma unroll
-      for (int q = 0; q < U; ++q) {
-        const int b = b0 + q * kCpWarps;
-        while (J < nb && b >= first + nb - J) {
-          first += nb - J;
-          ++J;
-        }
-        const int I = J + b - first, r = 8 * I + g, c = 8 * J + 2 * t;
-        v[q] = make_double2(r == c ? 1.0 : 0.0, r == c + 1 ? 1.0 : 0.0);
-        if constexpr (CX) {
-          if (b < nblk && r < k && c < k) {
-            const int rr = r >> 1, cc = c >> 1;
-            double2 z = reinterpret_cast<const double2*>(G)[min(rr, cc) + int64_t(max(rr, cc)) * ldg];
-            if (rr > cc) z.y = -z.y;  // the upper triangle is stored
-            if (rr == cc) z.y = 0.0;
-            v[q] = (r & 1) ? make_double2(z.y, z.x) : make_double2(z.x, -z.y);
-          }
-        } else if (b < nblk && r < k) {
-          if (c < k) v[q].x = G[min(r, c) + int64_t(max(r, c)) * ldg];
-          if (c + 1 < k) v[q].y = G[min(r, c + 1) + int64_t(max(r, c + 1)) * ldg];
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < U; ++q)
-        if (b0 + q * kCpWarps < nblk) S[(b0 + q * kCpWarps) * 32 + lane] = v[q];
-    }
-  }
-  __syncthreads();
-
+// In the end S holds the packed R; it is also written to Rpk if that is given, and R's
+// diagonal blocks to G.
+__device__ __forceinline__ void factor_panels(double2* S, int k, double shift_factor, double2* __restrict__ Rpk,
+                                              double* G, int64_t ldg) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nb = (k + 7) >> 3;
   if (warp == 0) {
     double tr = 0;
     for (int i = lane; i < k; i += 32) {
@@ -187,10 +147,10 @@ __global__ void __launch_bounds__(kCpThreads, 1)
         *N = n;
         __syncwarp();
         bar_post<1, 32 + kUpdateThreads>();
-        Rpk[(col_base(p, nb) + 1) * 32 + lane] = make_double2(x0, x1);
+        if (Rpk) Rpk[(col_base(p, nb) + 1) * 32 + lane] = make_double2(x0, x1);
       }
-      Rpk[col_base(p, nb) * 32 + lane] = q;
-      if (write_g && lane < 8) {
+      if (Rpk) Rpk[col_base(p, nb) * 32 + lane] = q;
+      if (G && lane < 8) {
 #pragma unroll
         for (int c = 0; c < 8; ++c)
           if (c == me && 8 * p + c < k) {
@@ -211,7 +171,7 @@ __global__ void __launch_bounds__(kCpThreads, 1)
         dmma8(x0, x1, c.x, q.x);
         dmma8(x0, x1, c.y, q.y);
         L[32 * I] = make_double2(x0, x1);
-        Rpk[(col_base(p, nb) + I - p) * 32 + lane] = make_double2(x0, x1);
+        if (Rpk) Rpk[(col_base(p, nb) + I - p) * 32 + lane] = make_double2(x0, x1);
       }
       bar_wait<3, kUpdateThreads>();
       // the blocks right of the panel in 2 x 2 groups of rows I, I + 1 and columns J, J + 1
@@ -262,6 +222,55 @@ __global__ void __launch_bounds__(kCpThreads, 1)
       }
     }
   }
+}
+
+// CX: G is complex Hermitian of k / 2 columns, taken as the real symmetric matrix of
+// its 2 x 2 blocks [[re, -im], [im, re]].  The factor of that is the same form of the
+// complex factor (the Cholesky factor is unique), so the real kernels do the work.
+template <bool CX>
+__global__ void __launch_bounds__(kCpThreads, 1)
+    chol_panel_kernel(double* G, int k, int64_t ldg, double shift_factor, double2* __restrict__ Rpk, int write_g) {
+  pdl_wait();
+  extern __shared__ __align__(16) double2 S[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int nb = (k + 7) >> 3, nblk = nb * (nb + 1) / 2;
+
+  // G's upper triangle (columns from k on: the identity)
+  {
+    constexpr int U = 7;  // blocks in flight per warp
+    int J = 0, first = 0;
+    for (int b0 = warp; b0 < nblk; b0 += U * kCpWarps) {
+      double2 v[U];
+#pragma unroll
+      for (int q = 0; q < U; ++q) {
+        const int b = b0 + q * kCpWarps;
+        while (J < nb && b >= first + nb - J) {
+          first += nb - J;
+          ++J;
+        }
+        const int I = J + b - first, r = 8 * I + g, c = 8 * J + 2 * t;
+        v[q] = make_double2(r == c ? 1.0 : 0.0, r == c + 1 ? 1.0 : 0.0);
+        if constexpr (CX) {
+          if (b < nblk && r < k && c < k) {
+            const int rr = r >> 1, cc = c >> 1;
+            double2 z = reinterpret_cast<const double2*>(G)[min(rr, cc) + int64_t(max(rr, cc)) * ldg];
+            if (rr > cc) z.y = -z.y;  // the upper triangle is stored
+            if (rr == cc) z.y = 0.0;
+            v[q] = (r & 1) ? make_double2(z.y, z.x) : make_double2(z.x, -z.y);
+          }
+        } else if (b < nblk && r < k) {
+          if (c < k) v[q].x = G[min(r, c) + int64_t(max(r, c)) * ldg];
+          if (c + 1 < k) v[q].y = G[min(r, c + 1) + int64_t(max(r, c + 1)) * ldg];
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < U; ++q)
+        if (b0 + q * kCpWarps < nblk) S[(b0 + q * kCpWarps) * 32 + lane] = v[q];
+    }
+  }
+  __syncthreads();
+
+  factor_panels(S, k, shift_factor, Rpk, write_g ? G : nullptr, ldg);
   if (write_g) {
     // R's rows right of the diagonal blocks, and zeros below the diagonal
     __syncthreads();
@@ -276,13 +285,41 @@ __global__ void __launch_bounds__(kCpThreads, 1)
   }
 }
 
-// Q = Y R^-1: x R = y for eight rows per warp, held as NB accumulator blocks, the
-// current block column in a[0] (the array moves down by one block per step, so the
-// loop's code stays small: executed once, an unrolled one waits for its own
-// instructions).  X_J = T_J R_JJ^-1 with the inverse from R's diagonal block, then
-// X_J times R's block row J is subtracted from the columns after it.  An
-// accumulator block is an A operand as it stands: lane (g, t) holds the columns
-// 2t and 2t + 1.  The CTA's warps beyond those with rows only help to stage R.
+// x R = y for eight rows per warp, held as NB accumulator blocks, the current block
+// column in a[0] (the array moves down by one block per step, so the loop's code stays
+// small: executed once, an unrolled one waits for its own instructions).  X_J = T_J
+// R_JJ^-1 with the inverse from R's diagonal block, then X_J times R's block row J is
+// subtracted from the columns after it.  An accumulator block is an A operand as it
+// stands: lane (g, t) holds the columns 2t and 2t + 1.  R: the packed factor at the
+// lane's offset; three blocks after its end are read.
+template <int NB, class Store>
+__device__ __forceinline__ void solve_rows(double (&a)[NB][2], const double2* R, int nb, Store store) {
+  for (int J = 0; J < nb; ++J) {
+    const double2 b = R[0];
+    double x0 = 0.0, x1 = 0.0;
+    dmma8(x0, x1, a[0][0], b.x);
+    dmma8(x0, x1, a[0][1], b.y);
+    store(J, x0, x1);
+    const double m0 = -x0, m1 = -x1;
+    // four blocks at a time, as far as there are any (a group may run over the end of
+    // the block row: what it computes there is not used)
+#pragma unroll
+    for (int K0 = 1; K0 < NB; K0 += 4)
+      if (J + K0 < nb) {
+        double2 q[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) q[i] = R[(K0 + i) * 32];
+#pragma unroll
+        for (int i = 0; i < 4 && K0 + i < NB; ++i)
+          dmma8(a[K0 + i - 1][0], a[K0 + i - 1][1], m0, q[i].x, a[K0 + i][0], a[K0 + i][1]);
+#pragma unroll
+        for (int i = 0; i < 4 && K0 + i < NB; ++i) dmma8(a[K0 + i - 1][0], a[K0 + i - 1][1], m1, q[i].y);
+      }
+    R += (nb - J) * 32;
+  }
+}
+
+// Q = Y R^-1.  The CTA's warps beyond those with rows only help to stage R.
 constexpr int kTpThreads = 256;
 
 // CX: complex Y and Q of k / 2 columns; a row enters as (re, -im) pairs, the first row
@@ -318,12 +355,7 @@ __global__ void __launch_bounds__(kTpThreads) trsm_panel_kernel(const double* __
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
   __syncthreads();
   if (warp >= warps) return;
-  const double2* R = Rs + lane;
-  for (int J = 0; J < nb; ++J) {
-    const double2 b = R[0];
-    double x0 = 0.0, x1 = 0.0;
-    dmma8(x0, x1, a[0][0], b.x);
-    dmma8(x0, x1, a[0][1], b.y);
+  solve_rows<NB>(a, Rs + lane, nb, [&](int J, double x0, double x1) {
     const int c = 8 * J + 2 * t;
     if constexpr (CX) {
       if (mine && c < k) reinterpret_cast<double2*>(Q)[row + int64_t(c >> 1) * ldq] = make_double2(x0, -x1);
@@ -331,22 +363,157 @@ __global__ void __launch_bounds__(kTpThreads) trsm_panel_kernel(const double* __
       if (mine && c < k) Q[row + int64_t(c) * ldq] = x0;
       if (mine && c + 1 < k) Q[row + int64_t(c + 1) * ldq] = x1;
     }
-    const double m0 = -x0, m1 = -x1;
-    // four blocks at a time, as far as there are any (a group may run over the end of
-    // the block row: what it computes there is not used)
-#pragma unroll
-    for (int K0 = 1; K0 < NB; K0 += 4)
-      if (J + K0 < nb) {
-        double2 q[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) q[i] = R[(K0 + i) * 32];
-#pragma unroll
-        for (int i = 0; i < 4 && K0 + i < NB; ++i)
-          dmma8(a[K0 + i - 1][0], a[K0 + i - 1][1], m0, q[i].x, a[K0 + i][0], a[K0 + i][1]);
-#pragma unroll
-        for (int i = 0; i < 4 && K0 + i < NB; ++i) dmma8(a[K0 + i - 1][0], a[K0 + i - 1][1], m1, q[i].y);
+  });
+}
+
+// All passes of one orthonormalisation in one launch of one CTA: the Gram product (one
+// warp per strip of a block and the one below it), the factor and the solve, in shared
+// memory.  The separate kernels of a pass are three launches of 5 to 10 us, most of
+// it the way to global memory and back.  Gradient at D = 2, chi = 16 71.4 -> 65.4 ms
+// (64 rows), chi = 30 75.6 -> 70.9 ms (120 rows); complex energy at chi = 8 24.8 -> 21.1
+// ms (32 rows), chi = 14 25.6 -> 22.6 ms.
+// The columns from k to 8 nb are zero (G: the identity).  CX: complex rows enter the
+// Gram product as both rows of their 2 x 2 blocks.
+// smem: R, then Y row by row, ld = 8 nb + 4 (the fragments' reads then meet no bank conflict).
+__host__ __device__ __forceinline__ int orth_ld(int nb) { return 8 * nb + 4; }
+
+struct OrthArgs {
+  const double* Y;
+  double* Q;
+  double2* Rpk;  // packed R per pass, or null
+  int64_t N, ldy, ldq;
+  int k, rows, passes;  // rows: N rounded up to a multiple of 8
+  double shift;         // first pass
+};
+
+template <int NB, bool CX>
+__global__ void __launch_bounds__(kCpThreads, 1) orth_kernel(OrthArgs o) {
+  pdl_wait();
+  extern __shared__ __align__(16) double2 S[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int k = o.k, nb = (k + 7) >> 3, nblk = nb * (nb + 1) / 2, ld = orth_ld(nb);
+  double* Ys = reinterpret_cast<double*>(S + (nblk + 3) * 32);  // (the solve reads three blocks past R)
+  const int groups = o.rows >> 3, steps = o.rows / 4 * (CX ? 2 : 1);
+
+  // rows from global memory, a warp 8 rows of 4 columns at a time (complex: 16 of 2)
+  {
+    constexpr int CPW = CX ? 2 : 4;
+    const int cols = CX ? k / 2 : k, wide = CX ? 4 * nb : 8 * nb;
+    constexpr int RPW = 32 / CPW;
+    const int cc = lane % CPW, rr = lane / CPW;
+    const int cg_ = (wide + CPW - 1) / CPW, rg = (o.rows + RPW - 1) / RPW;
+    for (int u = warp; u < cg_ * rg; u += kCpWarps) {
+      const int c = (u / rg) * CPW + cc, r = (u % rg) * RPW + rr;
+      if (r >= o.rows || c >= wide) continue;
+      const bool in = r < o.N && c < cols;
+      if constexpr (CX) {
+        double2 z = make_double2(0.0, 0.0);
+        if (in) z = reinterpret_cast<const double2*>(o.Y)[r + int64_t(c) * o.ldy];
+        *reinterpret_cast<double2*>(Ys + (2 * r) * ld + 2 * c) = make_double2(z.x, -z.y);
+        *reinterpret_cast<double2*>(Ys + (2 * r + 1) * ld + 2 * c) = make_double2(z.y, z.x);
+      } else {
+        Ys[r * ld + c] = in ? o.Y[r + int64_t(c) * o.ldy] : 0.0;
       }
-    R += (nb - J) * 32;
+    }
+  }
+  __syncthreads();
+
+  for (int pass = 0; pass < o.passes; ++pass) {
+    // the Gram product's lower blocks (I, J), (I + 1, J) for strips of two block rows
+    int J = 0, first = 0;
+    for (int u = warp;; u += kCpWarps) {
+      while (J < nb && u - first >= (nb - J + 1) / 2) {
+        first += (nb - J + 1) / 2;
+        ++J;
+      }
+      if (J >= nb) break;
+      const int I = J + 2 * (u - first);
+      const bool two = I + 1 < nb;
+      const double *yi = Ys + t * ld + 8 * I + g, *yj = Ys + t * ld + 8 * J + g, *yk = two ? yi + 8 : yi;
+      double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll 4
+      for (int q = 0; q < steps; ++q) {
+        const double b = yj[q * 4 * ld];
+        dmma8(c[0][0], c[0][1], yi[q * 4 * ld], b);
+        dmma8(c[1][0], c[1][1], yk[q * 4 * ld], b);
+      }
+      if (I == J) {  // columns from k on
+        const int r = 8 * I + g, cc = 8 * J + 2 * t;
+        if (r >= k && r == cc) c[0][0] = 1.0;
+        if (r >= k && r == cc + 1) c[0][1] = 1.0;
+      }
+      double2* d = S + (col_base(J, nb) + I - J) * 32 + lane;
+      d[0] = make_double2(c[0][0], c[0][1]);
+      if (two) d[32] = make_double2(c[1][0], c[1][1]);
+    }
+    __syncthreads();
+    factor_panels(S, k, pass == 0 ? o.shift : 0.0, o.Rpk ? o.Rpk + int64_t(pass) * nblk * 32 : nullptr,
+                  nullptr, 0);
+    __syncthreads();
+    const bool last = pass + 1 == o.passes;
+    for (int w = warp; w < groups; w += kCpWarps) {
+      double* y = Ys + (CX ? 2 : 1) * (w * 8 + g) * ld + 2 * t;  // this lane's row
+      double a[NB][2];
+#pragma unroll
+      for (int j = 0; j < NB; ++j) {
+        const double2 v = j < nb ? *reinterpret_cast<const double2*>(y + 8 * j) : make_double2(0.0, 0.0);
+        a[j][0] = v.x;
+        a[j][1] = v.y;
+      }
+      const int64_t row = w * 8 + g;
+      const bool mine = row < o.N;
+      solve_rows<NB>(a, S + lane, nb, [&](int j, double x0, double x1) {
+        const int c = 8 * j + 2 * t;
+        if (!last) {
+          *reinterpret_cast<double2*>(y + 8 * j) = make_double2(x0, x1);
+          if constexpr (CX) *reinterpret_cast<double2*>(y + ld + 8 * j) = make_double2(-x1, x0);
+        } else if constexpr (CX) {
+          if (mine && c < k) reinterpret_cast<double2*>(o.Q)[row + int64_t(c >> 1) * o.ldq] = make_double2(x0, -x1);
+        } else {
+          if (mine && c < k) o.Q[row + int64_t(c) * o.ldq] = x0;
+          if (mine && c + 1 < k) o.Q[row + int64_t(c + 1) * o.ldq] = x1;
+        }
+      });
+    }
+    __syncthreads();
+  }
+}
+
+constexpr size_t kOrthSmem = 226 * 1024;
+
+int orth_rows(int64_t N) { return int((N + 7) / 8 * 8); }
+size_t orth_smem(int k, int64_t N, bool cx) {
+  const int nb = (k + 7) / 8, nblk = nb * (nb + 1) / 2;
+  return size_t(nblk + 3) * 512 + size_t(orth_rows(N)) * (cx ? 2 : 1) * orth_ld(nb) * 8;
+}
+
+// Up to 128 rows (64 complex ones, 128 in shared memory).  Gradient with one CTA's kernel
+// up to 0 / 128 / 400 rows, ms: 120 rows 75.6 / 70.9 / 71.0, 200 rows 92.4 / 91.5 / 102.7,
+// 252 rows 84.9 / 83.1 / 85.8: beyond that the Gram product and the solve take longer on
+// one SM than they save.  Clusters of 2 to 8 CTAs with the sum through distributed
+// shared memory gave nothing at 333 and 1024 rows and lost 8% at 432.
+constexpr int kOrthMaxRows = 128;
+
+// k real columns
+bool fits_one(int64_t N, int k, bool cx) {
+  return N >= 1 && k >= 1 && N * (cx ? 2 : 1) <= kOrthMaxRows && k <= kOrthMaxK && orth_smem(k, N, cx) <= kOrthSmem;
+}
+
+template <int NB, bool CX>
+void launch_orth(Ctx& c, const OrthArgs& o) {
+  static SmemAttrOnce attr;
+  attr.ensure(orth_kernel<NB, CX>, int(kOrthSmem));
+  launch(c.stream, orth_kernel<NB, CX>, 1, kCpThreads, orth_smem(o.k, o.N, CX), o);
+  IPEPS_LAUNCH_CHECK();
+}
+
+template <bool CX>
+void orth_by_width(Ctx& c, const OrthArgs& o) {
+  switch ((o.k + 31) / 32) {
+    case 1: launch_orth<4, CX>(c, o); break;
+    case 2: launch_orth<8, CX>(c, o); break;
+    case 3: launch_orth<12, CX>(c, o); break;
+    default: launch_orth<16, CX>(c, o); break;
   }
 }
 
@@ -421,6 +588,25 @@ void trsm_packed_c(Ctx& c, const void* Y, int64_t ldy, int64_t N, int k, const d
   ProfScope ps(c, KFam::SmallLinalg);
   trsm_by_width<true>(c, static_cast<const double*>(Y), ldy, N, 2 * k, Rpk, static_cast<double*>(Q), ldq);
   c.count(KFam::SmallLinalg, 4.0 * double(N) * k * k);
+}
+
+bool orth_fits(int64_t N, int k) { return fits_one(N, k, false); }
+bool orth_fits_c(int64_t N, int k) { return fits_one(N, 2 * k, true); }
+
+void orth_small(Ctx& c, const double* Y, int64_t N, int k, int passes, double shift_factor, double* Rpk, double* Q) {
+  IPEPS_CHECK(orth_fits(N, k) && passes > 0, "orth_small: size out of range");
+  ProfScope ps(c, KFam::SmallLinalg);
+  orth_by_width<false>(c, OrthArgs{Y, Q, reinterpret_cast<double2*>(Rpk), N, N, N, k, orth_rows(N), passes, shift_factor});
+  c.count(KFam::SmallLinalg, passes * (2.0 * N * k * k + double(k) * k * k / 3.0));
+}
+
+// (the real form of G has twice its trace: half the shift factor is the same shift)
+void orth_small_c(Ctx& c, const void* Y, int64_t N, int k, int passes, double shift_factor, void* Q) {
+  IPEPS_CHECK(orth_fits_c(N, k) && passes > 0, "orth_small_c: size out of range");
+  ProfScope ps(c, KFam::SmallLinalg);
+  orth_by_width<true>(c, OrthArgs{static_cast<const double*>(Y), static_cast<double*>(Q), nullptr, N, N, N, 2 * k,
+                                  orth_rows(N), passes, 0.5 * shift_factor});
+  c.count(KFam::SmallLinalg, passes * (8.0 * N * k * k + 8.0 * double(k) * k * k / 6.0));
 }
 
 }  // namespace ipeps

@@ -53,6 +53,13 @@ void trsm_packed(Ctx& c, const double* Y, int64_t ldy, int64_t N, int k, const d
 // 2k x 2k factor (cholqr_packed(2 k) doubles)
 void chol_packed_c(Ctx& c, const void* G, int k, int64_t ldg, double shift_factor, double* Rpk);
 void trsm_packed_c(Ctx& c, const void* Y, int64_t ldy, int64_t N, int k, const double* Rpk, void* Q, int64_t ldq);
+// All passes of CholeskyQR on a small N x k matrix in one kernel; Rpk (or null): the packed R of each pass, one after
+// another.  Q may be Y.  _c: complex of k columns.
+constexpr int kOrthMaxK = 128;
+bool orth_fits(int64_t N, int k);
+bool orth_fits_c(int64_t N, int k);
+void orth_small(Ctx& c, const double* Y, int64_t N, int k, int passes, double shift_factor, double* Rpk, double* Q);
+void orth_small_c(Ctx& c, const void* Y, int64_t N, int k, int passes, double shift_factor, void* Q);
 // jacobi_svd with X held in shared memory and J formed from the logged
 // rotations when it fits; tol <= 0 means m * eps
 void jacobi_svd_auto(Ctx& c, double* X, int m, int k, int64_t ldx, double* J, int64_t ldj, double* S,

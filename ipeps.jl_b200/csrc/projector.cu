@@ -104,12 +104,27 @@ Tensor apply_left_T(Ctx& c, const Tensor& X, const MatRef& R, char op) {
 Tensor orth(Ctx& c, const Tensor& Y0, int passes, Tensor* Rout, std::vector<Tensor>* factors) {
   const int64_t N = Y0.dims[0];
   const int k = int(Y0.dims[1]);
+  const double u = 1.1102230246251565e-16;
+  // shifted CholeskyQR: the first pass adds 11 (N k + k (k+1)) u trace(G) to the diagonal
+  const double sf0 = 11.0 * (double(N) * k + double(k) * (k + 1)) * u;
+  if (!Rout && orth_fits(N, k)) {
+    const int64_t np = cholqr_packed(k);
+    Tensor R = factors ? c.alloc(DType::F64, {np * passes}) : Tensor();
+    Tensor Q = c.alloc(DType::F64, {N, k});
+    orth_small(c, Y0.f64(), N, k, passes, sf0, factors ? R.f64() : nullptr, Q.f64());
+    for (int p = 0; factors && p < passes; ++p) {
+      Tensor v = R;
+      v.offset += size_t(p) * np * 8;
+      v.dims[0] = np;
+      factors->push_back(v);
+    }
+    return Q;
+  }
   Tensor Y = Y0;
   Tensor G = c.alloc(DType::F64, {k, k});
   Tensor Ri = c.alloc(DType::F64, {k, k});
   Tensor Racc;
   double* d_tr = reinterpret_cast<double*>(c.scal->p) + 8;
-  const double u = 1.1102230246251565e-16;
   const bool packed = cholqr_fits(k), blocked = !packed && chol_fits(k) && trsm_fits(k);
   Tensor Rrow = packed    ? c.alloc(DType::F64, {cholqr_packed(k)})
                 : blocked ? c.alloc(DType::F64, {int64_t(k) * (k + 1) / 2})
@@ -118,8 +133,7 @@ Tensor orth(Ctx& c, const Tensor& Y0, int passes, Tensor* Rout, std::vector<Tens
     // G = Y^T Y  (FP64 always: the Gram matrix is where precision is lost), its upper triangle: all
     // that the Cholesky kernels read
     gemm_f64_dmma(c, 'T', 'N', k, k, N, 1.0, Y.f64(), N, Y.f64(), N, 0.0, G.f64(), k, true);
-    // shifted CholeskyQR: the first pass adds 11 (N k + k (k+1)) u trace(G) to the diagonal
-    const double sf = (pass == 0) ? 11.0 * (double(N) * k + double(k) * (k + 1)) * u : 0.0;
+    const double sf = (pass == 0) ? sf0 : 0.0;
     Tensor Yn = c.alloc(DType::F64, {N, k});
     if (packed) {
       if (factors && pass > 0) Rrow = c.alloc(DType::F64, {cholqr_packed(k)});
@@ -260,14 +274,20 @@ Tensor cmm(Ctx& c, char oa, char ob, int64_t m, int64_t n, int64_t k, const Tens
 Tensor orth_c(Ctx& c, const Tensor& Y0, int passes) {
   const int64_t N = Y0.dims[0];
   const int k = int(Y0.dims[1]);
+  const double u = 1.1102230246251565e-16;
+  const double sf0 = 11.0 * (double(N) * k + double(k) * (k + 1)) * u;
+  if (orth_fits_c(N, k)) {
+    Tensor Q = c.alloc(DType::C128, {N, k});
+    orth_small_c(c, Y0.data(), N, k, passes, sf0, Q.data());
+    return Q;
+  }
   Tensor Y = Y0;
   Tensor G = c.alloc(DType::C128, {k, k});
-  const double u = 1.1102230246251565e-16;
   const bool packed = cholqr_fits(2 * k);
   Tensor Rpk = packed ? c.alloc(DType::F64, {cholqr_packed(2 * k)}) : Tensor();
   for (int pass = 0; pass < passes; ++pass) {
     gemm(c, DType::C128, 'C', 'N', k, k, N, cplx(1), Y.data(), N, Y.data(), N, cplx(0), G.data(), k, true);
-    const double sf = (pass == 0) ? 11.0 * (double(N) * k + double(k) * (k + 1)) * u : 0.0;
+    const double sf = (pass == 0) ? sf0 : 0.0;
     Tensor Yn = c.alloc(DType::C128, {N, k});
     if (packed) {
       chol_packed_c(c, G.data(), k, k, sf, Rpk.f64());

@@ -112,3 +112,24 @@ def test_projector_rank_deficient_corners(engine, pkg, n, rank):
         P1, P2, s = pkg.get_projector(R1, R2, rank, engine=engine)
         assert np.isfinite(P1).all() and np.isfinite(P2).all()
         assert np.abs(s[:rank] / scale ** 2 - s_ref[:rank]).max() <= 20 * n * np.finfo(float).eps * s_ref[0]
+
+
+# one launch for all passes (no R asked for): one column, ragged rows and columns, the largest, and the first
+# sizes beyond it
+@pytest.mark.parametrize("N,k", [(1, 1), (8, 8), (13, 13), (64, 31), (120, 41), (127, 97), (128, 128), (129, 9),
+                                 (333, 62)])
+def test_orth_in_one_launch(engine, pkg, N, k):
+    rng = np.random.default_rng(3 * N + k)
+    Y = np.asfortranarray(rng.standard_normal((N, k)))
+    Qn, Rn = np.linalg.qr(Y)
+    Qn = Qn * np.sign(np.diag(Rn))
+    # a backward-stable Q moves by rounding times the condition number of Y
+    cond = np.linalg.cond(Y)
+    for passes, bar in ((1, 1e-6), (2, 1e-14 * k ** 0.5), (3, 1e-14 * k ** 0.5)):
+        Q = np.empty((N, k), order="F")
+        engine.check(engine.lib.ipeps_orth(engine.h, pkg.host._dp(Y), N, k, passes, pkg.host._dp(Q), None))
+        if N > 2 * k:  # (a square Gaussian's condition number is unbounded: the shift then shows)
+            assert np.abs(Q.T @ Q - np.eye(k)).max() <= bar, passes
+        if passes == 3:
+            assert np.abs(Q.T @ Q - np.eye(k)).max() <= 1e-14 * k ** 0.5
+            assert np.linalg.norm(Q - Qn) <= 1e-14 * cond * k
