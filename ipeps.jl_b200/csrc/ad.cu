@@ -631,7 +631,7 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
     constexpr int kMaxTerms = 160;
     constexpr double kTol = 1e-11;
     constexpr double kCheckTol = 1e-10;
-    constexpr int kCheckEvery = 4;
+    constexpr int kFirstCheck = 3;
     Tensor Xu = c.zeros(DType::F64, {N1, n}), Xv = c.zeros(DType::F64, {N2, n});
     // M = R1 R2 formed once (N1 x N2): each application of M M^T or M^T M is
     // then two products instead of four
@@ -753,14 +753,14 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
         Tensor Tu = Yu0, Tv = Yv0;  // T_m
         bool blew_up = false, converged = false;
         fill(Tu, Tv);
-        // The stopping tests read the sums of squares back, at some of the terms
-        // kCheckEvery - 1, 2 kCheckEvery - 1, ...: at the first of them, then where the
-        // coefficients' tail has fallen far enough for the |X| seen last.
-        int next = kCheckEvery - 1;
+        // The stopping tests read the sums of squares back (a round trip to the host): at
+        // term kFirstCheck, then where the coefficients' tail has fallen far enough for the
+        // |X| seen last.
+        int next = kFirstCheck;
         for (int m = 0; m < kMaxTerms; ++m) {
           c.series_terms++;
           if (m == next || m == kMaxTerms - 1) {
-            const bool first = m == kCheckEvery - 1;
+            const bool first = m == kFirstCheck;
             sumsq_dev(c, {Tu, Tv, Xu, Xv}, d_sums);
             IPEPS_CUDA(cudaMemcpyAsync(sums, d_sums, first ? sizeof(sums) : 4 * 8, cudaMemcpyDeviceToHost, c.stream));
             c.sync();
@@ -775,7 +775,7 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
               converged = true;
               break;
             }
-            do next += kCheckEvery;
+            do ++next;
             while (next < kMaxTerms && cmax[next + 1] * ny0 > bound);
           }
           Tensor &nu = Ku[m & 1], &nv = Kv[m & 1];
