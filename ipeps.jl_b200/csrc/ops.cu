@@ -2,6 +2,7 @@
 // shared-memory tile when the fastest index moves), max-abs reduction,
 // scaling, axpy, conj, RNG, and the context / allocator plumbing.
 #include "ctx.cuh"
+#include "fastdiv.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -116,26 +117,41 @@ void* Ctx::workspace(size_t bytes) {
 // ------------------------------------------------------------------ permute
 namespace {
 
+// An element, row or tile index is taken apart with one division per dim.  SMALL: all
+// counts are below 2^31 and the divisions are multiplications (FastDiv); a 64-bit
+// division is about twenty times the instructions, and in short rows and in tiles they
+// were most of the work.  Divisions -> multiplications, us: tiles at 100 x 25 x 100 x 25
+// (100 MB moved) 34.0 -> 23.8, 2500 x 2500 23.8 -> 15.5 (6.4 TB/s); rows of 100 elements
+// 21.9 -> 21.0 (4.8 TB/s), of 25 68.8 -> 45.
 struct PermArgs {
   int nd;
   int64_t odims[kMaxDims];    // output dims
+  FastDiv fdims[kMaxDims];    // (SMALL)
   int64_t istride[kMaxDims];  // input stride of output dim i
 };
 
-template <typename T>
+template <typename T, bool SMALL>
 __global__ void permute_simple(PermArgs a, int64_t total, const T* __restrict__ in, T* __restrict__ out) {
   pdl_wait();
-  for (int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-       idx += int64_t(gridDim.x) * blockDim.x) {
-    int64_t r = idx, off = 0;
+  const int64_t step = int64_t(gridDim.x) * blockDim.x;
+  for (int64_t i0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i0 < total; i0 += 4 * step) {
+    T v[4];
 #pragma unroll
-    for (int i = 0; i < kMaxDims; ++i) {
-      if (i >= a.nd) break;
-      int64_t q = r / a.odims[i];
-      off += (r - q * a.odims[i]) * a.istride[i];
-      r = q;
+    for (int j = 0; j < 4; ++j) {  // four loads in flight
+      if (i0 + j * step >= total) break;
+      int64_t r = i0 + j * step, off = 0;
+#pragma unroll
+      for (int i = 0; i < kMaxDims; ++i) {
+        if (i >= a.nd) break;
+        const int64_t q = SMALL ? int64_t(a.fdims[i].div(uint32_t(r))) : r / a.odims[i];
+        off += (r - q * a.odims[i]) * a.istride[i];
+        r = q;
+      }
+      v[j] = in[off];
     }
-    out[idx] = in[off];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i0 + j * step < total) out[i0 + j * step] = v[j];
   }
 }
 
@@ -147,6 +163,7 @@ struct RowArgs {
   int nd;                     // output dims after the first
   int64_t n0;                 // row length (extent of the shared first dim)
   int64_t odims[kMaxDims];    // output dims 1.. (innermost first)
+  FastDiv fdims[kMaxDims], fchunk;  // (SMALL)
   int64_t istride[kMaxDims];  // their input strides
 };
 
@@ -154,11 +171,13 @@ struct RowArgs {
 // row, so that a few very long rows still spread over the whole GPU and many
 // short rows take one warp each.
 constexpr int64_t kPermChunk = 2048;
+// Rows from here on, in at least eight units per SM, else element by element with four
+// loads in flight (permute_simple), by rows -> by elements, us: 25-element rows (25 x 100
+// x 25 x 100) 45 -> 26.4, 40 x 4 x 40 x 4 3.9 -> 3.6, 64 x 100 x 100 x 5 10.7 -> 14.5, 100 x 25
+// x 100 x 25 21.0 -> 26.5; few long rows (4099 x 3 x 5, 45 units) 12.5 -> 3.5, 1000 x 25 x 25
+// 5.8 -> 4.8.
+constexpr int64_t kRowMin = 64;
 
-// SMALL: the unit count and every output dim fit in 32 bits, so the row
-// index is decomposed with 32-bit divisions (a 64-bit division is several
-// times the instructions, and the decomposition is most of the work of a
-// short row).
 template <typename T, bool SMALL>
 __global__ void permute_rows(RowArgs a, int64_t rows, int64_t nchunk, const T* __restrict__ in, T* __restrict__ out) {
   pdl_wait();
@@ -168,14 +187,12 @@ __global__ void permute_rows(RowArgs a, int64_t rows, int64_t nchunk, const T* _
   for (int64_t u = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; u < units; u += nwarps) {
     int64_t r, c0, off = 0;
     if constexpr (SMALL) {
-      const uint32_t uu = uint32_t(u), nc = uint32_t(nchunk);
-      uint32_t q = uu / nc;
+      uint32_t q = a.fchunk.div(uint32_t(u));
       r = q;
-      c0 = int64_t(uu - q * nc) * kPermChunk;
+      c0 = int64_t(uint32_t(u) - q * a.fchunk.d) * kPermChunk;
       for (int i = 0; i < a.nd; ++i) {
-        const uint32_t od = uint32_t(a.odims[i]);
-        const uint32_t t = q / od;
-        off += int64_t(q - t * od) * a.istride[i];
+        const uint32_t t = a.fdims[i].div(q);
+        off += int64_t(q - t * a.fdims[i].d) * a.istride[i];
         q = t;
       }
     } else {
@@ -212,12 +229,13 @@ struct TileArgs {
   int64_t out_p_stride;  // output stride of input dim 0
   int nrest;
   int64_t rdims[kMaxDims];
+  FastDiv fdims[kMaxDims];  // (SMALL)
   int64_t rin[kMaxDims];
   int64_t rout[kMaxDims];
   int64_t rest_total;
 };
 
-template <typename T>
+template <typename T, bool SMALL>
 __global__ void permute_tiled(TileArgs a, const T* __restrict__ in, T* __restrict__ out) {
   pdl_wait();
   __shared__ T tile[32][33];
@@ -226,17 +244,22 @@ __global__ void permute_tiled(TileArgs a, const T* __restrict__ in, T* __restric
   for (int64_t rest = blockIdx.z; rest < a.rest_total; rest += gridDim.z) {
     int64_t r = rest, oin = 0, oout = 0;
     for (int i = 0; i < a.nrest; ++i) {
-      int64_t q = r / a.rdims[i];
-      int64_t v = r - q * a.rdims[i];
+      const int64_t q = SMALL ? int64_t(a.fdims[i].div(uint32_t(r))) : r / a.rdims[i];
+      const int64_t v = r - q * a.rdims[i];
       oin += v * a.rin[i];
       oout += v * a.rout[i];
       r = q;
     }
-    // load: coalesced along input dim 0
-    for (int j = ty; j < 32; j += 8) {
-      int64_t i0 = x0 + tx, iq = y0 + j;
-      if (i0 < a.n0 && iq < a.nq) tile[j][tx] = in[oin + i0 + iq * a.in_q_stride];
+    // load: coalesced along input dim 0, all four in flight
+    T v[4];
+    const int64_t i0 = x0 + tx;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int64_t iq = y0 + ty + 8 * j;
+      if (i0 < a.n0 && iq < a.nq) v[j] = in[oin + i0 + iq * a.in_q_stride];
     }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) tile[ty + 8 * j][tx] = v[j];
     __syncthreads();
     // store: coalesced along output dim 0 (= input dim q)
     for (int j = ty; j < 32; j += 8) {
@@ -256,21 +279,23 @@ void permute_impl(Ctx& c, const Tensor& in, const std::vector<int>& perm, Tensor
   ostr[0] = 1;
   for (int i = 1; i < nd; ++i) ostr[i] = ostr[i - 1] * out.dims[i - 1];
   const int64_t total = in.numel();
+  const bool small = total < (int64_t(1) << 31);  // no count exceeds the number of elements
+  auto fast = [&](int64_t d) { return FastDiv(small ? uint32_t(d) : 1); };
   const T* ip = static_cast<const T*>(in.data());
   T* op = static_cast<T*>(out.data());
-  if (perm[0] == 0 && in.dims[0] >= 16 && nd > 1) {
+  const int64_t nchunk = (in.dims[0] + kPermChunk - 1) / kPermChunk, units = total / in.dims[0] * nchunk;
+  if (perm[0] == 0 && in.dims[0] >= kRowMin && units >= 8 * int64_t(c.sm_count) && nd > 1) {
     RowArgs a{};
     a.nd = nd - 1;
     a.n0 = in.dims[0];
     for (int i = 1; i < nd; ++i) {
       a.odims[i - 1] = out.dims[i];
+      a.fdims[i - 1] = fast(out.dims[i]);
       a.istride[i - 1] = istr[perm[i]];
     }
     const int64_t rows = total / a.n0;
-    const int64_t nchunk = (a.n0 + kPermChunk - 1) / kPermChunk;
-    const int64_t blocks = std::min<int64_t>((rows * nchunk + 7) / 8, int64_t(c.sm_count) * 16);
-    bool small = rows * nchunk <= int64_t(UINT32_MAX);
-    for (int i = 0; i < a.nd; ++i) small = small && a.odims[i] <= int64_t(UINT32_MAX);
+    const int64_t blocks = std::min<int64_t>((units + 7) / 8, int64_t(c.sm_count) * 16);
+    a.fchunk = fast(nchunk);
     if (small)
       launch(c.stream, permute_rows<T, true>, unsigned(std::max<int64_t>(blocks, 1)), 256, 0, a, rows, nchunk, ip, op);
     else
@@ -280,10 +305,13 @@ void permute_impl(Ctx& c, const Tensor& in, const std::vector<int>& perm, Tensor
     a.nd = nd;
     for (int i = 0; i < nd; ++i) {
       a.odims[i] = out.dims[i];
+      a.fdims[i] = fast(out.dims[i]);
       a.istride[i] = istr[perm[i]];
     }
     int64_t blocks = std::min<int64_t>((total + 255) / 256, int64_t(c.sm_count) * 16);
-    launch(c.stream, permute_simple<T>, unsigned(std::max<int64_t>(blocks, 1)), 256, 0, a, total, ip, op);
+    const unsigned grid = unsigned(std::max<int64_t>(blocks, 1));
+    if (small) launch(c.stream, permute_simple<T, true>, grid, 256, 0, a, total, ip, op);
+    else launch(c.stream, permute_simple<T, false>, grid, 256, 0, a, total, ip, op);
   } else {
     const int q = perm[0];
     int p = 0;
@@ -302,6 +330,7 @@ void permute_impl(Ctx& c, const Tensor& in, const std::vector<int>& perm, Tensor
       for (int t = 0; t < nd; ++t)
         if (perm[t] == i) oi = t;
       a.rdims[a.nrest] = in.dims[i];
+      a.fdims[a.nrest] = fast(in.dims[i]);
       a.rin[a.nrest] = istr[i];
       a.rout[a.nrest] = ostr[oi];
       a.nrest++;
@@ -310,7 +339,8 @@ void permute_impl(Ctx& c, const Tensor& in, const std::vector<int>& perm, Tensor
     dim3 grid(unsigned((a.n0 + 31) / 32), unsigned((a.nq + 31) / 32),
               unsigned(std::min<int64_t>(a.rest_total, 65535)));
     IPEPS_CHECK(grid.x <= 2147483647u && grid.y <= 65535u, "permute: grid too large");
-    launch(c.stream, permute_tiled<T>, grid, dim3(32, 8), 0, a, ip, op);
+    if (small) launch(c.stream, permute_tiled<T, true>, grid, dim3(32, 8), 0, a, ip, op);
+    else launch(c.stream, permute_tiled<T, false>, grid, dim3(32, 8), 0, a, ip, op);
   }
   IPEPS_LAUNCH_CHECK();
   c.count(KFam::Permute, 0, 2.0 * double(total) * sizeof(T));
