@@ -252,9 +252,8 @@ struct RealOps {
     const double tol = (c.precision == kPrecMixed) ? std::max(sp.jacobi_tol, sp.jacobi_tol_mixed) : sp.jacobi_tol;
     jacobi_svd_auto(c, X.f64(), k, k, k, J.f64(), k, S.f64(), sp.jacobi_max_sweeps, tol, d_sweeps);
   }
-  // sketch width: 128 columns when that still oversamples by want/2 (the
-  // Jacobi then rotates all of its 64 pairs in one pass of its 8-lane groups),
-  // else at most 160 (the widest sketch whose Jacobi fits in shared memory)
+  // sketch width: 128 columns when that still oversamples by want/2, else at most 160
+  // (every column lengthens the serial steps, the Cholesky factor and the Jacobi SVD)
   int width(int want, int kw, const SvdParams& sp) const {
     if (kw > 128 && want + std::max(sp.min_oversample, want / 2) <= 128) return 128;
     if (kw > 160 && want + sp.min_oversample <= 160) return 160;
