@@ -251,7 +251,7 @@ Tensor tcon(Ctx& c, const Tensor& A, const std::vector<int>& la, const Tensor& B
 class Contraction {
  public:
   Contraction(const Tensor& A, const std::vector<int>& la, const Tensor& B, const std::vector<int>& lb);
-  // raw += A B (raw is allocated by the first product)
+  // raw += A B (raw is allocated by the first product); both of the shapes the plan was made for
   void add(Ctx& c, Tensor& raw, const Tensor& A, const Tensor& B);
   // the sum in output order
   Tensor finish(Ctx& c, const Tensor& raw) const;
@@ -268,7 +268,7 @@ class Contraction {
   Side a_, b_;
   bool swapped_ = false;
   int64_t m_ = 1, n_ = 1, k_ = 1;
-  std::vector<int64_t> odims_, raw_dims_;
+  std::vector<int64_t> a_dims_, b_dims_, odims_, raw_dims_;
   std::vector<int> final_;  // permutation of the product to output order; empty: none
 };
 
