@@ -104,6 +104,21 @@ struct Loader {
   }
 };
 
+// Grid of a product's gm x gn tiles: the row tiles along x, the column tiles along y, as
+// long as y holds them (65535); beyond that turned, so that neither side of the
+// output is limited by the width of its tiles (2.1 million columns at 32).
+struct TileGrid {
+  unsigned x, y;
+  int turned;
+};
+inline TileGrid tile_grid(int64_t gm, int64_t gn) {
+  constexpr int64_t kMaxY = 65535, kMaxX = 2147483647;
+  const bool turned = gn > kMaxY;
+  const int64_t x = turned ? gn : gm, y = turned ? gm : gn;
+  IPEPS_CHECK(x <= kMaxX && y <= kMaxY, "gemm: output too large for the grid");
+  return {unsigned(x), unsigned(y), int(turned)};
+}
+
 constexpr int kMaxCluster = 8;
 
 // CTAs of one kernel that run at the same time in clusters of cs, asked of the

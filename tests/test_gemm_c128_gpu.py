@@ -61,3 +61,12 @@ def test_nested_pullback_ragged(engine, pkg, D, chi):
     ts.close()
     for got, want in ((hH, gH.detach().numpy()), (hN, gN.detach().numpy())):
         assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
+
+
+def test_complex_wide_output(engine, pkg):
+    """More column tiles (32 wide) than a grid's y side holds; bar as above."""
+    m, n, k = 8, 65535 * 32 + 33, 4
+    rng = np.random.default_rng(6)
+    A, B = _rand(rng, m, k), np.asfortranarray(_rand(rng, k, n))
+    out = pkg.tcon([A, B], [[-1, 1], [1, -2]], engine=engine)
+    assert np.all(np.abs(out - A @ B) <= 8 * k * EPS * (np.abs(A) @ np.abs(B)) + 1e-300)

@@ -88,3 +88,17 @@ def test_gemm_f64_tiles_and_splits(engine, pkg, op, m, n, k, beta):
     assert np.all(np.abs(out - (1.25 * (a @ b) + beta * C)) <= bound)
     again = pkg.host.gemm_f64(op[0], op[1], A, B, alpha=1.25, beta=beta, C=C, engine=engine)
     assert np.array_equal(out, again)
+
+
+@pytest.mark.parametrize("op", ["NN", "TT"])
+def test_gemm_f64_wide_output(engine, pkg, op):
+    """More column tiles than a grid's y side holds (65535; 32-column tiles at this size); bound as above."""
+    m, n, k = 4, 65535 * 32 + 33, 17
+    rng = np.random.default_rng(5)
+    A = np.asfortranarray(rng.standard_normal((m, k) if op[0] == "N" else (k, m)))
+    B = np.asfortranarray(rng.standard_normal((k, n) if op[1] == "N" else (n, k)))
+    C = rng.standard_normal((m, n))
+    a, b = (A if op[0] == "N" else A.T), (B if op[1] == "N" else B.T)
+    out = pkg.host.gemm_f64(op[0], op[1], A, B, alpha=1.25, beta=-0.5, C=C, engine=engine)
+    bound = 2 * k * EPS * 1.25 * (np.abs(a) @ np.abs(b)) + 2 * EPS * np.abs(0.5 * C) + 1e-300
+    assert np.all(np.abs(out - (1.25 * (a @ b) - 0.5 * C)) <= bound)
