@@ -136,7 +136,8 @@ __device__ __forceinline__ bool rotate_pair(double2 (&u)[NR], double& nu, double
     ci += __shfl_xor_sync(0xffffffffu, ci, o);
   }
   const double mag2 = fma(cr, cr, ci * ci);
-  // (an underflowing |c|^2 has no usable phase: null columns of a rank-deficient X are left as they are)
+  // (an underflowing |c|^2 has no usable phase: null columns of a rank-deficient X are left as they are; X is
+  // scaled, so the threshold is relative to its largest entry)
   if (!(mag2 >= 1e-300 && nu > 0.0 && nv > 0.0 && mag2 > tol2 * (nu * nv))) return false;
   const double im = rsqrt_normal(mag2), mag = mag2 * im;
   const double ex = cr * im, ey = -ci * im;        // e^{-i phi}
@@ -163,6 +164,10 @@ __device__ __forceinline__ double norm2_of(double x) { return x * x; }
 __device__ __forceinline__ double norm2_of(double2 x) { return fma(x.x, x.x, x.y * x.y); }
 __device__ __forceinline__ void set_real(double& x, double r) { x = r; }
 __device__ __forceinline__ void set_real(double2& x, double r) { x = make_double2(r, 0.0); }
+// x 2^e (real columns are not scaled)
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+__device__ __forceinline__ double scaled(double x, int) { return x; }
+__device__ __forceinline__ double2 scaled(double2 x, int e) { return make_double2(x.x * pow2(e), x.y * pow2(e)); }
 
 template <class T, int NR>
 __device__ __forceinline__ void load_col(T (&u)[NR], const T* x, int lane) {
@@ -174,6 +179,32 @@ template <class T, int NR>
 __device__ __forceinline__ void store_col(const T (&u)[NR], T* x, int lane) {
 #pragma unroll
   for (int j = 0; j < NR; ++j) x[lane + 32 * j] = u[j];
+}
+
+// Exponent by which a complex X is scaled down while it is rotated: that of its largest
+// component (`mx`, this CTA's, of all CTAs through `all` in their shared memory), where
+// that lies beyond 2^+-100 = 1e+-30: the rotations work with fourth powers of the
+// entries, and columns of 1e-13 of the largest are resolved to rounding.  A power of
+// two, so nothing is rounded.  All CTAs of the cluster must have started.
+constexpr int kJScaleExp = 100;
+__device__ int scale_exponent(double mx, double* all, double* red) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (lane == 0) red[warp] = mx;
+  __syncthreads();
+  if (threadIdx.x < kJP) {
+    for (int w = 0; w < kJWarps; ++w) mx = fmax(mx, red[w]);
+    *cluster.map_shared_rank(all + cluster.block_rank(), threadIdx.x) = mx;
+  }
+  cluster.sync();
+  mx = 0.0;
+  for (int r = 0; r < kJP; ++r) mx = fmax(mx, all[r]);
+  if (!(mx > 0.0) || isinf(mx)) return 0;
+  const int e = ilogb(mx);
+  return e < -kJScaleExp || e > kJScaleExp ? max(-1022, min(1022, e)) : 0;
 }
 
 // NR: rows of [X; J] per lane, H = 32 NR.  Bound by the latency of a sub-round (load,
@@ -189,6 +220,7 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
   extern __shared__ __align__(16) double jsm[];
   cg::cluster_group cluster = cg::this_cluster();
   constexpr int H = 32 * NR;
+  constexpr bool CX = sizeof(T) == 16;
   const int rank = int(cluster.block_rank());
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int b = a.b, m = a.m, nx = (a.m + 31) >> 5;
@@ -201,12 +233,15 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
   double* buf = jsm;
   int* blk = reinterpret_cast<int*>(jsm + 4 * slot_sz);  // [2 buffers][2 slots]
   int* flags = blk + 4;                                   // [kJP]
+  double* xmax = jsm + 4 * slot_sz + 16;                  // [kJP]
   __shared__ int s_rot;
+  __shared__ double red[kJWarps];
 
   int cur = 0;
   if (tid < 2) blk[tid] = (tid == 0) ? rank : kJBlocks - 1 - rank;
   __syncthreads();
   // load [X; I] columns of both blocks (columns >= k are zero)
+  double mx = 0.0;
   for (int s = 0; s < 2; ++s) {
     T* dst = reinterpret_cast<T*>(buf + (0 * 2 + s) * slot_sz);
     const int b0 = blk[s] * b;
@@ -218,10 +253,25 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
         if (r < m && col < a.k) v = X[r + int64_t(col) * a.ldx];
         if (col >= a.k) set_real(v, 0.0);
         dst[j * H + r] = v;
+        if constexpr (CX)
+          if (r < m) mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
       }
     }
   }
   cluster.sync();
+  int ex = 0;  // X is rotated as X 2^-ex
+  if constexpr (CX) {
+    ex = scale_exponent(mx, xmax, red);
+    if (ex != 0) {
+      for (int s = 0; s < 2; ++s)
+        for (int j = warp; j < b; j += kJWarps)
+          for (int r = lane; r < m; r += 32) {
+            T* x = reinterpret_cast<T*>(buf + s * slot_sz) + j * H + r;
+            *x = scaled(*x, -ex);
+          }
+      __syncthreads();
+    }
+  }
 
   int sweep = 0;
   bool converged = false;
@@ -321,7 +371,7 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
       for (int r = lane; r < H; r += 32) {
         const T v = src[j * H + r];
         if (r < m) {
-          Xout[r + int64_t(col) * a.ldx] = v;
+          Xout[r + int64_t(col) * a.ldx] = scaled(v, ex);
           nn += norm2_of(v);
         } else if (r - m < a.k) {
           J[(r - m) + int64_t(col) * a.ldj] = v;
@@ -329,7 +379,7 @@ __global__ void __cluster_dims__(kJP, 1, 1) __launch_bounds__(kJWarps * 32, 1) j
       }
 #pragma unroll
       for (int o = 16; o; o >>= 1) nn += __shfl_xor_sync(0xffffffffu, nn, o);
-      if (lane == 0) a.S[col] = sqrt(nn);
+      if (lane == 0) a.S[col] = CX ? sqrt(nn) * pow2(ex) : sqrt(nn);
     }
   }
   if (rank == 0 && tid == 0) {

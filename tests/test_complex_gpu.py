@@ -144,3 +144,17 @@ def test_projector_complex_rank_deficient(engine, pkg, n, rank):
     P1, P2, s = pkg.get_projector(R1, R2, rank, engine=engine)
     assert np.isfinite(P1).all() and np.isfinite(P2).all()
     assert np.abs(s[:rank] - s_ref[:rank]).max() <= 20 * n * np.finfo(float).eps * s_ref[0]
+
+
+@pytest.mark.parametrize("n,rank,scale", [(12, 3, 1e-20), (16, 4, 1e-20), (16, 4, 1e-40), (33, 7, 1e-40),
+                                          (66, 5, 1e-20), (66, 5, 1e-40)])
+def test_projector_complex_small_corners(engine, pkg, n, rank, scale):
+    """Corners whose product lies around 1e-38 and 1e-76: the fourth powers that the Jacobi rotations work with
+    underflow unless the cluster kernel (from 16 columns) scales X; bars as above."""
+    rng = np.random.default_rng(n)
+    R1 = scale * (_crandn(rng, n, rank) @ _crandn(rng, rank, n))
+    R2 = scale * (_crandn(rng, n, rank) @ _crandn(rng, rank, n))
+    s_ref = np.linalg.svd(R1 / scale @ (R2 / scale), compute_uv=False)
+    P1, P2, s = pkg.get_projector(R1, R2, rank, engine=engine)
+    assert np.isfinite(P1).all() and np.isfinite(P2).all()
+    assert np.abs(s[:rank] / scale ** 2 - s_ref[:rank]).max() <= 20 * n * np.finfo(float).eps * s_ref[0]
