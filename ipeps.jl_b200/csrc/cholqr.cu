@@ -57,7 +57,7 @@ __device__ __forceinline__ void bar_post() {
 
 // Packed upper block triangle of R, block row by block row: block (I, J) at
 // col_base(I) + J - I.  Inside a block the entries (2t, g) and (2t + 1, g) are
-// neighbours, at 2 (8 t + g): lane (g, t) of a warp then has with one 16-byte
+// neighbours, at 2 (4 g + t): lane (g, t) of a warp then has with one 16-byte
 // access what it needs of the block as the B operand of two m8n8k4 products
 // over k = {2t} and k = {2t + 1}, and what an accumulator or an A operand
 // holds of the transposed block.
@@ -76,12 +76,15 @@ __host__ __device__ __forceinline__ int col_base(int I, int nb) { return I * nb 
 // rolled: with the trailing blocks in registers (unrolled by slot) the SM spent
 // its time fetching instructions (55 us at k = 160).
 // The contract is that of chol_blocked: shift_factor * trace is added to the
-// diagonal, a pivot at or below 1e-32 trace leaves R[j][j] = 1 and row j zero.
+// diagonal, a pivot at or below 1e-32 trace leaves R[j][j] = 1 and row j zero (inside the
+// diagonal block by the pivot's factor 0, right of it by leaving its column out of the
+// inverse in L_Ip = C_Ip R_pp^-1; `failed` has the panel's failed pivots as bits).
 // In the end S holds the packed R; it is also written to Rpk if that is given, and R's
 // diagonal blocks to G.
 __device__ __forceinline__ void factor_panels(double2* S, int k, double shift_factor, double2* __restrict__ Rpk,
                                               double* G, int64_t ldg) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  __shared__ int failed[kCholqrMax / 8];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2;
   const int nb = (k + 7) >> 3;
   if (warp == 0) {
     double tr = 0;
@@ -97,6 +100,7 @@ __device__ __forceinline__ void factor_panels(double2* S, int k, double shift_fa
     for (int p = 0; p < nb; ++p) {
       double2* D = S + col_base(p, nb) * 32;
       double d[8][8], x[8];  // d[c][r], c <= r: entry (r, c) of the block; x: row `me` of the inverse
+      int fail = 0;
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
 #pragma unroll
@@ -112,6 +116,7 @@ __device__ __forceinline__ void factor_panels(double2* S, int k, double shift_fa
       for (int j = 0; j < 8; ++j) {
         const double piv = d[j][j];
         const bool ok = piv > tiny || 8 * p + j >= k;
+        fail |= int(!ok) << j;
         const double rt = rsqrt_normal(piv);  // (without rsqrt's cases the chain's shadow is filled)
         const double rs = __hiloint2double(ok ? __double2hiint(rt) : 0, ok ? __double2loint(rt) : 0);
         x[j] *= ok ? rs : 1.0;
@@ -137,14 +142,16 @@ __device__ __forceinline__ void factor_panels(double2* S, int k, double shift_fa
         if (p > 0) bar_wait<2, 64>();
         const double2 c = D[32 + lane];
         double x0 = 0.0, x1 = 0.0;
-        dmma8(x0, x1, c.x, q.x);
-        dmma8(x0, x1, c.y, q.y);
+        const bool out = fail >> g & 1;
+        dmma8(x0, x1, c.x, out ? 0.0 : q.x);
+        dmma8(x0, x1, c.y, out ? 0.0 : q.y);
         D[32 + lane] = make_double2(x0, x1);
         double2* N = S + col_base(p + 1, nb) * 32 + lane;
         double2 n = *N;
         dmma8(n.x, n.y, -x0, x0);
         dmma8(n.x, n.y, -x1, x1);
         *N = n;
+        if (lane == 0) failed[p] = fail;
         __syncwarp();
         bar_post<1, 32 + kUpdateThreads>();
         if (Rpk) Rpk[(col_base(p, nb) + 1) * 32 + lane] = make_double2(x0, x1);
@@ -164,7 +171,8 @@ __device__ __forceinline__ void factor_panels(double2* S, int k, double shift_fa
     for (int p = 0; p + 1 < nb; ++p) {
       double2* L = S + (col_base(p, nb) - p) * 32 + lane;  // L_Ip at L[32 I]
       bar_wait<1, 32 + kUpdateThreads>();
-      const double2 q = L[32 * p];
+      double2 q = L[32 * p];
+      if (failed[p] >> g & 1) q = make_double2(0.0, 0.0);
       for (int I = p + 2 + u; I < nb; I += kUpdateWarps) {
         const double2 c = L[32 * I];
         double x0 = 0.0, x1 = 0.0;

@@ -133,3 +133,22 @@ def test_orth_in_one_launch(engine, pkg, N, k):
         if passes == 3:
             assert np.abs(Q.T @ Q - np.eye(k)).max() <= 1e-14 * k ** 0.5
             assert np.linalg.norm(Q - Qn) <= 1e-14 * cond * k
+
+
+@pytest.mark.parametrize("k,j", [(40, 3), (40, 8), (33, 15), (160, 20), (200, 3)])
+def test_orth_failed_pivot(engine, pkg, k, j):
+    """A column 1e-25 of the others: the shift of the first pass leaves it at ~1e-21, so its pivot in the second
+    pass is below 1e-32 of the trace.  That pass then has R[j, j] = 1 and row j zero, so row j of the product of
+    both factors is the first factor's (from its definition, in numpy).  The entries left in the row instead
+    would double it.  Rounding: k eps in the sums behind an entry, with a factor 1e3 for their cancellation."""
+    N = 2 * k
+    rng = np.random.default_rng(k + j)
+    Y = rng.standard_normal((N, k))
+    Y[:, j] *= 1e-25
+    G = Y.T @ Y
+    u = 0.5 * np.finfo(float).eps
+    R1 = np.linalg.cholesky(G + 11.0 * (N * k + k * (k + 1)) * u * np.trace(G) * np.eye(k)).T
+    _, R = pkg.orth(Y, 2, engine=engine)
+    bar = 1e3 * k * 2 * u
+    assert abs(R[j, j] - R1[j, j]) <= bar * R1[j, j]
+    assert np.abs(R[j, j + 1:] - R1[j, j + 1:]).max() <= bar * np.abs(R1[j, j + 1:]).max()
