@@ -483,7 +483,7 @@ ProjResult projector_impl(Ctx& c, Ops& o, int chi, const SvdParams& sp, ProjCach
   }
   const bool adapt = q > 0 && cache && inter >= 3 && !shift;
   if (adapt) q += cache->qbonus;
-  int iters = q;  // power iterations of all passes
+  int iters = q;  // power iterations behind the accepted sketch
   int extra = 0;
   double res_final = 1.0;
 
@@ -515,6 +515,7 @@ ProjResult projector_impl(Ctx& c, Ops& o, int chi, const SvdParams& sp, ProjCach
       randn(c, Om);
       q = sp.power_iters;
       b = 0;
+      iters = q;  // the abandoned sketch says nothing about the next call
       --attempt;
       continue;
     }
