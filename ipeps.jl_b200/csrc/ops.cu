@@ -122,7 +122,7 @@ namespace {
 // division is about twenty times the instructions, and in short rows and in tiles they
 // were most of the work.  Divisions -> multiplications, us: tiles at 100 x 25 x 100 x 25
 // (100 MB moved) 34.0 -> 23.8, 2500 x 2500 23.8 -> 15.5 (6.4 TB/s); rows of 100 elements
-// 21.9 -> 21.0 (4.8 TB/s), of 25 68.8 -> 45.
+// 21.9 -> 21.0, of 25 68.8 -> 45.
 struct PermArgs {
   int nd;
   int64_t odims[kMaxDims];    // output dims
@@ -173,10 +173,31 @@ struct RowArgs {
 constexpr int64_t kPermChunk = 2048;
 // Rows from here on, in at least eight units per SM, else element by element with four
 // loads in flight (permute_simple), by rows -> by elements, us: 25-element rows (25 x 100
-// x 25 x 100) 45 -> 26.4, 40 x 4 x 40 x 4 3.9 -> 3.6, 64 x 100 x 100 x 5 10.7 -> 14.5, 100 x 25
-// x 100 x 25 21.0 -> 26.5; few long rows (4099 x 3 x 5, 45 units) 12.5 -> 3.5, 1000 x 25 x 25
-// 5.8 -> 4.8.
+// x 25 x 100) 53 -> 26.5, 40 x 100 x 40 x 25 22.0 -> 16.9, 48 x 48 x 48 x 9 6.5 -> 6.5, 64 x 100
+// x 100 x 5 12.1 -> 14.4, 100 x 25 x 100 x 25 20.4 -> 26.4; few long rows (4099 x 3 x 5, 45
+// units) 6.1 -> 4.8, 1000 x 33 x 33 (1089) 5.9 -> 5.8, 1000 x 45 x 45 (2025) 5.6 -> 8.1.
 constexpr int64_t kRowMin = 64;
+// The same from 2^31 elements on, where the element-wise kernel divides in 64 bits while
+// the row index mostly still fits in 31, by rows -> by elements at 35 to 37 GB moved, ms:
+// rows of 25 elements 19.2 -> 14.8, 32 15.8 -> 14.7, 40 13.1 -> 14.4, 60 9.5 -> 14.6.
+constexpr int64_t kRowMinLarge = 40;
+
+// One warp copies n elements, four loads in flight per lane.  (Left to the compiler, the
+// memory clobber of pdl_wait keeps the loads behind the stores: rows of 999 doubles,
+// 66 MB, 35.7 us, 24.8 so; of 500000, 64 MB, 30.0 and 18.7; of 100, 50 MB, 21.0 and 20.4
+// (4.9 TB/s).  With registers for eight CTAs per SM it spills: 29.3 and 27.1.)
+template <typename E>
+__device__ __forceinline__ void copy_run(const E* __restrict__ src, E* __restrict__ dst, int64_t n, int lane) {
+  for (int i = lane; i < int(n); i += 128) {
+    E v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i + 32 * j < int(n)) v[j] = src[i + 32 * j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i + 32 * j < int(n)) dst[i + 32 * j] = v[j];
+  }
+}
 
 template <typename T, bool SMALL>
 __global__ void permute_rows(RowArgs a, int64_t rows, int64_t nchunk, const T* __restrict__ in, T* __restrict__ out) {
@@ -213,12 +234,10 @@ __global__ void permute_rows(RowArgs a, int64_t rows, int64_t nchunk, const T* _
       // both runs 16-byte aligned: two doubles per load and store
       const double2* s2 = reinterpret_cast<const double2*>(src);
       double2* d2 = reinterpret_cast<double2*>(dst);
-#pragma unroll 4
-      for (int64_t i = (c0 >> 1) + lane; i < (c1 >> 1); i += 32) d2[i] = s2[i];
+      copy_run(s2 + (c0 >> 1), d2 + (c0 >> 1), (c1 >> 1) - (c0 >> 1), lane);
       if ((c1 & 1) && lane == 0) dst[c1 - 1] = src[c1 - 1];
     } else {
-#pragma unroll 4
-      for (int64_t i = c0 + lane; i < c1; i += 32) dst[i] = src[i];
+      copy_run(src + c0, dst + c0, c1 - c0, lane);
     }
   }
 }
@@ -284,19 +303,21 @@ void permute_impl(Ctx& c, const Tensor& in, const std::vector<int>& perm, Tensor
   const T* ip = static_cast<const T*>(in.data());
   T* op = static_cast<T*>(out.data());
   const int64_t nchunk = (in.dims[0] + kPermChunk - 1) / kPermChunk, units = total / in.dims[0] * nchunk;
-  if (perm[0] == 0 && in.dims[0] >= kRowMin && units >= 8 * int64_t(c.sm_count) && nd > 1) {
+  if (perm[0] == 0 && in.dims[0] >= (small ? kRowMin : kRowMinLarge) && units >= 8 * int64_t(c.sm_count) && nd > 1) {
+    const bool small_rows = units < (int64_t(1) << 31);  // no count of the row index exceeds that of the units
+    auto fast_row = [&](int64_t d) { return FastDiv(small_rows ? uint32_t(d) : 1); };
     RowArgs a{};
     a.nd = nd - 1;
     a.n0 = in.dims[0];
     for (int i = 1; i < nd; ++i) {
       a.odims[i - 1] = out.dims[i];
-      a.fdims[i - 1] = fast(out.dims[i]);
+      a.fdims[i - 1] = fast_row(out.dims[i]);
       a.istride[i - 1] = istr[perm[i]];
     }
     const int64_t rows = total / a.n0;
     const int64_t blocks = std::min<int64_t>((units + 7) / 8, int64_t(c.sm_count) * 16);
-    a.fchunk = fast(nchunk);
-    if (small)
+    a.fchunk = fast_row(nchunk);
+    if (small_rows)
       launch(c.stream, permute_rows<T, true>, unsigned(std::max<int64_t>(blocks, 1)), 256, 0, a, rows, nchunk, ip, op);
     else
       launch(c.stream, permute_rows<T, false>, unsigned(std::max<int64_t>(blocks, 1)), 256, 0, a, rows, nchunk, ip, op);
