@@ -104,20 +104,13 @@ struct Loader {
   }
 };
 
-// Grid of a product's gm x gn tiles: the row tiles along x, the column tiles along y, as
-// long as y holds them (65535); beyond that turned, so that neither side of the
-// output is limited by the width of its tiles (2.1 million columns at 32).
-struct TileGrid {
-  unsigned x, y;
-  int turned;
-};
-inline TileGrid tile_grid(int64_t gm, int64_t gn) {
-  constexpr int64_t kMaxY = 65535, kMaxX = 2147483647;
-  const bool turned = gn > kMaxY;
-  const int64_t x = turned ? gn : gm, y = turned ? gm : gn;
-  IPEPS_CHECK(x <= kMaxX && y <= kMaxY, "gemm: output too large for the grid");
-  return {unsigned(x), unsigned(y), int(turned)};
-}
+// Tiles that the grid's y side (the columns) holds, and the columns of one launch: wider
+// outputs are formed in panels of as many (2.1 million at the narrowest tiles, and a
+// multiple of 32, so that operands keep their alignment).  The alternative, the column tiles
+// along x in such cases, costs every launch of many small tiles (8 x 1000000 x 4:
+// 106.4 -> 108.5 us).
+constexpr int64_t kMaxGridY = 65535;
+constexpr int64_t kMaxColumns = 32 * kMaxGridY;
 
 constexpr int kMaxCluster = 8;
 

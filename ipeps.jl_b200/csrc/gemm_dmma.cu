@@ -52,13 +52,12 @@ struct Geo {
 // CTA a slice of the rows-by-columns of all of them, in rank order (so the
 // result does not depend on timing).  More than one cluster per tile (cz > 1):
 // the clusters' sums go to `partial` for dmma_splitk_reduce.  upper: only tiles
-// that reach the upper triangle are formed (C symmetric).  turned: the column tiles
-// are along x (see tile_grid).
+// that reach the upper triangle are formed (C symmetric).
 template <int BM, int BN, int WGM, int WGN, int KW, int MINB, bool AK, bool BK_, int VEC>
 __global__ void __launch_bounds__(WGM * WGN * KW * 32, MINB)
     dmma_gemm_kernel(int64_t M, int64_t N, int64_t K, int64_t kchunk, double alpha, const double* __restrict__ A,
                      int64_t lda, const double* __restrict__ B, int64_t ldb, double beta, double* __restrict__ C,
-                     int64_t ldc, double* __restrict__ partial, int cs, int upper, int turned) {
+                     int64_t ldc, double* __restrict__ partial, int cs, int upper) {
   pdl_wait();
   using GE = Geo<BM, BN, WGM, WGN, KW, AK, BK_>;
   constexpr int NT = GE::NT;
@@ -74,7 +73,7 @@ __global__ void __launch_bounds__(WGM * WGN * KW * 32, MINB)
   const int g = lane >> 2, t = lane & 3;
   const int kw = warp / (WGM * WGN), wmn = warp % (WGM * WGN);
   const int wm0 = (wmn % WGM) * WM, wn0 = (wmn / WGM) * WN;
-  const int64_t m0 = int64_t(turned ? blockIdx.y : blockIdx.x) * BM, n0 = int64_t(turned ? blockIdx.x : blockIdx.y) * BN;
+  const int64_t m0 = int64_t(blockIdx.x) * BM, n0 = int64_t(blockIdx.y) * BN;
   if (upper && n0 + BN <= m0) return;  // the whole cluster: its CTAs share the tile
   const int64_t kb = int64_t(blockIdx.z) * kchunk;
   const int64_t ke = imin(K, kb + kchunk);
@@ -275,15 +274,16 @@ void launch_cfg(Ctx& c, const Args& a, Split sp) {
   auto kern = dmma_gemm_kernel<BM, BN, WGM, WGN, KW, MINB, AK, BK_, VEC>;
   static SmemAttrOnce attr;
   attr.ensure(kern, int(GE::smem));
-  const TileGrid g = tile_grid((a.m + BM - 1) / BM, (a.n + BN - 1) / BN);
+  const int64_t gx = (a.m + BM - 1) / BM, gy = (a.n + BN - 1) / BN;
+  IPEPS_CHECK(gy <= kMaxGridY, "gemm: n too large for grid");
   int64_t kchunk = (a.k + sp.S - 1) / sp.S;
   kchunk = ((kchunk + kBK - 1) / kBK) * kBK;
   const int cz = sp.S / sp.cs;
   double* partial = nullptr;
   if (cz > 1) partial = static_cast<double*>(c.workspace(size_t(cz) * a.m * a.n * sizeof(double)));
-  launch_clusters(c.stream, kern, dim3(g.x, g.y, unsigned(sp.S)), GE::NT, GE::smem, dim3(1, 1, unsigned(sp.cs)), a.m,
-                  a.n, a.k, kchunk, a.alpha, a.A, a.lda, a.B, a.ldb, a.beta, a.C, a.ldc, partial, sp.cs, int(a.upper),
-                  g.turned);
+  launch_clusters(c.stream, kern, dim3(unsigned(gx), unsigned(gy), unsigned(sp.S)), GE::NT, GE::smem,
+                  dim3(1, 1, unsigned(sp.cs)), a.m, a.n, a.k, kchunk, a.alpha, a.A, a.lda, a.B, a.ldb, a.beta, a.C,
+                  a.ldc, partial, sp.cs, int(a.upper));
   if (cz > 1) {
     const int64_t tot = a.m * a.n;
     const bool pairs = a.ldc == a.m && (tot & 1) == 0 && (reinterpret_cast<uintptr_t>(a.C) & 15) == 0;
@@ -374,6 +374,12 @@ void gemm_f64_dmma(Ctx& c, char opA, char opB, int64_t m, int64_t n, int64_t k, 
   if (m <= 0 || n <= 0) return;
   IPEPS_CHECK(k > 0, "gemm: k == 0 is not supported");
   const bool ta = (opA == 'T' || opA == 't'), tb = (opB == 'T' || opB == 't');
+  if (n > kMaxColumns) {  // (upper: square outputs are never this wide)
+    for (int64_t j = 0; j < n; j += kMaxColumns)
+      gemm_f64_dmma(c, opA, opB, m, std::min(kMaxColumns, n - j), k, alpha, A, lda, B + (tb ? j : j * ldb), ldb, beta,
+                    C + j * ldc, ldc);
+    return;
+  }
   IPEPS_CHECK(ta || opA == 'N' || opA == 'n', "gemm: bad op");
   IPEPS_CHECK(tb || opB == 'N' || opB == 'n', "gemm: bad op");
   ProfScope ps(c, KFam::GemmF64);

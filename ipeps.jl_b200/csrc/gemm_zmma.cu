@@ -49,7 +49,7 @@ template <int BM, int BN, int WGM, int WGN, int KW, class EA, class EB, bool AK,
 __global__ void __launch_bounds__(WGM * WGN * KW * 32)
     zmma_gemm_kernel(int64_t M, int64_t N, int64_t K, int64_t kchunk, double2 alpha, const EA* __restrict__ A,
                      int64_t lda, double sa, const EB* __restrict__ B, int64_t ldb, double sb, double2 beta,
-                     double2* __restrict__ C, int64_t ldc, double2* __restrict__ partial, int cs, int turned) {
+                     double2* __restrict__ C, int64_t ldc, double2* __restrict__ partial, int cs) {
   pdl_wait();
   using GE = Geo<BM, BN, WGM, WGN, KW, EA, EB, AK, BK_>;
   constexpr bool CA = std::is_same_v<EA, double2>, CB = std::is_same_v<EB, double2>;
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(WGM * WGN * KW * 32)
   const int g = lane >> 2, t = lane & 3;
   const int kw = warp / (WGM * WGN), wmn = warp % (WGM * WGN);
   const int wm0 = (wmn % WGM) * WM, wn0 = (wmn / WGM) * WN;
-  const int64_t m0 = int64_t(turned ? blockIdx.y : blockIdx.x) * BM, n0 = int64_t(turned ? blockIdx.x : blockIdx.y) * BN;
+  const int64_t m0 = int64_t(blockIdx.x) * BM, n0 = int64_t(blockIdx.y) * BN;
   const int64_t kb = int64_t(blockIdx.z) * kchunk;
   const int64_t ke = imin(K, kb + kchunk);
   const int nk = ke > kb ? int((ke - kb + kBK - 1) / kBK) : 0;
@@ -251,15 +251,16 @@ void launch_cfg(Ctx& c, const Args& a, int S, int cs) {
   auto kern = zmma_gemm_kernel<BM, BN, WGM, WGN, KW, EA, EB, AK, BK_>;
   static SmemAttrOnce attr;
   attr.ensure(kern, int(GE::smem));
-  const TileGrid g = tile_grid((a.m + BM - 1) / BM, (a.n + BN - 1) / BN);
+  const int64_t gx = (a.m + BM - 1) / BM, gy = (a.n + BN - 1) / BN;
+  IPEPS_CHECK(gy <= kMaxGridY, "gemm: n too large for grid");
   int64_t kchunk = (a.k + S - 1) / S;
   kchunk = ((kchunk + kBK - 1) / kBK) * kBK;
   const int cz = S / cs;
   double2* partial = nullptr;
   if (cz > 1) partial = static_cast<double2*>(c.workspace(size_t(cz) * a.m * a.n * sizeof(double2)));
-  launch_clusters(c.stream, kern, dim3(g.x, g.y, unsigned(S)), GE::NT, GE::smem, dim3(1, 1, unsigned(cs)), a.m, a.n,
-                  a.k, kchunk, a.alpha, static_cast<const EA*>(a.A), a.lda, a.sa, static_cast<const EB*>(a.B), a.ldb,
-                  a.sb, a.beta, a.C, a.ldc, partial, cs, g.turned);
+  launch_clusters(c.stream, kern, dim3(unsigned(gx), unsigned(gy), unsigned(S)), GE::NT, GE::smem,
+                  dim3(1, 1, unsigned(cs)), a.m, a.n, a.k, kchunk, a.alpha, static_cast<const EA*>(a.A), a.lda, a.sa,
+                  static_cast<const EB*>(a.B), a.ldb, a.sb, a.beta, a.C, a.ldc, partial, cs);
   if (cz > 1) {
     const int64_t tot = a.m * a.n;
     launch(c.stream, zmma_splitk_reduce, unsigned((tot + 255) / 256), 256, 0, a.m, a.n, cz, partial, a.alpha, a.beta,
@@ -338,6 +339,13 @@ void gemm_c128_dmma(Ctx& c, char opA, DType dtA, char opB, DType dtB, int64_t m,
     throw Error(kEInval, "gemm: bad op");
   };
   const int oa = op(opA), ob = op(opB);
+  if (n > kMaxColumns) {
+    for (int64_t j = 0; j < n; j += kMaxColumns)
+      gemm_c128_dmma(c, opA, dtA, opB, dtB, m, std::min(kMaxColumns, n - j), k, alpha, A, lda,
+                     static_cast<const char*>(B) + (ob ? j : j * ldb) * int64_t(dtype_size(dtB)), ldb, beta,
+                     static_cast<double2*>(C) + j * ldc, ldc);
+    return;
+  }
   const int type = dtA == DType::F64 ? 2 : dtB == DType::F64 ? 1 : 0;
   IPEPS_CHECK(dtA == DType::C128 || dtB == DType::C128, "gemm: a complex operand is needed");
   ProfScope ps(c, KFam::GemmF64);
