@@ -67,17 +67,25 @@ def test_gemm_f64_split_k_is_deterministic(engine, pkg):
 
 @pytest.mark.parametrize("op", ["NN", "TN", "NT", "TT"])
 @pytest.mark.parametrize("m,n,k,beta", [
-    (33, 31, 65, 0.0),      # a 32 x 32 tile and its remainders, two K chunks at most
-    (120, 62, 120, 0.5),    # 32 x 32 tiles in clusters of three
-    (37, 37, 333, 0.0),     # clusters of seven, odd leading dimensions (8-byte copies)
-    (65, 33, 1000, -1.0),   # 64 x 32 tiles' remainders, clusters of eight
-    (9, 18, 12321, 0.0),    # more than one cluster per tile: sums through the workspace
-    (17, 23, 40001, 2.0),   # the same with a remainder in K and beta
-    (2500, 79, 1111, 0.0),  # one 80-column tile, partial sums without clusters
+    # (the plans named are those of a B200: tile, K chunks, CTAs per cluster)
+    (33, 31, 65, 0.0),      # 32 x 32 and its remainders, no split
+    (120, 62, 120, 0.5),    # 32 x 32, 2 chunks in a cluster of two
+    (37, 37, 150, 0.0),     # 32 x 32, 4 chunks in a cluster of four; odd leading dimensions (8-byte copies)
+    (37, 37, 333, 0.0),     # 32 x 32, 8 chunks in a cluster of eight
+    (65, 33, 1000, -1.0),   # the same with remainders in both sides
+    (2500, 160, 2500, 0.0),  # 64 x 32, clusters of two
+    (9, 18, 12321, 0.0),    # 32 x 32, 128 chunks in clusters of eight: their sums through the workspace
+    (17, 23, 40001, 2.0),   # 256 chunks with a remainder in K and beta
+    (2500, 128, 2500, 1.0),  # 64 x 64, 5 chunks without clusters, all through the workspace
+    (2500, 79, 1111, 0.0),  # 128 x 80, 7 chunks without clusters
+    (20000, 50, 25, 0.0),   # 64 x 64
+    (30000, 64, 40, 0.0),   # 128 x 64
+    (100000, 40, 16, 0.0),  # 128 x 48
     (300, 900, 5, 1.0),     # less than one K step
 ])
 def test_gemm_f64_tiles_and_splits(engine, pkg, op, m, n, k, beta):
-    """Every tile configuration and way of summing the K chunks, with remainders; bound as above."""
+    """Every tile configuration, and K chunks summed in clusters, through the workspace and both, with remainders;
+    bound as above."""
     rng = np.random.default_rng(m + 3 * n + 7 * k)
     A = np.asfortranarray(rng.standard_normal((m, k) if op[0] == "N" else (k, m)))
     B = np.asfortranarray(rng.standard_normal((k, n) if op[1] == "N" else (n, k)))

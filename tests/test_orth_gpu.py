@@ -1,8 +1,9 @@
 """The projector's orthonormalisation (shifted CholeskyQR, csrc/projector.cu
 `orth`) through ``ipeps_orth``: the range-finder step that stands in for the
-Q factor of the reference's full SVD (ctmrg.jl:257).  It exercises the
-register-resident Cholesky (k <= 160), the blocked Cholesky (larger k) and the
-row-parallel triangular solve directly, against numpy's QR:
+Q factor of the reference's full SVD (ctmrg.jl:257).  It exercises the packed
+panel Cholesky and triangular solve (k <= 192), the blocked Cholesky with the
+row-parallel solve (larger k) and the one-launch kernel of small sketches directly,
+against numpy's QR:
 
 * Q^T Q = I to 1e-14 and Q R = Y to 1e-14 relative (sCholQR3 on a
   well-conditioned Y); one pass (shifted) orthogonal to 1e-6, two to 1e-14;
@@ -62,8 +63,8 @@ def test_orth_ill_conditioned_and_rank_deficient(engine, pkg, k):
 @pytest.mark.parametrize("N,k", [(1, 1), (7, 7), (8, 8), (40, 9), (33, 16), (129, 24), (120, 62), (333, 76), (97, 97),
                                  (1201, 104), (160, 159), (3000, 160), (170, 161)])
 def test_orth_block_edges(engine, pkg, N, k):
-    """Panel edges of the blocked Cholesky and triangular solve (8 columns, 8 rows; k <= 160 and the
-    first k beyond), square Y among them.  Bars: two unshifted CholeskyQR passes after the shifted one
+    """Panel edges of the packed Cholesky and triangular solve (8 columns, 8 rows, 32 columns per
+    instance of the solve), square Y among them; the widest packed k follows below.  Bars: two unshifted CholeskyQR passes after the shifted one
     leave rounding, 10 k eps in Q^T Q and in Q R = Y; R against the Cholesky factor of Y^T Y (64-bit,
     backward stable) differs by its conditioning, 100 k eps cond(Y)^2."""
     rng = np.random.default_rng(N * 1000 + k)
@@ -133,6 +134,20 @@ def test_orth_in_one_launch(engine, pkg, N, k):
         if passes == 3:
             assert np.abs(Q.T @ Q - np.eye(k)).max() <= 1e-14 * k ** 0.5
             assert np.linalg.norm(Q - Qn) <= 1e-14 * cond * k
+
+
+@pytest.mark.parametrize("N,k", [(400, 191), (400, 192), (400, 193), (250, 192), (3000, 192)])
+def test_orth_largest_packed(engine, pkg, N, k):
+    """The widest sketches of the packed Cholesky and solve (192 columns) and the first beyond them; bars as in
+    test_orth_block_edges."""
+    rng = np.random.default_rng(N + k)
+    Y = rng.standard_normal((N, k)) + (4.0 * N ** 0.5 * np.eye(N, k) if N < 2 * k else 0.0)
+    eps = np.finfo(float).eps
+    Q, R = pkg.orth(Y, 3, engine=engine)
+    assert np.abs(Q.T @ Q - np.eye(k)).max() <= 10 * k * eps
+    assert np.linalg.norm(Q @ R - Y) <= 10 * k * eps * np.linalg.norm(Y)
+    ref = np.linalg.cholesky(Y.T @ Y).T
+    assert np.linalg.norm(R - ref) <= 100 * k * eps * np.linalg.cond(Y) ** 2 * np.linalg.norm(ref)
 
 
 @pytest.mark.parametrize("k,j", [(40, 3), (40, 8), (33, 15), (160, 20), (200, 3)])
