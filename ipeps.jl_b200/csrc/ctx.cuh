@@ -5,6 +5,7 @@
 
 #include "common.cuh"
 
+#include <algorithm>
 #include <array>
 #include <atomic>
 #include <map>
@@ -268,7 +269,14 @@ class Contraction {
   Side a_, b_;
   bool swapped_ = false;
   int64_t m_ = 1, n_ = 1, k_ = 1;
-  std::vector<int64_t> a_dims_, b_dims_, odims_, raw_dims_;
+  struct Shape {  // (no allocation: a plan is made for every product)
+    int nd = 0;
+    int64_t dims[kMaxDims] = {0};
+    Shape() = default;
+    explicit Shape(const Tensor& t) : nd(t.nd) { std::copy(t.dims, t.dims + t.nd, dims); }
+    bool of(const Tensor& t) const { return t.nd == nd && std::equal(dims, dims + nd, t.dims); }
+  } a_shape_, b_shape_;
+  std::vector<int64_t> odims_, raw_dims_;
   std::vector<int> final_;  // permutation of the product to output order; empty: none
 };
 

@@ -72,10 +72,6 @@ Contraction::Side plan_side(const std::vector<int>& lx, const std::vector<int>& 
   return s;
 }
 
-bool has_shape(const Tensor& t, const std::vector<int64_t>& dims) {
-  return t.nd == int(dims.size()) && std::equal(dims.begin(), dims.end(), t.dims);
-}
-
 // op(A) op(B) of real and complex operands; the result is complex when either is
 void gemm_any(Ctx& c, char opA, const Tensor& A, int64_t lda, char opB, const Tensor& B, int64_t ldb, int64_t m,
               int64_t n, int64_t k, double beta, void* C, int64_t ldc) {
@@ -90,8 +86,8 @@ void gemm_any(Ctx& c, char opA, const Tensor& A, int64_t lda, char opB, const Te
 Contraction::Contraction(const Tensor& A, const std::vector<int>& la, const Tensor& B, const std::vector<int>& lb) {
   IPEPS_CHECK(int(la.size()) == A.nd, "tcon: label count != rank of A " + shape_str(A));
   IPEPS_CHECK(int(lb.size()) == B.nd, "tcon: label count != rank of B " + shape_str(B));
-  a_dims_ = A.shape();
-  b_dims_ = B.shape();
+  a_shape_ = Shape(A);
+  b_shape_ = Shape(B);
   std::map<int, int64_t> ext;
   for (int i = 0; i < A.nd; ++i) ext[la[i]] = A.dims[i];
   for (int i = 0; i < B.nd; ++i) {
@@ -162,7 +158,7 @@ Tensor Contraction::prepared(Ctx& c, Side& s, const Tensor& X) {
 void Contraction::add(Ctx& c, Tensor& raw, const Tensor& A, const Tensor& B) {
   // The plan's extents are those of the operands it was made for.  Another component of a
   // nested tensor can differ: set_CT replaces component 0 of an environment alone.
-  IPEPS_CHECK(has_shape(A, a_dims_) && has_shape(B, b_dims_),
+  IPEPS_CHECK(a_shape_.of(A) && b_shape_.of(B),
               "tcon: operands " + shape_str(A) + " " + shape_str(B) + " differ from the sum's other terms");
   const DType dt = (A.dt == DType::C128 || B.dt == DType::C128) ? DType::C128 : DType::F64;
   if (!raw.empty() && raw.dt == DType::F64 && dt == DType::C128) raw = to_complex(c, raw);
