@@ -704,7 +704,7 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
       // sums of squares, cmax per term, coefficients per term and column
       Tensor tab = c.alloc(DType::F64, {4 + (kMaxTerms + 1) * int64_t(n + 1)});
       double *d_sums = tab.f64(), *d_cmax = d_sums + 4, *d_coef = d_cmax + kMaxTerms + 1;
-      double sums[4 + kMaxTerms + 1];  // the host's copy of the first two
+      double sums[4 + kMaxTerms + 1];  // the host's copy of the first two, cmax summed from each term on
       IPEPS_CHECK(n <= 65535, "projector adjoint: too many columns for the grid");
       const dim3 gu(unsigned((N1 + 255) / 256), unsigned(n)), gv(unsigned((N2 + 255) / 256), unsigned(n));
       // W1 = M^T W2 and W2 = M W1 (with M_P in place of M)
@@ -754,8 +754,8 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
         bool blew_up = false, converged = false;
         fill(Tu, Tv);
         // The stopping tests read the sums of squares back (a round trip to the host): at
-        // term kFirstCheck, then where the coefficients' tail has fallen far enough for the
-        // |X| seen last.
+        // term kFirstCheck, then where the sum of the coefficients left has fallen far enough
+        // for the |X| seen last.
         int next = kFirstCheck;
         for (int m = 0; m < kMaxTerms; ++m) {
           c.series_terms++;
@@ -764,19 +764,21 @@ void projector_backward(Ctx& c, const Tensor& R1t, bool t1, const Tensor& R2t, b
             sumsq_dev(c, {Tu, Tv, Xu, Xv}, d_sums);
             IPEPS_CUDA(cudaMemcpyAsync(sums, d_sums, first ? sizeof(sums) : 4 * 8, cudaMemcpyDeviceToHost, c.stream));
             c.sync();
+            double* tail = sums + 4;
+            if (first)
+              for (int j = kMaxTerms; j > 0; --j) tail[j - 1] += tail[j];
             if (!(std::sqrt(sums[0] + sums[1]) <= 8.0 * ny0)) {
               blew_up = true;  // spectrum beyond b
               break;
             }
-            // |T_m| <= |T_0| on [0, b]: the remaining terms are bounded by the coefficient tail
-            const double* cmax = sums + 4;
+            // |T_m| <= |T_0| on [0, b]: the remaining terms are bounded by the sum of their coefficients
             const double bound = kTol * std::sqrt(sums[2] + sums[3]);
-            if (cmax[m + 1] * ny0 <= bound) {
+            if (tail[m + 1] * ny0 <= bound) {
               converged = true;
               break;
             }
             do ++next;
-            while (next < kMaxTerms && cmax[next + 1] * ny0 > bound);
+            while (next < kMaxTerms && tail[next + 1] * ny0 > bound);
           }
           Tensor &nu = Ku[m & 1], &nv = Kv[m & 1];
           const double* pu = m > 1 ? nu.f64() : m > 0 ? Yu0.f64() : nullptr;  // T_{m-1}
